@@ -1,16 +1,26 @@
 // Large-displacement tangent and secant stiffness (Get_MatrixKN, FEM_model_bsr.py:134-145;
 // UnitK :476-515, InslocalBN :544-592, MatrixS :517-525), FP64.
 //
-// k_hex8_tangent: 8 threads per element, 8 elements per CTA.
-//   phase A (thread = Gauss point g): J, det, DN = dN/dx, T = grad u = CoordU . DN;
-//   phase S (thread = corner j): c[g][j] = (D0 (B1_j + BN1_j/2) u_j, D1 (B2_j + BN2_j/2) u_j);
-//   phase P (thread = Gauss point g): S_g = sum over g' <= g and all j of c[g'][j], in the
-//     reference's accumulation order (S is never reset between Gauss points);
-//   phase B (thread = row corner j): for every column corner k, over g,
-//     KT_jk += det ((B1+BN1)_j^T D0 (B1+BN1)_k + (B2+BN2)_j^T D1 (B2+BN2)_k) + det (DN_j . S_g . DN_k) I
-//     KM_jk += det ((B1+BN1)_j^T D0 (B1+BN1/2)_k + (B2+BN2)_j^T D1 (B2+BN2/2)_k)
-//   and writes row j's 8 blocks of each matrix as one row-ordered chunk (the format the
-//   double-float gather consumes) at the corner's incidence position.
+// With T = grad u, Fd = I + T and a_j = grad N_j at a Gauss point, the strain operators of
+// InslocalBN are B1 + BN1 and B2 + BN2 = the linear ones with Fd^T applied to the node's
+// displacement, so UnitK's products collapse to vectors pushed forward by Fd, A_j = Fd a_j:
+//   (B+BN)_j^T D (B+BN)_k   = lam A_j A_k^T + mu A_k A_j^T + mu (a_j.a_k) Fd Fd^T
+//   (B+BN)_j^T D (B+BN/2)_k = 1/2 [the above + lam A_j a_k^T + mu A_k a_j^T + mu (a_j.a_k) Fd]
+// KT adds the geometric term (a_j . S a_k) I, S the second Piola-Kirchhoff stress of the Green
+// strain T + T^T + T^T T, summed over the Gauss points so far and never reset (UnitK does the
+// same: S of Gauss point g holds the points before it).
+//
+// k_hex8_tangent: 8 threads per element, an element's threads in one warp (no block barrier).
+//   phase A (thread = Gauss point g): Jacobian and displacement gradient from trilinear
+//     coefficients, T, Fd, S (prefix sum over the 8 lanes), and per corner a_j, A_j,
+//     mu det a_j, mu det A_j, det S a_j into shared memory;
+//   phase B (thread = corner pair j <= k): the five sums over g above, both matrices' blocks (j, k)
+//     and (k, j), written as float pairs into the row-ordered chunks the double-float gather reads.
+// Bound by the FP64 pipe (about 2,900 FP64 instructions per thread, conversions included).  The
+// direct 3x3x3 products of UnitK, every (j, k, g) with its structural zeros, were about 16,000:
+// KT and KM of 64 x 48 x 15 elements 15.25 -> 2.28 ms, the two gathers (0.21 ms) included.  The 28
+// off-diagonal pairs are 3.5 per thread: the last four are shared by two threads, four Gauss points
+// each, instead of idling half the lanes of a fourth round.
 // Both matrices are then gathered (atomic-free, fixed order) with the penalty applied.
 #include "fem_common.cuh"
 
@@ -20,7 +30,11 @@ namespace {
 constexpr int kEpcT = 8;
 constexpr int kThreadsT = kEpcT * 8;
 constexpr int kChunkT = 84;  // float pairs per (element, corner) chunk: 8 blocks x 10 + F 3 + pad
-constexpr int kChunkFT = 80;
+// Shared doubles per (Gauss point, corner): a, A, mu det a, mu det A, det S a.  An odd row keeps
+// 8 corners in 8 different bank pairs; 8 more doubles per element move the second element of a
+// half warp to the other 8.
+constexpr int kRowT = 15;
+constexpr int kElemT = 64 * kRowT + 8;
 
 struct TangentParams {
     const double* xyz;
@@ -31,18 +45,15 @@ struct TangentParams {
     float2* recT;
     float2* recM;
     double D0d, lam, mu;
+    double lm;  // lam / mu = 2 PO / (1 - 2 PO)
     double dnr[8][8][3];
 };
 
 struct TangentSmem {
-    double dnr[8][8][3];
-    double xl[kEpcT][8][3];
-    double ue[kEpcT][8][3];
-    double DN[kEpcT][8][8][3];  // [g][a][d]
-    double T[kEpcT][8][3][3];   // [g][k][d]
-    double det[kEpcT][8];
-    double c[kEpcT][8][8][6];   // [g][j]
-    double S[kEpcT][8][6];      // accumulated S after Gauss point g
+    double v[kEpcT][kElemT];
+    double q[kEpcT][8][15];   // Fd Fd^T (00, 11, 22, 01, 02, 12), Fd (row-major)
+    double cf[kEpcT][8][6];   // Walsh sums of the coordinates and displacements
+    double dnr[8][25];
 };
 
 __device__ __forceinline__ float2 split(double x) {
@@ -50,59 +61,163 @@ __device__ __forceinline__ float2 split(double x) {
     return make_float2(hi, __double2float_rn(x - double(hi)));
 }
 
-// B1 = diag(DN), B2 rows (yz, xz, xy) of corner a (installLocalB, FEM_model_bsr.py:303-347);
-// BN1, BN2 of corner a (InslocalBN, :544-592); all 3x3 [row][col].
-__device__ __forceinline__ void strain_ops(const double (&dn)[3], const double (&T)[3][3], double (&B1)[3][3],
-                                           double (&B2)[3][3], double (&N1)[3][3], double (&N2)[3][3]) {
+// Block as 9 float pairs + a zero pair at dst (16-byte aligned).
+__device__ __forceinline__ void split_block(const double (&v)[9], float2 (&w)[10]) {
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+    for (int i = 0; i < 9; ++i) w[i] = split(v[i]);
+    w[9] = make_float2(0.f, 0.f);
+}
+template <bool kTranspose>
+__device__ __forceinline__ void store_block(float2* dst, const float2 (&w)[10]) {
+    float4* d = reinterpret_cast<float4*>(dst);
+    auto at = [](int i) { return kTranspose && i < 9 ? 3 * (i % 3) + i / 3 : i; };
 #pragma unroll
-        for (int c = 0; c < 3; ++c) B1[r][c] = r == c ? dn[r] : 0.0;
-    B2[0][0] = 0.0, B2[0][1] = dn[2], B2[0][2] = dn[1];
-    B2[1][0] = dn[2], B2[1][1] = 0.0, B2[1][2] = dn[0];
-    B2[2][0] = dn[1], B2[2][1] = dn[0], B2[2][2] = 0.0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        N1[0][k] = T[k][0] * dn[0];
-        N1[1][k] = T[k][1] * dn[1];
-        N1[2][k] = T[k][2] * dn[2];
-        N2[0][k] = T[k][2] * dn[1] + T[k][1] * dn[2];
-        N2[1][k] = T[k][2] * dn[0] + T[k][0] * dn[2];
-        N2[2][k] = T[k][1] * dn[0] + T[k][0] * dn[1];
+    for (int i = 0; i < 5; ++i) {
+        const float2 x = w[at(2 * i)], y = w[at(2 * i + 1)];
+        d[i] = make_float4(x.x, x.y, y.x, y.y);
     }
+}
+
+// The sums over Gauss points of one corner pair (j, k).
+struct PairSums {
+    double p1[9];   // sum mu det A_j A_k^T
+    double pjk[9];  // sum mu det A_j a_k^T
+    double pkj[9];  // sum mu det A_k a_j^T
+    double sb[6];   // sum mu det (a_j.a_k) Fd Fd^T
+    double sf[9];   // sum mu det (a_j.a_k) Fd
+    double geo;     // sum det a_j . S a_k
+};
+
+template <bool kDiag>
+__device__ __forceinline__ void pair_sums(const TangentSmem& s, int el, int j, int k, int g0, int ng, PairSums& r) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) r.p1[i] = r.pjk[i] = r.pkj[i] = r.sf[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) r.sb[i] = 0.0;
+    r.geo = 0.0;
+#pragma unroll 1
+    for (int g = g0; g < g0 + ng; ++g) {
+        const double* vj = s.v[el] + (g * 8 + j) * kRowT;
+        const double* vk = s.v[el] + (g * 8 + k) * kRowT;
+        const double* q = s.q[el][g];
+        const double ak[3] = {vk[0], vk[1], vk[2]};
+        const double sc = fma(vj[8], ak[2], fma(vj[7], ak[1], vj[6] * ak[0]));   // mu det a_j . a_k
+        r.geo = fma(vj[14], ak[2], fma(vj[13], ak[1], fma(vj[12], ak[0], r.geo)));
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const double Aj = vj[3 + p], Ak = vk[3 + p];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (!kDiag || c >= p) r.p1[3 * p + c] = fma(Aj, vk[9 + c], r.p1[3 * p + c]);
+                r.pjk[3 * p + c] = fma(Aj, vk[6 + c], r.pjk[3 * p + c]);
+                if (!kDiag) r.pkj[3 * p + c] = fma(Ak, vj[6 + c], r.pkj[3 * p + c]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 6; ++i) r.sb[i] = fma(sc, q[i], r.sb[i]);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) r.sf[i] = fma(sc, q[6 + i], r.sf[i]);
+    }
+}
+
+// KT_jk, KM_jk and KM_kj of a pair (KT_kj is KT_jk transposed); lm = lam / mu.
+template <bool kDiag>
+__device__ __forceinline__ void pair_blocks(const PairSums& r, double lm, double (&KT)[9], double (&KM)[9],
+                                            double (&KMt)[9]) {
+    const double B[9] = {r.sb[0], r.sb[3], r.sb[4], r.sb[3], r.sb[1], r.sb[5], r.sb[4], r.sb[5], r.sb[2]};
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int i = 3 * p + c, t = 3 * c + p;
+            if (kDiag) {
+                const double x = c >= p ? r.p1[i] : r.p1[t];
+                KT[i] = fma(lm, x, x + B[i]);
+            } else {
+                KT[i] = fma(lm, r.p1[i], r.p1[t] + B[i]);
+            }
+        }
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int i = 3 * p + c, t = 3 * c + p;
+            if (kDiag) {
+                KM[i] = 0.5 * (KT[i] + fma(lm, r.pjk[i], r.pjk[i] + r.sf[i]));
+            } else {
+                KM[i] = 0.5 * (KT[i] + fma(lm, r.pjk[i], r.pkj[i] + r.sf[i]));
+                KMt[i] = 0.5 * (KT[t] + fma(lm, r.pkj[i], r.pjk[i] + r.sf[i]));
+            }
+        }
+    KT[0] += r.geo;
+    KT[4] += r.geo;
+    KT[8] += r.geo;
+}
+
+// Off-diagonal pair q of 28 (j < k, row-major).
+__device__ __forceinline__ void offdiag_pair(int q, int& j, int& k) {
+    int a = 0, rem = q;
+    while (rem >= 7 - a) {
+        rem -= 7 - a;
+        ++a;
+    }
+    j = a;
+    k = a + 1 + rem;
 }
 
 __global__ void __launch_bounds__(kThreadsT) k_hex8_tangent(const TangentParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TangentSmem& s = *reinterpret_cast<TangentSmem*>(smem_raw);
+    const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, el = tid >> 3, t = tid & 7;
-    const int64_t e = int64_t(blockIdx.x) * kEpcT + el;
-    const bool valid = e < p.n_elem;
-    for (int k = tid; k < 8 * 8 * 3; k += kThreadsT) (&s.dnr[0][0][0])[k] = (&p.dnr[0][0][0])[k];
-    const double D0[3][3] = {{p.D0d, p.lam, p.lam}, {p.lam, p.D0d, p.lam}, {p.lam, p.lam, p.D0d}};
-    if (valid) {
-        const int* cn = reinterpret_cast<const int*>(p.conn4) + 8 * e;
-        const int64_t node = __ldg(cn + t), node0 = __ldg(cn);
+    const int64_t e_raw = int64_t(blockIdx.x) * kEpcT + el;
+    const bool valid = e_raw < p.n_elem;
+    const int64_t e = valid ? e_raw : p.n_elem - 1;   // the lanes of absent elements repeat the last one
+    for (int i = tid; i < 192; i += kThreadsT) s.dnr[i / 24][i % 24] = (&p.dnr[0][0][0])[i];
+    const int64_t pos = __ldg(p.ne_inv + 8 * e + t);
+    double c[6];
+    {
+        const int64_t node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            s.xl[el][t][i] = __ldg(p.xyz + 3 * node + i) - __ldg(p.xyz + 3 * node0 + i);
-            s.ue[el][t][i] = __ldg(p.u + 3 * node + i);
+            c[i] = __ldg(p.xyz + 3 * node + i);
+            c[3 + i] = __ldg(p.u + 3 * node + i);
         }
     }
-    __syncthreads();
-    // phase A: Gauss point g = t
-    if (valid) {
+    const int corner0 = tid & 24;  // lane of the element's corner 0
+#pragma unroll
+    for (int i = 0; i < 6; ++i) c[i] -= __shfl_sync(full, c[i], corner0);   // gradients need differences only
+    // Walsh sums over the 8 corners, W_s = sum_a (-1)^popc(s & a) v_a on lane s.  With xi, eta, zeta
+    // negative at corners {1,2,5,6}, {2,3,6,7}, {0,1,2,3}, the trilinear coefficients are xi: W_3,
+    // eta: W_2, zeta: -W_4, xi eta: W_1, eta zeta: -W_6, xi zeta: -W_7, xi eta zeta: -W_5 (all / 8).
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const double o = __shfl_xor_sync(full, c[i], m);
+            c[i] = (t & m) ? o - c[i] : o + c[i];
+        }
+    const double eighth = (t & 4) ? -0.125 : 0.125;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) s.cf[el][t][i] = eighth * c[i];
+    __syncthreads();  // the shape table is shared by the two warps
+
+    // ---- phase A: Gauss point g = t -----------------------------------------------------------
+    {
         const int g = t;
-        double J[3][3];
+        const double xi = (g & 4) ? kGS1 : -kGS1, et = (g & 2) ? kGS1 : -kGS1, ze = (g & 1) ? kGS1 : -kGS1;
+        double J[3][3], G[3][3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                double a = 0.0;
-                for (int c = 0; c < 8; ++c) a += s.xl[el][c][i] * s.dnr[g][c][d];
-                J[i][d] = a;
-            }
-        double A[3][3];  // adjugate
+        for (int i = 0; i < 6; ++i) {
+            const double c1 = s.cf[el][3][i], c2 = s.cf[el][2][i], c3 = s.cf[el][4][i], c4 = s.cf[el][1][i];
+            const double c5 = s.cf[el][6][i], c6 = s.cf[el][7][i], c7 = s.cf[el][5][i];
+            double* d = i < 3 ? J[i] : G[i - 3];
+            const double m = fma(xi, c7, c5);
+            d[0] = fma(ze, fma(et, c7, c6), fma(et, c4, c1));
+            d[1] = fma(ze, m, fma(xi, c4, c2));
+            d[2] = fma(et, m, fma(xi, c6, c3));
+        }
+        double A[3][3];  // adjugate, then the inverse
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -112,120 +227,125 @@ __global__ void __launch_bounds__(kThreadsT) k_hex8_tangent(const TangentParams 
             }
         const double det = J[0][0] * A[0][0] + J[1][0] * A[0][1] + J[2][0] * A[0][2];
         const double inv = 1.0 / det;
-        s.det[el][g] = det;
-        for (int a = 0; a < 8; ++a)
 #pragma unroll
-            for (int d = 0; d < 3; ++d)
-                s.DN[el][g][a][d] = (s.dnr[g][a][0] * A[0][d] + s.dnr[g][a][1] * A[1][d] + s.dnr[g][a][2] * A[2][d]) * inv;
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
+            for (int j = 0; j < 3; ++j) A[i][j] *= inv;
+        double T[3][3];  // T[i][d] = du_i / dx_d
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) T[i][d] = fma(G[i][2], A[2][d], fma(G[i][1], A[1][d], G[i][0] * A[0][d]));
+        double S[6];  // xx, yy, zz, yz, xz, xy of the Green strain's stress
+        {
+            double E[3], gm[3];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const double sq = fma(T[2][m], T[2][m], fma(T[1][m], T[1][m], T[0][m] * T[0][m]));
+                E[m] = fma(0.5, sq, T[m][m]);
+                const int a = (m + 1) % 3, b = (m + 2) % 3;   // m = 0: yz, 1: zx, 2: xy
+                gm[m] = fma(T[2][a], T[2][b], fma(T[1][a], T[1][b], fma(T[0][a], T[0][b], T[a][b] + T[b][a])));
+            }
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                S[m] = fma(p.D0d, E[m], p.lam * (E[(m + 1) % 3] + E[(m + 2) % 3]));
+                S[3 + m] = p.mu * gm[m];
+            }
+        }
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1)
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                const double o = __shfl_up_sync(full, S[i], off, 8);
+                if (t >= off) S[i] += o;
+            }
+        const double md = p.mu * det;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) S[i] *= det;
+        double* q = s.q[el][g];
+        double Fd[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                double a = 0.0;
-                for (int c = 0; c < 8; ++c) a += s.ue[el][c][k] * s.DN[el][g][c][d];
-                s.T[el][g][k][d] = a;
-            }
-    }
-    __syncthreads();
-    // phase S: corner j = t, every Gauss point
-    if (valid) {
-        const int j = t;
-        const double uj[3] = {s.ue[el][j][0], s.ue[el][j][1], s.ue[el][j][2]};
-        for (int g = 0; g < 8; ++g) {
-            const double dn[3] = {s.DN[el][g][j][0], s.DN[el][g][j][1], s.DN[el][g][j][2]};
-            const double(&T)[3][3] = s.T[el][g];
-            double B1[3][3], B2[3][3], N1[3][3], N2[3][3];
-            strain_ops(dn, T, B1, B2, N1, N2);
-            double t1[3], t2[3];
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                t1[r] = (B1[r][0] + 0.5 * N1[r][0]) * uj[0] + (B1[r][1] + 0.5 * N1[r][1]) * uj[1] +
-                        (B1[r][2] + 0.5 * N1[r][2]) * uj[2];
-                t2[r] = (B2[r][0] + 0.5 * N2[r][0]) * uj[0] + (B2[r][1] + 0.5 * N2[r][1]) * uj[1] +
-                        (B2[r][2] + 0.5 * N2[r][2]) * uj[2];
+                Fd[i][d] = i == d ? 1.0 + T[i][d] : T[i][d];
+                q[6 + 3 * i + d] = Fd[i][d];
             }
 #pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                s.c[el][g][j][r] = D0[r][0] * t1[0] + D0[r][1] * t1[1] + D0[r][2] * t1[2];
-                s.c[el][g][j][3 + r] = p.mu * t2[r];
+        for (int i = 0; i < 6; ++i) {
+            const int a = i < 3 ? i : (i == 5 ? 1 : 0), b = i < 3 ? i : (i == 3 ? 1 : 2);
+            q[i] = fma(Fd[a][2], Fd[b][2], fma(Fd[a][1], Fd[b][1], Fd[a][0] * Fd[b][0]));
+        }
+#pragma unroll 2
+        for (int j = 0; j < 8; ++j) {
+            double* v = s.v[el] + (g * 8 + j) * kRowT;
+            const double* dn = s.dnr[g] + 3 * j;
+            double a[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) a[d] = fma(dn[2], A[2][d], fma(dn[1], A[1][d], dn[0] * A[0][d]));
+            const double Sa[3] = {fma(S[4], a[2], fma(S[5], a[1], S[0] * a[0])),
+                                  fma(S[3], a[2], fma(S[1], a[1], S[5] * a[0])),
+                                  fma(S[2], a[2], fma(S[3], a[1], S[4] * a[0]))};
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double Aj = fma(Fd[d][2], a[2], fma(Fd[d][1], a[1], Fd[d][0] * a[0]));
+                v[d] = a[d];
+                v[3 + d] = Aj;
+                v[6 + d] = md * a[d];
+                v[9 + d] = md * Aj;
+                v[12 + d] = Sa[d];
             }
         }
     }
-    __syncthreads();
-    // phase P: S after Gauss point g = t (accumulated in the reference's g, j order)
-    if (valid) {
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        for (int g = 0; g <= t; ++g)
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int q = 0; q < 6; ++q) acc[q] += s.c[el][g][j][q];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) s.S[el][t][q] = acc[q];
+    __syncwarp();
+
+    // ---- phase B: corner pairs ---------------------------------------------------------------
+    const double lm = p.lm;
+    const int base = tid & 24;
+    auto chunk = [&](float2* rec, int row) { return rec + __shfl_sync(full, pos, base | row) * kChunkT; };
+    PairSums r;
+    double KT[9], KM[9], KMt[9];
+    {
+        pair_sums<true>(s, el, t, t, 0, 8, r);
+        pair_blocks<true>(r, lm, KT, KM, KMt);
+        float2 w[10];
+        split_block(KT, w);
+        if (valid) store_block<false>(p.recT + pos * kChunkT + 10 * t, w);
+        split_block(KM, w);
+        if (valid) store_block<false>(p.recM + pos * kChunkT + 10 * t, w);
     }
-    __syncthreads();
-    if (!valid) return;
-    // phase B: row corner j = t
-    const int j = t;
-    float2* cT = p.recT + int64_t(__ldg(p.ne_inv + 8 * e + j)) * kChunkT;
-    float2* cM = p.recM + int64_t(__ldg(p.ne_inv + 8 * e + j)) * kChunkT;
-    for (int k = 0; k < 8; ++k) {
-        double KT[3][3] = {}, KM[3][3] = {};
-        for (int g = 0; g < 8; ++g) {
-            const double(&T)[3][3] = s.T[el][g];
-            const double dj[3] = {s.DN[el][g][j][0], s.DN[el][g][j][1], s.DN[el][g][j][2]};
-            const double dk[3] = {s.DN[el][g][k][0], s.DN[el][g][k][1], s.DN[el][g][k][2]};
-            double B1j[3][3], B2j[3][3], N1j[3][3], N2j[3][3], B1k[3][3], B2k[3][3], N1k[3][3], N2k[3][3];
-            strain_ops(dj, T, B1j, B2j, N1j, N2j);
-            strain_ops(dk, T, B1k, B2k, N1k, N2k);
-            // M1 = (B1 + BN1)_j^T D0, M2 = (B2 + BN2)_j^T D1 (= mu (B2 + BN2)_j^T)
-            double M1[3][3], M2[3][3];
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const bool shared_pair = i == 3;   // the last four pairs: two threads, four Gauss points each
+        int j, k;
+        offdiag_pair(shared_pair ? 24 + (t >> 1) : 8 * i + t, j, k);
+        pair_sums<false>(s, el, j, k, shared_pair ? 4 * (t & 1) : 0, shared_pair ? 4 : 8, r);
+        if (shared_pair) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    M1[a][b] = (B1j[0][a] + N1j[0][a]) * D0[0][b] + (B1j[1][a] + N1j[1][a]) * D0[1][b] +
-                               (B1j[2][a] + N1j[2][a]) * D0[2][b];
-                    M2[a][b] = p.mu * (B2j[b][a] + N2j[b][a]);
-                }
-            const double det = s.det[el][g];
-            const double* Sg = s.S[el][g];
-            // geometric term DN_j . s . DN_k with s = [[S0x, S1z, S1y], [S1z, S0y, S1x], [S1y, S1x, S0z]]
-            const double sm[3][3] = {{Sg[0], Sg[5], Sg[4]}, {Sg[5], Sg[1], Sg[3]}, {Sg[4], Sg[3], Sg[2]}};
-            double geo = 0.0;
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) geo += dj[a] * sm[a][b] * dk[b];
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    double Av = 0.0, Bv = 0.0;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        Av += M1[a][c] * B1k[c][b] + M2[a][c] * B2k[c][b];
-                        Bv += M1[a][c] * N1k[c][b] + M2[a][c] * N2k[c][b];
-                    }
-                    KT[a][b] += det * (Av + Bv);
-                    KM[a][b] += det * (Av + 0.5 * Bv);
-                }
-#pragma unroll
-            for (int a = 0; a < 3; ++a) KT[a][a] += det * geo;
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                cT[k * 10 + 3 * a + b] = split(KT[a][b]);
-                cM[k * 10 + 3 * a + b] = split(KM[a][b]);
+            for (int m = 0; m < 9; ++m) {
+                r.p1[m] += __shfl_xor_sync(full, r.p1[m], 1);
+                r.pjk[m] += __shfl_xor_sync(full, r.pjk[m], 1);
+                r.pkj[m] += __shfl_xor_sync(full, r.pkj[m], 1);
+                r.sf[m] += __shfl_xor_sync(full, r.sf[m], 1);
             }
-        cT[k * 10 + 9] = make_float2(0.f, 0.f);
-        cM[k * 10 + 9] = make_float2(0.f, 0.f);
-    }
 #pragma unroll
-    for (int q = 0; q < kChunkT - kChunkFT; ++q) {
-        cT[kChunkFT + q] = make_float2(0.f, 0.f);
-        cM[kChunkFT + q] = make_float2(0.f, 0.f);
+            for (int m = 0; m < 6; ++m) r.sb[m] += __shfl_xor_sync(full, r.sb[m], 1);
+            r.geo += __shfl_xor_sync(full, r.geo, 1);
+        }
+        pair_blocks<false>(r, lm, KT, KM, KMt);
+        float2* Tj = chunk(p.recT, j) + 10 * k;
+        float2* Tk = chunk(p.recT, k) + 10 * j;
+        float2* Mj = chunk(p.recM, j) + 10 * k;
+        float2* Mk = chunk(p.recM, k) + 10 * j;
+        const bool wT = valid && !(shared_pair && (t & 1)), wM = valid && !(shared_pair && !(t & 1));
+        float2 w[10];
+        split_block(KT, w);
+        if (wT) store_block<false>(Tj, w);
+        if (wT) store_block<true>(Tk, w);
+        split_block(KM, w);
+        if (wM) store_block<false>(Mj, w);
+        split_block(KMt, w);
+        if (wM) store_block<false>(Mk, w);
     }
 }
 
@@ -280,6 +400,7 @@ extern "C" int fem_assemble_tangent(const fem_mesh* mesh, const fem_material* ma
         tp.D0d = EX * (1 - PO) / (1 + PO) / (1 - 2 * PO);  // FEM_model_bsr.py:435-449
         tp.lam = EX * PO / (1 + PO) / (1 - 2 * PO);
         tp.mu = EX / 2 / (1 + PO);
+        tp.lm = 2 * PO / (1 - 2 * PO);
         const ShapeTables& T = shape_tables();
         for (int g = 0; g < 8; ++g)
             for (int a = 0; a < 8; ++a)
