@@ -26,9 +26,9 @@
 //  k_prol_*      one warp per row: the distinct aggregates of the row's neighbours (sorted),
 //                then P_ia = -omega D_i^-1 sum_j A_ij T_j (+ T_i on the row's own aggregate)
 //  k_tr_*        R = P^T: column counts, scan, scatter, then a per-row sort by fine row
-//  k_sg_*        Z = X Y one warp per row: distinct columns in a shared-memory hash table,
-//                sorted; each output block accumulates X_l Y_t over the row's X entries l in
-//                ascending order (the host's Gustavson order), lanes over (t, block entry)
+//  k_sg_*        Z = X Y: distinct columns in a shared-memory hash table, sorted; each output
+//                block accumulates X_l Y_t over the row's X entries l in ascending order (the
+//                host's Gustavson order); a warp per row on level 0, a block per row below
 // The FP32 copies the V-cycle reads (amg.cu) are written directly from the FP64 results.
 #include <math.h>
 
@@ -286,63 +286,145 @@ __global__ void k_rigid_modes(int64_t n, const double* __restrict__ xyz, double 
 
 // One thread per aggregate, in the host setup's order (amg_setup.cpp:tentative): T rows of
 // the members (T[node][B][6], rows in member order) = the aggregate's rows of the near-null
-// space, orthonormalised column by column by two-pass modified Gram-Schmidt; Bc[a] = R.
-template <int B>
+// space, orthonormalised column by column by two-pass modified Gram-Schmidt; Bc[a] = R.  The sums
+// are serial chains of 42 passes over the rows.  kShared: the rows stay in shared memory
+// meanwhile, value v of thread t at [v * blockDim.x + t], and loads run four rows ahead of the
+// chains (columns c and c2 never overlap, which the compiler cannot know).  On the T rows in global
+// memory every step of a chain was an L2 load: 2.52 ms for 12,410 aggregates of 17 nodes, 1.53 ms
+// here.  The global form serves levels with an aggregate too large for shared memory.
+template <int B, bool kShared>
 __global__ void k_tentative(int64_t na, const int32_t* __restrict__ aptr, const int32_t* __restrict__ mem,
                             const double* __restrict__ Bn, double* T, double* Bc) {
     constexpr int k = kModes;
+    extern __shared__ __align__(16) double trows[];
     for (int64_t a = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; a < na; a += int64_t(gridDim.x) * blockDim.x) {
         const int s0 = aptr[a], cnt = aptr[a + 1] - s0, rows = cnt * B;
-        auto rowp = [&](int r) { return T + (int64_t(mem[s0 + r / B]) * B + r % B) * k; };
+        auto gat = [&](int r) { return (int64_t(mem[s0 + r / B]) * B + r % B) * k; };
+        auto at = [&](int r, int c) -> double& {
+            if constexpr (kShared) return trows[(r * k + c) * int(blockDim.x) + int(threadIdx.x)];
+            else return T[gat(r) + c];
+        };
+        // sum over the rows, in order, of column c2 times column c
+        auto dot = [&](int c2, int c) {
+            double d = 0.0;
+            int r = 0;
+            for (; r + 4 <= rows; r += 4) {
+                double p[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) p[j] = at(r + j, c2) * at(r + j, c);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d += p[j];
+            }
+            for (; r < rows; ++r) d += at(r, c2) * at(r, c);
+            return d;
+        };
         for (int r = 0; r < rows; ++r) {
-            const double* src = Bn + (int64_t(mem[s0 + r / B]) * B + r % B) * k;
-            double* dst = rowp(r);
-            for (int m = 0; m < k; ++m) dst[m] = src[m];
+            const double* src = Bn + gat(r);
+            for (int m = 0; m < k; ++m) at(r, m) = src[m];
         }
         double R[k][k];
         for (int i = 0; i < k; ++i)
             for (int j = 0; j < k; ++j) R[i][j] = 0.0;
         for (int c = 0; c < k; ++c) {
-            double n0 = 0.0;
-            for (int r = 0; r < rows; ++r) n0 += rowp(r)[c] * rowp(r)[c];
-            n0 = sqrt(n0);
+            const double n0 = sqrt(dot(c, c));
             for (int pass = 0; pass < 2; ++pass)
                 for (int c2 = 0; c2 < c; ++c2) {
-                    double d = 0.0;
-                    for (int r = 0; r < rows; ++r) d += rowp(r)[c2] * rowp(r)[c];
-                    for (int r = 0; r < rows; ++r) rowp(r)[c] -= d * rowp(r)[c2];
+                    const double d = dot(c2, c);
+                    int r = 0;
+                    for (; r + 4 <= rows; r += 4) {
+                        double p[4], q[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) p[j] = at(r + j, c), q[j] = at(r + j, c2);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) at(r + j, c) = p[j] - d * q[j];
+                    }
+                    for (; r < rows; ++r) at(r, c) -= d * at(r, c2);
                     R[c2][c] += d;
                 }
-            double nr = 0.0;
-            for (int r = 0; r < rows; ++r) nr += rowp(r)[c] * rowp(r)[c];
-            nr = sqrt(nr);
+            const double nr = sqrt(dot(c, c));
             if (nr > 1e-10 * n0 && nr > 0.0) {
-                for (int r = 0; r < rows; ++r) rowp(r)[c] /= nr;
+                for (int r = 0; r < rows; ++r) at(r, c) /= nr;
                 R[c][c] = nr;
             } else {
-                for (int r = 0; r < rows; ++r) rowp(r)[c] = 0.0;
+                for (int r = 0; r < rows; ++r) at(r, c) = 0.0;
                 R[c][c] = 0.0;
             }
         }
         for (int i = 0; i < k; ++i)
             for (int j = 0; j < k; ++j) Bc[(a * k + i) * k + j] = R[i][j];
+        if constexpr (kShared)
+            for (int r = 0; r < rows; ++r)
+                for (int m = 0; m < k; ++m) T[gat(r) + m] = at(r, m);
     }
 }
 
 // ---- Lanczos estimate of lambda_max(D^-1 A) ---------------------------------------------------
+// y = A x.  One thread per scalar row (i, r): its sum runs over l and c in the host's order, one
+// rounded product and one add per term, so a block row's B chains are the parallelism.  Groups of kU
+// blocks are software-pipelined (the next group's values and vector entries load while this one is
+// added, the column after next is already there), else every block waits out two dependent loads:
+// one thread per block row took 1.26 ms a product on the coarse levels of the 214k-node 4:1 block,
+// 0.13-0.21 ms here.  (Staging products through shared memory a warp at a time, measured too, was
+// slower than the plain form: 370 us, bound by its index arithmetic.)
 template <int B>
-__global__ void k_spmv64(int64_t n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
-                         const double* __restrict__ val, const double* __restrict__ x, double* y) {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        double acc[B];
-        for (int r = 0; r < B; ++r) acc[r] = 0.0;
-        for (int l = ptr[i]; l < ptr[i + 1]; ++l) {
-            const double* a = val + int64_t(l) * B * B;
-            const double* xc = x + int64_t(col[l]) * B;
-            for (int r = 0; r < B; ++r)
-                for (int c = 0; c < B; ++c) acc[r] += a[r * B + c] * xc[c];
+__device__ __forceinline__ void load_row(const double* __restrict__ p, double (&v)[B]) {
+    if constexpr (B % 2 == 0) {  // rows of 6 start on 16-byte boundaries
+#pragma unroll
+        for (int c = 0; c < B / 2; ++c) {
+            const double2 d = __ldg(reinterpret_cast<const double2*>(p) + c);
+            v[2 * c] = d.x;
+            v[2 * c + 1] = d.y;
         }
-        for (int r = 0; r < B; ++r) y[i * B + r] = acc[r];
+    } else {
+#pragma unroll
+        for (int c = 0; c < B; ++c) v[c] = __ldg(p + c);
+    }
+}
+
+template <int B>
+__global__ void __launch_bounds__(128) k_spmv64(int64_t n, const int32_t* __restrict__ ptr,
+                                                const int32_t* __restrict__ col, const double* __restrict__ val,
+                                                const double* __restrict__ x, double* y) {
+    constexpr int kU = 4;
+    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n * B; t += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t i = t / B;
+        const int r = int(t - i * B);
+        const int s = ptr[i], e = ptr[i + 1];
+        double a[2][kU][B], v[2][kU][B];
+        int cn[kU];
+        auto load_cols = [&](int l0) {
+#pragma unroll
+            for (int j = 0; j < kU; ++j) cn[j] = l0 + j < e ? __ldg(col + l0 + j) : 0;
+        };
+        auto load_group = [&](int l0, double (&ga)[kU][B], double (&gv)[kU][B]) {
+#pragma unroll
+            for (int j = 0; j < kU; ++j)
+                if (l0 + j < e) {
+                    load_row<B>(val + (int64_t(l0) + j) * B * B + r * B, ga[j]);
+                    load_row<B>(x + int64_t(cn[j]) * B, gv[j]);
+                }
+        };
+        double acc = 0.0;
+        auto add_group = [&](int l0, double (&ga)[kU][B], double (&gv)[kU][B]) {
+#pragma unroll
+            for (int j = 0; j < kU; ++j)
+                if (l0 + j < e) {
+#pragma unroll
+                    for (int c = 0; c < B; ++c) acc += ga[j][c] * gv[j][c];
+                }
+        };
+        load_cols(s);
+        load_group(s, a[0], v[0]);
+        load_cols(s + kU);
+        for (int l = s; l < e; l += 2 * kU) {
+            load_group(l + kU, a[1], v[1]);
+            load_cols(l + 2 * kU);
+            add_group(l, a[0], v[0]);
+            load_group(l + 2 * kU, a[0], v[0]);
+            load_cols(l + 3 * kU);
+            add_group(l + kU, a[1], v[1]);
+        }
+        y[t] = acc;
     }
 }
 
@@ -371,20 +453,40 @@ __global__ void k_splitmix(int64_t N, double* v) {
 }
 
 // part[c] = sum over chunk c (kSumChunk consecutive elements, in order) of a[i] * b[i], or of
-// a[i * stride + off] when b is null: the host setup's order (amg_setup.cpp:dot)
-__global__ void k_chunk_sums(int64_t N, const double* __restrict__ a, const double* __restrict__ b, int stride,
-                             int off, double* part) {
-    const int64_t nc = (N + kSumChunk - 1) / kSumChunk;
-    for (int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < nc; c += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t e = std::min(N, (c + 1) * kSumChunk);
-        double s = 0.0;
-        if (b) {
-            for (int64_t i = c * kSumChunk; i < e; ++i) s += a[i] * b[i];
-        } else {
-            for (int64_t i = c * kSumChunk; i < e; ++i) s += a[i * stride + off];
-        }
-        part[c] = s;
+// a[i * stride + off] when b is null: the host setup's order (amg_setup.cpp:dot).  A chunk's sum is
+// a serial chain, so the block loads 32 chunks into shared memory, every load in flight at once, and
+// one warp sums them, a chunk per lane (one thread per chunk on global memory: 279 us a launch at
+// 642,663 elements, its loads one sector each and in line with the sum; here 21 us).
+__global__ void __launch_bounds__(kT) k_chunk_sums(int64_t N, const double* __restrict__ a,
+                                                   const double* __restrict__ b, int stride, int off, double* part) {
+    extern __shared__ __align__(16) double tile[];  // [32][kSumChunk + 1]
+    static_assert(kSumChunk == kT, "one element of each chunk per thread");
+    const int tid = threadIdx.x;
+    const int64_t nc = (N + kSumChunk - 1) / kSumChunk, c0 = int64_t(blockIdx.x) * 32;
+    double v[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+        const int64_t i = (c0 + c) * kSumChunk + tid;
+        v[c] = i < N ? (b ? a[i] : a[i * stride + off]) : 0.0;
     }
+    if (b) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+            const int64_t i = (c0 + c) * kSumChunk + tid;
+            if (i < N) v[c] *= b[i];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 32; ++c) tile[c * (kSumChunk + 1) + tid] = v[c];
+    __syncthreads();
+    if (tid >= 32 || c0 + tid >= nc) return;
+    const int64_t left = N - (c0 + tid) * kSumChunk;
+    const int m = int(left < kSumChunk ? left : kSumChunk);
+    const double* row = tile + tid * (kSumChunk + 1);
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) s += row[k];
+    part[c0 + tid] = s;
 }
 
 __global__ void k_lanczos_w(int64_t N, double* w, double a, const double* __restrict__ v, double bj,
@@ -409,12 +511,6 @@ __device__ void mark_first(const int32_t* keys, int L, uint8_t* flags, int lane)
     }
     __syncwarp();
 }
-__device__ int rank_of(const int32_t* keys, const uint8_t* flags, int L, int32_t k) {
-    int r = 0;
-    for (int p = 0; p < L; ++p) r += (flags[p] && keys[p] < k) ? 1 : 0;
-    return r;
-}
-
 // ---- smoothed prolongator ------------------------------------------------------------------------
 // per row: the number of distinct aggregates among the row's neighbours (0 on Dirichlet rows;
 // P = T when not smoothing)
@@ -444,28 +540,73 @@ __global__ void k_prol_count(int64_t n, const int32_t* __restrict__ ptr, const i
     }
 }
 
-// Per row: the sorted distinct aggregates u of the row's neighbours (rank order), then for
-// every (u, entry (r, c)) -- lanes over these items, so all lanes do FP64 work --
-// acc = sum over the row's entries l with aggregate u, ascending, of sum_q A_il[r][q] T_l[q][c]
+// The row's (aggregate, entry) pairs sorted by aggregate, then entry, as 64-bit keys (aggregate in
+// the high word; unaggregated neighbours last) in buf[0 .. p2), p2 a power of two >= 32 and >= L.
+__device__ void sort_entries(const int32_t* __restrict__ col, const int32_t* __restrict__ agg, int rs, int L, int p2,
+                             unsigned long long* buf, int lane) {
+    auto key = [&](int q) {
+        const int32_t a = q < L ? agg[col[rs + q]] : -1;
+        return a < 0 ? ~0ull : (static_cast<unsigned long long>(a) << 32) | unsigned(q);
+    };
+    if (p2 == 32) {
+        unsigned long long v = key(lane);
+#pragma unroll
+        for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, stride);
+                const bool keep_min = ((lane & size) == 0) == ((lane & stride) == 0);
+                v = (o < v) == keep_min ? o : v;
+            }
+        buf[lane] = v;
+        __syncwarp();
+        return;
+    }
+    for (int q = lane; q < p2; q += 32) buf[q] = key(q);
+    __syncwarp();
+    for (int size = 2; size <= p2; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int h = lane; h < p2 / 2; h += 32) {
+                const int q = 2 * h - (h & (stride - 1)), o = q + stride;
+                const unsigned long long x = buf[q], y = buf[o];
+                if ((x > y) == ((q & size) == 0)) {
+                    buf[q] = y;
+                    buf[o] = x;
+                }
+            }
+            __syncwarp();
+        }
+}
+
+// Per row: its entries sorted by aggregate, so the distinct aggregates u are segments in rank order
+// with their entries ascending; then for every (u, entry (r, c)) -- lanes over these items, so all
+// lanes do FP64 work -- acc = sum over the segment's entries l of sum_q A_il[r][q] T_l[q][c]
 // (the host's Gustavson order), and P_iu = -omega D_i^-1 acc (+ T_i on the row's own
-// aggregate).  Shared memory per warp: keys and first-occurrence flags (maxL each), the
-// distinct keys (maxU) and the accumulators (maxU blocks).
+// aggregate).  Shared memory per warp: the sorted entries (p2), the accumulators (maxU blocks) and the
+// segment starts (maxU + 1); rows too long for it sort in `scratch` in global memory.  (Ranking aggregates by pairwise comparison and testing every entry
+// for every u took 3.92 ms on level 0 of the 214k-node 4:1 block and 4.8 ms below; 1.25 and 2.2 ms here.)
+__host__ __device__ inline size_t prol_row_bytes(int p2, int maxU, int bk) {
+    const size_t per = size_t(p2) * 8 + size_t(maxU) * bk * sizeof(double) + size_t(maxU + 1) * sizeof(int32_t);
+    return (per + 15) & ~size_t(15);
+}
+
 template <int B>
-__global__ void k_prol_fill(int64_t n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
-                            const double* __restrict__ val, const int32_t* __restrict__ agg,
-                            const uint8_t* __restrict__ iso, int smooth, double omega, const double* __restrict__ dinv,
-                            const double* __restrict__ T, int maxL, int maxU, int warps,
-                            const int32_t* __restrict__ pptr, int32_t* pcol, double* pval) {
+__global__ void __launch_bounds__(kT) k_prol_fill(int64_t n, const int32_t* __restrict__ ptr,
+                                                  const int32_t* __restrict__ col, const double* __restrict__ val,
+                                                  const int32_t* __restrict__ agg, const uint8_t* __restrict__ iso,
+                                                  int smooth, double omega, const double* __restrict__ dinv,
+                                                  const double* __restrict__ T, int p2_max, int maxU, int warps,
+                                                  unsigned long long* scratch, const int32_t* __restrict__ pptr,
+                                                  int32_t* pcol, double* pval) {
     constexpr int k = kModes, BK = B * k;
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t per = size_t(maxU) * BK * sizeof(double) + size_t(maxL + maxU) * sizeof(int32_t) + maxL;
-    const size_t per_al = (per + 15) & ~size_t(15);
+    const size_t per_al = prol_row_bytes(scratch ? 0 : p2_max, maxU, BK);
     unsigned char* base = smem + w * per_al;
-    double* acc = reinterpret_cast<double*>(base);
-    int32_t* keys = reinterpret_cast<int32_t*>(acc + size_t(maxU) * BK);
-    int32_t* ukeys = keys + maxL;
-    uint8_t* flags = reinterpret_cast<uint8_t*>(ukeys + maxU);
+    unsigned long long* ent = reinterpret_cast<unsigned long long*>(base);
+    double* acc = reinterpret_cast<double*>(ent + (scratch ? 0 : p2_max));
+    if (scratch) ent = scratch + (int64_t(blockIdx.x) * warps + w) * p2_max;
+    int32_t* seg = reinterpret_cast<int32_t*>(acc + size_t(maxU) * BK);
     const int64_t nw = int64_t(gridDim.x) * warps;
     for (int64_t i = int64_t(blockIdx.x) * warps + w; i < n; i += nw) {
         if (!smooth) {
@@ -479,21 +620,34 @@ __global__ void k_prol_fill(int64_t n, const int32_t* __restrict__ ptr, const in
         if (iso[i]) continue;
         const int rs = ptr[i], L = ptr[i + 1] - rs;
         const int ps = pptr[i], U = pptr[i + 1] - ps;
-        for (int q = lane; q < L; q += 32) keys[q] = agg[col[rs + q]];
-        __syncwarp();
-        mark_first(keys, L, flags, lane);
-        for (int q = lane; q < L; q += 32)
-            if (flags[q]) ukeys[rank_of(keys, flags, L, keys[q])] = keys[q];
+        int p2 = 32;
+        while (p2 < L) p2 <<= 1;
+        sort_entries(col, agg, rs, L, p2, ent, lane);
+        int found = 0;
+        for (int q0 = 0; q0 < L; q0 += 32) {
+            const int q = q0 + lane;
+            const unsigned long long x = q < L ? ent[q] : ~0ull;
+            const bool live = x != ~0ull;
+            const bool head = live && (q == 0 || (ent[q - 1] >> 32) != (x >> 32));
+            const unsigned m = __ballot_sync(0xffffffffu, head);
+            if (head) seg[found + __popc(m & ((1u << lane) - 1u))] = q;
+            found += __popc(m);
+            const unsigned lm = __ballot_sync(0xffffffffu, live);
+            if (lane == 0) seg[U] = q0 + __popc(lm);   // the last pass that has live entries sets it last
+            if (lm != 0xffffffffu) break;              // sorted: nothing live beyond
+        }
         __syncwarp();
         for (int it = lane; it < U * BK; it += 32) {
             const int u = it / BK, e = it - u * BK, r = e / k, c = e - r * k;
-            const int32_t kc = ukeys[u];
             double a = 0.0;
-            for (int l = 0; l < L; ++l) {
-                if (keys[l] != kc) continue;
+            const int m1 = seg[u + 1];
+#pragma unroll 2
+            for (int m = seg[u]; m < m1; ++m) {
+                const int l = int(unsigned(ent[m]));
                 const double* ab = val + int64_t(rs + l) * B * B + r * B;
-                const double* t = T + int64_t(col[rs + l]) * BK + c;
-                for (int q = 0; q < B; ++q) a = fma(ab[q], t[q * k], a);
+                const double* t = T + int64_t(__ldg(col + rs + l)) * BK + c;
+#pragma unroll
+                for (int q = 0; q < B; ++q) a = fma(__ldg(ab + q), __ldg(t + q * k), a);
             }
             acc[it] = a;
         }
@@ -502,12 +656,13 @@ __global__ void k_prol_fill(int64_t n, const int32_t* __restrict__ ptr, const in
         const int32_t own = agg[i];
         for (int it = lane; it < U * BK; it += 32) {
             const int u = it / BK, e = it - u * BK, r = e / k, c = e - r * k;
+            const int32_t ukey = int32_t(ent[seg[u]] >> 32);
             double sdot = 0.0;
             for (int q = 0; q < B; ++q) sdot += di[r * B + q] * acc[u * BK + q * k + c];
             double v = -omega * sdot;
-            if (ukeys[u] == own) v += T[i * BK + e];
+            if (ukey == own) v += T[i * BK + e];
             pval[int64_t(ps + u) * BK + e] = v;
-            if (e == 0) pcol[ps + u] = ukeys[u];
+            if (e == 0) pcol[ps + u] = ukey;
         }
         __syncwarp();
     }
@@ -636,9 +791,13 @@ __global__ void k_sg_count(int64_t n, const int32_t* __restrict__ xptr, const in
 }
 
 // Z row i: sorted distinct columns, then z_(i,col) = sum over X entries l ascending of
-// X_l Y_t (t: the entry of Y row xcol[l] with that column).  Per warp in shared memory: the
-// hash keys and positions (cap each), the distinct keys and their slots (maxu each) and the
-// positions of the current Y row (maxyl).
+// X_l Y_t (t: the entry of Y row xcol[l] with that column).  Two kernels, the same sums:
+//
+// k_sg_fill (3x3 or 6x3 times 3x6 blocks, the level-0 products): many rows whose Y rows are short,
+// so few of the row's distinct columns stand in any one Y row.  One warp per row, lanes over
+// (t, block entry) of one X entry at a time, Z read and written per entry.  It runs at the FP64
+// pipe's rate (3.6 and 5.3 ms on the 214k-node 4:1 block against 2.9 and 4.4 ms of FMAs); the
+// other kernel takes 11.7 and 16.3 ms there, testing each column against each entry.
 template <int BI, int BK, int BJ>
 __global__ void k_sg_fill(int64_t n, const int32_t* __restrict__ xptr, const int32_t* __restrict__ xcol,
                           const double* __restrict__ xval, const int32_t* __restrict__ yptr,
@@ -723,6 +882,151 @@ __global__ void k_sg_fill(int64_t n, const int32_t* __restrict__ xptr, const int
     }
 }
 
+// k_sg_fill_wide (6x6 times 6x6 blocks, the coarser levels): a few hundred to a few thousand rows of
+// up to hundreds of blocks, most columns in most Y rows.  kWarps warps share a row.  The sum of one
+// output is a serial chain over l and the outputs are independent, so each thread owns outputs
+// (column u, entry e) and walks the X entries itself, four at a time with their loads in flight; the
+// warps never wait for one another between entries.  Tables in shared memory, for lc <= 32 entries l
+// at a time, hold a bit mask per column u of the entries whose Y row has it and its place there: a
+// lane visits set bits only, so the two columns a warp spans advance on their own entries (testing
+// every entry left half the FP64 issue slots idle: 40.4 ms).  `splits` blocks share a row's outputs
+// when the rows alone leave SMs idle.  On the 214k-node 4:1 block the six products took 156 ms
+// with k_sg_fill's one warp per row, 37.6 ms here (about 26 ms
+// of FMAs at the FP64 rate).
+// Shared memory: the hash keys and their ranks (cap each), the distinct keys, their slots and their
+// masks (maxu each), the X blocks, the Y row starts and the places of the current lc entries.
+struct SgLayout {
+    size_t xs, hk, hv, ul, us, mk, nu, ts, tab, bytes;
+};
+__host__ __device__ inline SgLayout sg_layout(int cap, int maxu, int lc, int xb) {
+    SgLayout L;
+    size_t o = 0;
+    L.xs = o, o += sizeof(double) * size_t(lc) * xb;
+    L.hk = o, o += sizeof(int32_t) * size_t(cap);
+    L.hv = o, o += sizeof(int32_t) * size_t(cap);
+    L.ul = o, o += sizeof(int32_t) * size_t(maxu);
+    L.us = o, o += sizeof(int32_t) * size_t(maxu);
+    L.mk = o, o += sizeof(uint32_t) * size_t(maxu);
+    L.nu = o, o += sizeof(int32_t) * 2;
+    L.ts = o, o += sizeof(int32_t) * size_t(lc);
+    L.tab = o, o += sizeof(uint16_t) * size_t(lc) * maxu;
+    L.bytes = (o + 15) & ~size_t(15);
+    return L;
+}
+
+template <int B>
+__global__ void __launch_bounds__(kT) k_sg_fill_wide(int64_t n, const int32_t* __restrict__ xptr,
+                                                     const int32_t* __restrict__ xcol, const double* __restrict__ xval,
+                                                     const int32_t* __restrict__ yptr,
+                                                     const int32_t* __restrict__ ycol, const double* __restrict__ yval,
+                                                     int cap, int lg, int maxu, int lc, int splits,
+                                                     const int32_t* __restrict__ zptr, int32_t* zcol, double* zval,
+                                                     int* status) {
+    constexpr int BB = B * B, kU = 4;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const SgLayout Ls = sg_layout(cap, maxu, lc, BB);
+    double* xs = reinterpret_cast<double*>(smem + Ls.xs);
+    int32_t* hk = reinterpret_cast<int32_t*>(smem + Ls.hk);
+    int32_t* hv = reinterpret_cast<int32_t*>(smem + Ls.hv);
+    int32_t* ul = reinterpret_cast<int32_t*>(smem + Ls.ul);
+    int32_t* us = reinterpret_cast<int32_t*>(smem + Ls.us);
+    uint32_t* mk = reinterpret_cast<uint32_t*>(smem + Ls.mk);
+    int32_t* nu = reinterpret_cast<int32_t*>(smem + Ls.nu);   // distinct columns, "row is bad"
+    int32_t* ts = reinterpret_cast<int32_t*>(smem + Ls.ts);   // first block of each entry's Y row
+    uint16_t* tab = reinterpret_cast<uint16_t*>(smem + Ls.tab);
+    for (int64_t w = blockIdx.x; w < n * splits; w += gridDim.x) {
+        const int64_t i = w / splits;
+        const int part = int(w - i * splits);
+        __syncthreads();   // the row before is done with the tables
+        for (int q = tid; q < cap; q += kT) hk[q] = -1;
+        if (tid < 2) nu[tid] = 0;
+        __syncthreads();
+        const int xs0 = xptr[i], Lx = xptr[i + 1] - xs0;
+        for (int l = warp; l < Lx; l += kWarps) {
+            const int kk = xcol[xs0 + l];
+            for (int t = yptr[kk] + lane; t < yptr[kk + 1]; t += 32) {
+                bool fresh = false;
+                const int h = hinsert(hk, cap, lg, ycol[t], &fresh);
+                if (h < 0) {
+                    nu[1] = 1;
+                } else if (fresh) {
+                    const int u = atomicAdd(nu, 1);
+                    if (u < maxu) {
+                        ul[u] = ycol[t];
+                        us[u] = h;
+                    } else {
+                        nu[1] = 1;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        const int U = nu[0], zs = zptr[i];
+        if (nu[1] || U != zptr[i + 1] - zs) {   // uniform over the block
+            if (tid == 0) atomicOr(status, 4);
+            continue;
+        }
+        for (int u = tid; u < U; u += kT) {
+            const int32_t key = ul[u];
+            int rk = 0;
+            for (int p = 0; p < U; ++p) rk += ul[p] < key ? 1 : 0;
+            hv[us[u]] = rk;
+            if (part == 0) zcol[zs + rk] = key;
+        }
+        const int it0 = int(int64_t(U) * part / splits) * BB, it1 = int(int64_t(U) * (part + 1) / splits) * BB;
+        for (int l0 = 0; l0 < Lx; l0 += lc) {
+            const int nl = min(lc, Lx - l0);
+            __syncthreads();   // ranks written; the chunk before is done with tab and xs
+            for (int u = tid; u < U; u += kT) mk[u] = 0u;
+            for (int q = tid; q < nl * BB; q += kT) xs[q] = xval[int64_t(xs0 + l0) * BB + q];
+            __syncthreads();
+            for (int l = warp; l < nl; l += kWarps) {
+                const int kk = xcol[xs0 + l0 + l], t0 = yptr[kk], Lk = yptr[kk + 1] - t0;
+                if (lane == 0) ts[l] = t0;
+                for (int t = lane; t < Lk; t += 32) {
+                    const int h = hfind(hk, cap, lg, ycol[t0 + t]);
+                    if (h >= 0) {
+                        tab[l * U + hv[h]] = uint16_t(t);
+                        atomicOr(mk + hv[h], 1u << l);
+                    } else {
+                        atomicOr(status, 4);
+                    }
+                }
+            }
+            __syncthreads();
+            for (int it = it0 + tid; it < it1; it += kT) {
+                const int u = it / BB, e = it - u * BB, r = e / B, c = e - r * B;
+                double* z = zval + int64_t(zs) * BB + it;
+                double acc = l0 ? *z : 0.0;
+                uint32_t m = mk[u];
+                while (m) {
+                    int l[kU];
+                    double y[kU][B];
+#pragma unroll
+                    for (int j = 0; j < kU; ++j) {
+                        l[j] = __ffs(int(m)) - 1;   // -1: no entry left
+                        m &= m - 1u;
+                        if (l[j] >= 0) {
+                            const double* yb = yval + int64_t(ts[l[j]] + int(tab[l[j] * U + u])) * BB + c;
+#pragma unroll
+                            for (int q = 0; q < B; ++q) y[j][q] = __ldg(yb + q * B);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kU; ++j)
+                        if (l[j] >= 0) {
+                            const double* xb = xs + l[j] * BB + r * B;
+#pragma unroll
+                            for (int q = 0; q < B; ++q) acc = fma(xb[q], y[j][q], acc);
+                        }
+                }
+                *z = acc;
+            }
+        }
+    }
+}
+
 // coarse DOF whose prolongator column is zero have an exactly zero row and column: unit diagonal
 template <int B>
 __global__ void k_unit_diag(int64_t n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
@@ -737,16 +1041,22 @@ __global__ void k_unit_diag(int64_t n, const int32_t* __restrict__ ptr, const in
 }
 
 // ---- FP32 copies for the V-cycle ---------------------------------------------------------------
-__global__ void k_f32_layouts(int64_t n, const int32_t* __restrict__ ptr, const double* __restrict__ v64, int bb,
-                              float* soa, float* blk) {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t rs = ptr[i], L = ptr[i + 1] - rs;
-        for (int64_t l = 0; l < L; ++l)
-            for (int q = 0; q < bb; ++q) {
-                const float f = float(v64[(rs + l) * bb + q]);
-                soa[bb * rs + q * L + l] = f;
-                blk[(rs + l) * bb + q] = f;
-            }
+// One warp per block row, lanes over its values in block order: the FP64 reads and the block-major
+// writes are coalesced (one thread per row, one value at a time, took 1.47 ms a matrix where this
+// takes 0.15); the row-SoA writes scatter within the row and merge in L2.
+__global__ void __launch_bounds__(kT) k_f32_layouts(int64_t n, const int32_t* __restrict__ ptr,
+                                                    const double* __restrict__ v64, int bb, float* soa, float* blk) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+        const int64_t rs = ptr[i];
+        const int L = ptr[i + 1] - int(rs);
+        for (int o = lane; o < L * bb; o += 32) {
+            const int l = o / bb, q = o - l * bb;
+            const float f = float(v64[rs * bb + o]);
+            blk[rs * bb + o] = f;
+            soa[bb * rs + int64_t(q) * L + l] = f;
+        }
     }
 }
 
@@ -784,7 +1094,9 @@ struct Setup {
             FEM_TRY(parts.alloc(sizeof(double) * nc));
             parts_n = size_t(nc);
         }
-        k_chunk_sums<<<grid(nc, 64), 64, 0, st>>>(N, a, b, stride, off, parts.as<double>());
+        const size_t smem = sizeof(double) * 32 * (kSumChunk + 1);
+        FEM_CUDA(cudaFuncSetAttribute(k_chunk_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        k_chunk_sums<<<unsigned((nc + 31) / 32), kT, smem, st>>>(N, a, b, stride, off, parts.as<double>());
         FEM_LAUNCH_CHECK("k_chunk_sums");
         std::vector<double> h;
         FEM_TRY(down(h, parts.as<const double>(), size_t(nc)));
@@ -902,17 +1214,35 @@ int spgemm(Setup& S, const View& X, const View& Y, Mat& Z) {
     while ((1 << lg) < 2 * maxu) ++lg;
     cap = 1 << lg;
     maxu = std::max(maxu, 1);
-    const size_t per = sizeof(int32_t) * (2 * size_t(cap) + 2 * size_t(maxu) + size_t(maxyl) + 1);
-    int warps = kWarps;
-    while (warps > 1 && per * warps > 200 * 1024) warps >>= 1;
-    FEM_REQUIRE(per * warps <= 220 * 1024, "AMG device setup: a product row needs %zu bytes of shared memory", per);
-    auto kern = k_sg_fill<BI, BK, BJ>;
-    FEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * warps)));
     FEM_CUDA(cudaMemsetAsync(S.status.p, 0, sizeof(int), S.st));
-    kern<<<grid(X.n, warps), 32 * warps, per * warps, S.st>>>(X.n, X.ptr, X.col, X.val, Y.ptr, Y.col, Y.val, cap, lg,
-                                                               maxu, maxyl, warps, Z.P(), Z.col.as<int32_t>(),
-                                                               Z.val.as<double>(), S.status.as<int>());
-    FEM_LAUNCH_CHECK("k_sg_fill");
+    if constexpr (BI == kModes && BK == kModes && BJ == kModes) {
+        FEM_REQUIRE(maxyl <= 0xffff, "AMG device setup: a row has %d blocks", maxyl);
+        int lc = 32;  // a bit of the column masks each
+        while (lc > 4 && sg_layout(cap, maxu, lc, kModes * kModes).bytes > 72 * 1024) lc >>= 1;
+        const size_t bytes = sg_layout(cap, maxu, lc, kModes * kModes).bytes;
+        FEM_REQUIRE(bytes <= 220 * 1024, "AMG device setup: a product row needs %zu bytes of shared memory", bytes);
+        // at least four blocks per SM, so that the last wave is a small part of the whole
+        const int64_t want = int64_t(sm_count()) * 4;
+        const int splits = int(std::max<int64_t>(1, std::min<int64_t>(8, want / std::max<int64_t>(X.n, 1))));
+        auto kern = k_sg_fill_wide<kModes>;
+        FEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+        kern<<<grid(X.n * splits, 1), kT, bytes, S.st>>>(X.n, X.ptr, X.col, X.val, Y.ptr, Y.col, Y.val, cap, lg, maxu,
+                                                         lc, splits, Z.P(), Z.col.as<int32_t>(), Z.val.as<double>(),
+                                                         S.status.as<int>());
+        FEM_LAUNCH_CHECK("k_sg_fill_wide");
+    } else {
+        const size_t per = sizeof(int32_t) * (2 * size_t(cap) + 2 * size_t(maxu) + size_t(maxyl) + 1);
+        int warps = kWarps;
+        while (warps > 1 && per * warps > 200 * 1024) warps >>= 1;
+        FEM_REQUIRE(per * warps <= 220 * 1024, "AMG device setup: a product row needs %zu bytes of shared memory", per);
+        auto kern = k_sg_fill<BI, BK, BJ>;
+        FEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * warps)));
+        kern<<<grid(X.n, warps), 32 * warps, per * warps, S.st>>>(X.n, X.ptr, X.col, X.val, Y.ptr, Y.col, Y.val, cap,
+                                                                   lg, maxu, maxyl, warps, Z.P(),
+                                                                   Z.col.as<int32_t>(), Z.val.as<double>(),
+                                                                   S.status.as<int>());
+        FEM_LAUNCH_CHECK("k_sg_fill");
+    }
     FEM_CUDA(cudaMemcpyAsync(&status, S.status.p, sizeof(int), cudaMemcpyDeviceToHost, S.st));
     FEM_TRY(S.sync());
     FEM_REQUIRE(!(status & 4), "AMG device setup: inconsistent product row (internal error)");
@@ -965,7 +1295,7 @@ int to_devbsr(Setup& S, const View& M, DevBsr& D) {
     FEM_CUDA(cudaMemcpyAsync(D.ptr, M.ptr, sizeof(int32_t) * (M.n + 1), cudaMemcpyDeviceToDevice, S.st));
     if (M.nnzb)
         FEM_CUDA(cudaMemcpyAsync(D.col, M.col, sizeof(int32_t) * M.nnzb, cudaMemcpyDeviceToDevice, S.st));
-    k_f32_layouts<<<grid(M.n, kT), kT, 0, S.st>>>(M.n, M.ptr, M.val, int(bb), D.val, D.valb);
+    k_f32_layouts<<<grid(M.n, kWarps), kT, 0, S.st>>>(M.n, M.ptr, M.val, int(bb), D.val, D.valb);
     FEM_LAUNCH_CHECK("k_f32_layouts");
     return FEM_OK;
 }
@@ -1120,7 +1450,7 @@ int level_kernels(Setup& S, fem_amg* H, int l, const View& A, const double* Bnul
             std::vector<double> alpha, beta(1, 0.0);
             const int steps = std::max(2, o.eig_steps);
             for (int j = 0; j < steps; ++j) {
-                k_spmv64<B><<<grid(n, kT), kT, 0, S.st>>>(n, A.ptr, A.col, A.val, pv, u.as<double>());
+                k_spmv64<B><<<grid(n * B, 128), 128, 0, S.st>>>(n, A.ptr, A.col, A.val, pv, u.as<double>());
                 FEM_LAUNCH_CHECK("k_spmv64");
                 double a = 0.0;
                 FEM_TRY(S.dot(N, pv, u.as<double>(), a));
@@ -1167,8 +1497,22 @@ int level_kernels(Setup& S, fem_amg* H, int l, const View& A, const double* Bnul
     FEM_TRY(Bnext.alloc(sizeof(double) * na * kModes * kModes));
     FEM_TRY(S.up(daptr.as<int32_t>(), aptr));
     FEM_TRY(S.up(dmem.as<int32_t>(), mem));
-    k_tentative<B><<<grid(na, 64), 64, 0, S.st>>>(na, daptr.as<int32_t>(), dmem.as<int32_t>(), Bnull_in,
-                                                   T.as<double>(), Bnext.as<double>());
+    {
+        int rows_cap = 0;   // rows of the largest aggregate
+        for (int64_t a = 0; a < na; ++a) rows_cap = std::max(rows_cap, (aptr[a + 1] - aptr[a]) * B);
+        const size_t per = sizeof(double) * kModes * size_t(rows_cap);
+        if (4 * per <= 200 * 1024) {
+            int threads = 32;
+            while (threads > 4 && per * threads > 100 * 1024) threads >>= 1;
+            auto kern = k_tentative<B, true>;
+            FEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * threads)));
+            kern<<<grid(na, threads), threads, per * threads, S.st>>>(na, daptr.as<int32_t>(), dmem.as<int32_t>(),
+                                                                      Bnull_in, T.as<double>(), Bnext.as<double>());
+        } else {
+            k_tentative<B, false><<<grid(na, 64), 64, 0, S.st>>>(na, daptr.as<int32_t>(), dmem.as<int32_t>(), Bnull_in,
+                                                                  T.as<double>(), Bnext.as<double>());
+        }
+    }
     FEM_LAUNCH_CHECK("k_tentative");
     FEM_TRY(S.sync());
     H->setup_s[1] += since(tt);
@@ -1201,16 +1545,25 @@ int level_kernels(Setup& S, fem_amg* H, int l, const View& A, const double* Bnul
         int maxU = 1;
         FEM_TRY(max_row_len(S, View{n, na, B, kModes, nnz, P.P(), nullptr, nullptr}, maxU));
         maxU = std::max(maxU, 1);
-        const size_t per = size_t(maxU) * B * kModes * sizeof(double) + size_t(maxL + maxU) * sizeof(int32_t) + maxL;
-        const size_t per_al = (per + 15) & ~size_t(15);
+        int p2 = 32;
+        while (p2 < maxL) p2 <<= 1;
+        const bool spill = p2 > 1024;  // 8 KB of a warp's shared memory; meshes give rows of a few hundred
+        const size_t per = prol_row_bytes(spill ? 0 : p2, maxU, B * kModes);
         int warps = kWarps;
-        while (warps > 1 && per_al * warps > 200 * 1024) warps >>= 1;
-        FEM_REQUIRE(per_al * warps <= 220 * 1024, "AMG device setup: level %d needs %zu bytes per prolongator row", l,
-                    per_al);
-        FEM_CUDA(cudaFuncSetAttribute(k_prol_fill<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per_al * warps)));
-        k_prol_fill<B><<<grid(n, warps), 32 * warps, per_al * warps, S.st>>>(
+        while (warps > 1 && per * warps > 200 * 1024) warps >>= 1;
+        FEM_REQUIRE(per * warps <= 220 * 1024, "AMG device setup: level %d needs %zu bytes per prolongator row", l,
+                    per);
+        unsigned blocks = grid(n, warps);
+        DBuf scratch;
+        if (spill) {
+            blocks = std::min(blocks, unsigned(sm_count()) * 2);
+            FEM_TRY(scratch.alloc(size_t(blocks) * warps * p2 * 8));
+        }
+        FEM_CUDA(cudaFuncSetAttribute(k_prol_fill<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * warps)));
+        k_prol_fill<B><<<blocks, 32 * warps, per * warps, S.st>>>(
             n, A.ptr, A.col, A.val, agg.as<int32_t>(), iso.as<uint8_t>(), o.smooth != 0, L.omega, dinv64.as<double>(),
-            T.as<double>(), maxL, maxU, warps, P.P(), P.col.as<int32_t>(), P.val.as<double>());
+            T.as<double>(), p2, maxU, warps, scratch.as<unsigned long long>(), P.P(), P.col.as<int32_t>(),
+            P.val.as<double>());
         FEM_LAUNCH_CHECK("k_prol_fill");
         FEM_TRY(S.sync());
     }
