@@ -50,6 +50,14 @@ int64_t device_scan_tiles(int64_t n);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// x or -x by a sign-bit flip: integer work, where `flag ? o - x : o + x` costs two FP64 instructions
+// and a select.
+#ifdef __CUDACC__
+__device__ __forceinline__ double flip_sign(double x, bool flag) {
+    return __hiloint2double(__double2hiint(x) ^ (flag ? int(0x80000000u) : 0), __double2loint(x));
+}
+#endif
+
 // Gauss abscissa exactly as the reference literal (FEM_model_bsr.py:97).
 constexpr double kGS1 = 0.57735026918962;
 

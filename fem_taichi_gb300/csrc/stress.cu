@@ -1,21 +1,24 @@
 // Nodal stress recovery for sm_103a (POST_process.py:72-99, 172-223).
 //
-//  1. k_stress_element -- 8 threads per element.  Thread t first forms coefficient t of the
-//     trilinear interpolants of the element-local coordinates and of the displacements
-//     (c_k = 1/8 sum_a m_k(corner a) v_a for the monomials 1, xi, eta, zeta, xi eta, eta zeta,
-//     xi zeta, xi eta zeta), so that J and dU/dxi at a Gauss point cost 27 FMA each instead
-//     of 72.  Thread g then evaluates the displacement
-//     gradient at Gauss point g as H = (sum_a u_a (x) dN_a/dxi) . adj(J) / det, and the
+//  1. k_stress_element -- 8 threads per element, an element's threads in one warp.  Thread t
+//     loads corner t; a Walsh transform over the 8 lanes gives the trilinear coefficients of the
+//     element-local coordinates and displacements (c_k = 1/8 sum_a m_k(corner a) v_a for the monomials
+//     1, xi, eta, zeta, xi eta, eta zeta, xi zeta, xi eta zeta).  Thread g then evaluates J and
+//     dU/dxi at Gauss point g -- d/dxi does not depend on xi, so the two lanes that share it compute
+//     half of it each, and so for eta and zeta -- the displacement
+//     gradient H = (sum_a u_a (x) dN_a/dxi) . adj(J) / det, and the
 //     stresses  sigma_n = D0 (H00, H11, H22),  sigma_s = mu (H01+H10, H12+H21, H02+H20)
 //     (components xy, yz, xz as UnitVectorS orders them, POST_process.py:190-209).
 //     Corner j's extrapolated value is sum_k W[j][k] sigma(k) with the caller's 8x8 weight
 //     table (get_NdSol / shapefunc_GS, POST_process.py:172-181, 212-223); the dot products of
 //     the table's distinct rows are spread over the element's threads, and thread j writes
-//     corner j's values to the per-element workspace.
+//     corner j's values to the per-element workspace.  Bound by the FP64 pipe (one warp instruction
+//     per 16 cycles per SM), so shuffles and selects are spent to save FP64 instructions: about
+//     130 per thread, 200 before (960,000 elements: 2.55 -> 1.76 ms, the pipe 90 % busy in both).
 //  2. k_stress_node -- one thread per node: sums its incident (element, corner) values in
 //     ascending element order (no atomics), divides by the element count (get_NdAve,
 //     :183-187; one reciprocal, six products; an isolated node stays 0 * inf = NaN), then
-//     computes the principal stresses with cyclic Jacobi rotations (descending order) and the
+//     computes the principal stresses (descending order; sym3_eig_desc) and the
 //     reference's "VM" formula as written (:93-94).
 #include <cstring>
 #include <mutex>
@@ -36,7 +39,7 @@ struct StressParams {
     const double* u;
     int64_t n_elem;
     double* rec;  // [n_elem][8][6]
-    double D0d, lam, mu;
+    double lm, mu;   // lam / mu, mu
     double W[8][8];  // the distinct rows of the caller's extrapolation table
     int nrow;        // how many
     int row_of[8];   // corner j -> its row of W
@@ -45,87 +48,70 @@ struct StressParams {
 struct StressSmem {
     double W[8][8];
     double res[kEpc][8][6];  // extrapolated values of each distinct table row
-    double x[kEpc][8][3];
-    double u[kEpc][8][3];
-    double cx[kEpc][8][3];  // trilinear coefficients of the element-local coordinates
-    double cu[kEpc][8][3];  // and of the displacements
+    double cf[kEpc][8][7];   // Walsh sums of the coordinates and displacements
     double sv[kEpc][8][kSvPad];
 };
 
-// m_k(corner a) of the trilinear monomials (1, xi, eta, zeta, xi eta, eta zeta, xi zeta,
-// xi eta zeta) at the reference's corner order (POST_process.py:238-273): xi < 0 at corners
-// 1, 2, 5, 6 (0x66), eta < 0 at 2, 3, 6, 7 (0xCC), zeta < 0 at 0-3 (0x0F); monomial k holds
-// xi for k in {1, 4, 6, 7} (0xD2), eta for {2, 4, 5, 7} (0xB4), zeta for {3, 5, 6, 7} (0xE8).
-__device__ __forceinline__ double monomial_sign(int k, int a) {
-    const int neg = (((0xD2 >> k) & (0x66 >> a)) ^ ((0xB4 >> k) & (0xCC >> a)) ^ ((0xE8 >> k) & (0x0F >> a))) & 1;
-    return neg ? -1.0 : 1.0;
-}
-
-// d/dxi, d/deta, d/dzeta of sum_k c_k m_k at (xi, eta, zeta) for one component
-__device__ __forceinline__ void trilinear_grad(const double (*c)[3], int i, double xi, double et, double ze,
-                                               double& d0, double& d1, double& d2) {
-    const double c1 = c[1][i], c2 = c[2][i], c3 = c[3][i], c4 = c[4][i], c5 = c[5][i], c6 = c[6][i], c7 = c[7][i];
-    d0 = fma(ze, fma(et, c7, c6), fma(et, c4, c1));
-    d1 = fma(ze, fma(xi, c7, c5), fma(xi, c4, c2));
-    d2 = fma(et, fma(xi, c7, c5), fma(xi, c6, c3));
-}
-
 __global__ void __launch_bounds__(kThreads) k_stress_element(const StressParams p) {
     __shared__ StressSmem s;
+    const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x;
     const int el = tid >> 3;
     const int t = tid & 7;
-    const int64_t e = int64_t(blockIdx.x) * kEpc + el;
-    const bool valid = e < p.n_elem;
+    const int64_t e_raw = int64_t(blockIdx.x) * kEpc + el;
+    const bool valid = e_raw < p.n_elem;
+    const int64_t e = valid ? e_raw : p.n_elem - 1;   // the lanes of absent elements repeat the last one
     for (int k = tid; k < 64; k += kThreads) (&s.W[0][0])[k] = (&p.W[0][0])[k];
-    if (valid) {
-        const int node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
+    double c[6];
+    {
+        const int64_t node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            s.x[el][t][i] = __ldg(p.xyz + 3 * int64_t(node) + i);
-            s.u[el][t][i] = __ldg(p.u + 3 * int64_t(node) + i);
+            c[i] = __ldg(p.xyz + 3 * node + i);
+            c[3 + i] = __ldg(p.u + 3 * node + i);
         }
     }
-    __syncthreads();
-    // element-local values (corner 0 subtracted; the gradients depend on differences only)
-    double x0[3] = {0, 0, 0}, u0[3] = {0, 0, 0};
-    if (valid) {
+    // element-local values (corner 0 subtracted; the gradients depend on differences only), then
+    // Walsh sums over the corners, W_s = sum_a (-1)^popc(s & a) v_a on lane s.  The natural
+    // coordinates are negative at corners {1,2,5,6} (xi), {2,3,6,7} (eta), {0,1,2,3} (zeta), so the
+    // coefficients are xi: W_3, eta: W_2, zeta: -W_4, xi eta: W_1, eta zeta: -W_6, xi zeta: -W_7,
+    // xi eta zeta: -W_5 (POST_process.py:238-273 for the corner order).  The 1 / 8 of a coefficient
+    // cancels in G adj(J) / det: J and G stay 8 times theirs.
 #pragma unroll
-        for (int i = 0; i < 3; ++i) x0[i] = s.x[el][0][i], u0[i] = s.u[el][0][i];
-    }
-    __syncthreads();
-    if (valid) {
+    for (int i = 0; i < 6; ++i) c[i] -= __shfl_sync(full, c[i], tid & 24);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            s.x[el][t][i] -= x0[i];
-            s.u[el][t][i] -= u0[i];
+    for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const double o = __shfl_xor_sync(full, c[i], m);
+            c[i] = o + flip_sign(c[i], t & m);
         }
-    }
-    __syncthreads();
-    if (valid) {
-        // coefficient t of the interpolants (corner 0 is now zero)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            double ax = 0.0, au = 0.0;
-#pragma unroll
-            for (int a = 1; a < 8; ++a) {
-                const double m = monomial_sign(t, a);
-                ax = fma(m, s.x[el][a][i], ax);
-                au = fma(m, s.u[el][a][i], au);
-            }
-            s.cx[el][t][i] = 0.125 * ax;
-            s.cu[el][t][i] = 0.125 * au;
-        }
-    }
-    __syncthreads();
-    if (valid) {
+    for (int i = 0; i < 6; ++i) s.cf[el][t][i] = flip_sign(c[i], t & 4);
+    __syncthreads();  // the weight table is shared by the block's warps
+    {
         const int g = t;
         const double xi = (g & 4) ? kGS1 : -kGS1, et = (g & 2) ? kGS1 : -kGS1, ze = (g & 1) ? kGS1 : -kGS1;
+        // J (components 0-2) and G = dU/dxi (3-5): column d is the same on the two lanes that differ
+        // in direction d only; the lane on the negative side forms J's column, the other G's, and
+        // they swap.
+        const int hx = (g & 4) ? 3 : 0, he = (g & 2) ? 3 : 0, hz = (g & 1) ? 3 : 0;
         double J[3][3], G[3][3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            trilinear_grad(s.cx[el], i, xi, et, ze, J[i][0], J[i][1], J[i][2]);
-            trilinear_grad(s.cu[el], i, xi, et, ze, G[i][0], G[i][1], G[i][2]);
+            const double(*f)[7] = s.cf[el];
+            const double x0 = fma(ze, fma(et, f[5][hx + i], f[7][hx + i]), fma(et, f[1][hx + i], f[3][hx + i]));
+            const double y0 = fma(ze, fma(xi, f[5][he + i], f[6][he + i]), fma(xi, f[1][he + i], f[2][he + i]));
+            const double z0 = fma(et, fma(xi, f[5][hz + i], f[6][hz + i]), fma(xi, f[7][hz + i], f[4][hz + i]));
+            const double x1 = __shfl_xor_sync(full, x0, 4);
+            const double y1 = __shfl_xor_sync(full, y0, 2);
+            const double z1 = __shfl_xor_sync(full, z0, 1);
+            J[i][0] = hx ? x1 : x0;
+            G[i][0] = hx ? x0 : x1;
+            J[i][1] = he ? y1 : y0;
+            G[i][1] = he ? y0 : y1;
+            J[i][2] = hz ? z1 : z0;
+            G[i][2] = hz ? z0 : z1;
         }
         double A[3][3];
 #pragma unroll
@@ -136,40 +122,50 @@ __global__ void __launch_bounds__(kThreads) k_stress_element(const StressParams 
                 A[j][i] = J[i1][j1] * J[i2][j2] - J[i2][j1] * J[i1][j2];
             }
         const double det = J[0][0] * A[0][0] + J[1][0] * A[0][1] + J[2][0] * A[0][2];
-        const double inv = 1.0 / det;
-        double H[3][3];  // du_i/dx_k
+        const double mi = p.mu * (1.0 / det);
+        // h = det times du_i/dx_i and du_i/dx_k + du_k/dx_i
+        double h[6];
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 3; ++i) {
+            const int k = (i + 1) % 3;
+            h[i] = fma(G[i][2], A[2][i], fma(G[i][1], A[1][i], G[i][0] * A[0][i]));
+            h[3 + i] = fma(G[k][2], A[2][i], fma(G[k][1], A[1][i], fma(G[k][0], A[0][i],
+                       fma(G[i][2], A[2][k], fma(G[i][1], A[1][k], G[i][0] * A[0][k])))));
+        }
+        const double tr = p.lm * (h[0] + h[1] + h[2]);   // sigma = mu (2 H + (lam / mu) tr H I)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) H[i][k] = (G[i][0] * A[0][k] + G[i][1] * A[1][k] + G[i][2] * A[2][k]) * inv;
-        const double D0d = p.D0d, lam = p.lam, mu = p.mu;
-        s.sv[el][g][0] = D0d * H[0][0] + lam * (H[1][1] + H[2][2]);
-        s.sv[el][g][1] = D0d * H[1][1] + lam * (H[0][0] + H[2][2]);
-        s.sv[el][g][2] = D0d * H[2][2] + lam * (H[0][0] + H[1][1]);
-        s.sv[el][g][3] = mu * (H[0][1] + H[1][0]);
-        s.sv[el][g][4] = mu * (H[1][2] + H[2][1]);
-        s.sv[el][g][5] = mu * (H[0][2] + H[2][0]);
+        for (int i = 0; i < 3; ++i) {
+            s.sv[el][g][i] = mi * fma(2.0, h[i], tr);
+            s.sv[el][g][3 + i] = mi * h[3 + i];
+        }
     }
-    __syncthreads();
+    __syncwarp();
     // Extrapolation: the table's distinct rows only (the reference's aliased GMat gives every
     // even corner one row and every odd corner another: 12 dot products per element instead of
     // 48), spread over the element's 8 threads; corner j then takes its row's values.
-    if (valid) {
-        const int nout = p.nrow * 6;
-        for (int o = t; o < nout; o += 8) {
-            const int r = o / 6, c = o - 6 * r;
-            double acc = 0.0;
+    const int nout = p.nrow * 6;
+    for (int o0 = 0; o0 < nout; o0 += 8) {
+        const bool half = nout - o0 == 4;   // the last four outputs: two threads each, four Gauss points a thread
+        const int o = half ? o0 + (t >> 1) : o0 + t, k0 = half ? 4 * (t & 1) : 0;
+        if (o >= nout) break;
+        const int r = o / 6, cc = o - 6 * r;
+        double acc = 0.0;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) acc = fma(s.W[r][k], s.sv[el][k][c], acc);
-            s.res[el][r][c] = acc;
+        for (int k = 0; k < 4; ++k) acc = fma(s.W[r][k0 + k], s.sv[el][k0 + k][cc], acc);
+        if (half) {
+            acc += __shfl_xor_sync(full, acc, 1);
+        } else {
+#pragma unroll
+            for (int k = 4; k < 8; ++k) acc = fma(s.W[r][k], s.sv[el][k][cc], acc);
         }
+        s.res[el][r][cc] = acc;
     }
-    __syncthreads();
+    __syncwarp();
     if (!valid) return;
-    const int j = t, r = p.row_of[j];
-    double* o = p.rec + (e * 8 + j) * 6;
+    const double* r = s.res[el][p.row_of[t]];
+    double2* o = reinterpret_cast<double2*>(p.rec + (e * 8 + t) * 6);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) o[c] = s.res[el][r][c];
+    for (int q = 0; q < 3; ++q) o[q] = make_double2(r[2 * q], r[2 * q + 1]);
 }
 
 // Eigenvalues of the symmetric 3x3 [[a00,a01,a02],[a01,a11,a12],[a02,a12,a22]] by cyclic
@@ -180,7 +176,7 @@ __global__ void __launch_bounds__(kThreads) k_stress_element(const StressParams 
 // rotation would move the diagonal by about a_pq^2 / (a_qq - a_pp) -- which ends a 3 x 3 in
 // about three sweeps instead of five; c = rsqrt(1 + t^2); capped at 32 sweeps; returned
 // descending.
-__device__ void sym3_eig_desc(double a00, double a11, double a22, double a01, double a12, double a02,
+__device__ __noinline__ void sym3_eig_jacobi(double a00, double a11, double a22, double a01, double a12, double a02,
                               double& p1, double& p2, double& p3) {
     double d[3] = {a00, a11, a22};
     double o01 = a01, o02 = a02, o12 = a12;
@@ -227,6 +223,130 @@ __device__ void sym3_eig_desc(double a00, double a11, double a22, double a01, do
     p3 = e2;
 }
 
+// Eigenvalues, descending, of a symmetric 3x3 (the same entries as sym3_eig_jacobi) with few FP64
+// instructions: the FP32 pipes find the eigenvectors, FP64 only applies and corrects them.
+//  1. Cyclic Jacobi in FP32 accumulates its rotations in a quaternion q (components of 24 bits).
+//  2. R(q) is |q|^2 times an orthogonal matrix whatever q is, so B = R^T A R / |q|^4 has A's
+//     eigenvalues to FP64 rounding; its off-diagonals are FP32 noise, ~1e-7 |A|.
+//  3. Jacobi rotations in FP64 with tan(phi) = t from FP32.  The rotation is orthogonal for any t
+//     (c = 1 / sqrt(1 + t^2) refined to FP64), and what an inexact t leaves is carried, not dropped:
+//     each sweep takes the off-diagonals down by another ~1e-7, so one sweep serves separated
+//     eigenvalues (the neglected shift e^2 / gap is below 1e-18 |A|) and two serve equal ones.
+// About 150 FP64 instructions against 630 of the Jacobi form (no FP64 division or square root):
+// k_stress_node on 1,010,025 nodes 1.37 -> 0.45 ms.  A matrix outside the FP32 range, or with an
+// infinity or NaN, takes sym3_eig_jacobi.
+__device__ __forceinline__ float tan_rotation(float h, float apq) {  // h = a_qq - a_pp
+    const float theta = __fdividef(0.5f * h, apq);
+    const float t = __fdividef(1.f, fabsf(theta) + __fsqrt_rn(fmaf(theta, theta, 1.f)));
+    return fabsf(theta) < 1e18f ? copysignf(t, theta) : __fdividef(apq, h);
+}
+
+__device__ __forceinline__ void sym3_eig_desc(double a00, double a11, double a22, double a01, double a12, double a02,
+                                              double& p1, double& p2, double& p3) {
+    float f00 = float(a00), f11 = float(a11), f22 = float(a22), f01 = float(a01), f12 = float(a12), f02 = float(a02);
+    const float m = fmaxf(fmaxf(fabsf(f00), fabsf(f11)), fmaxf(fabsf(f22), fmaxf(fabsf(f01), fmaxf(fabsf(f12), fabsf(f02)))));
+    const float any = fabsf(f00) + fabsf(f11) + fabsf(f22) + fabsf(f01) + fabsf(f12) + fabsf(f02);
+    if (!(m > 1e-18f && any < 1e18f)) {   // also NaN, and the zero matrix
+        sym3_eig_jacobi(a00, a11, a22, a01, a12, a02, p1, p2, p3);
+        return;
+    }
+    float qw = 1.f, qx = 0.f, qy = 0.f, qz = 0.f;
+    for (int sweep = 0; sweep < 6; ++sweep) {
+        const float off = fabsf(f01) + fabsf(f02) + fabsf(f12);
+        if (!(off > 3e-8f * m)) break;
+#pragma unroll
+        for (int pq = 0; pq < 3; ++pq) {   // (p, q): (0, 1), (0, 2), (1, 2)
+            float& apq = pq == 0 ? f01 : pq == 1 ? f02 : f12;
+            float& app = pq == 2 ? f11 : f00;
+            float& aqq = pq == 0 ? f11 : f22;
+            float& x = pq == 0 ? f02 : f01;   // (p, r)
+            float& y = pq == 2 ? f02 : f12;   // (q, r)
+            if (fabsf(apq) <= 1e-9f * m) continue;
+            const float t = tan_rotation(aqq - app, apq);
+            const float c = rsqrtf(fmaf(t, t, 1.f)), sn = t * c;
+            app = fmaf(-t, apq, app);
+            aqq = fmaf(t, apq, aqq);
+            apq = 0.f;
+            const float x0 = x, y0 = y;
+            x = c * x0 - sn * y0;
+            y = sn * x0 + c * y0;
+            // half angle; the new axes are p' = c p - sn q, q' = sn p + c q: a turn by -phi about
+            // r for (0, 1) and (1, 2), by +phi for (0, 2)
+            const float hc = __fsqrt_rn(0.5f * (1.f + c));
+            const float hs = (pq == 1 ? 0.5f : -0.5f) * __fdividef(sn, hc);
+            const float w0 = qw, u0 = qx, v0 = qy, z0 = qz;
+            if (pq == 0) {          // q (hc + hs k)
+                qw = w0 * hc - z0 * hs, qx = u0 * hc + v0 * hs, qy = v0 * hc - u0 * hs, qz = z0 * hc + w0 * hs;
+            } else if (pq == 1) {   // q (hc + hs j)
+                qw = w0 * hc - v0 * hs, qx = u0 * hc - z0 * hs, qy = v0 * hc + w0 * hs, qz = z0 * hc + u0 * hs;
+            } else {                // q (hc + hs i)
+                qw = w0 * hc - u0 * hs, qx = u0 * hc + w0 * hs, qy = v0 * hc + z0 * hs, qz = z0 * hc - v0 * hs;
+            }
+        }
+    }
+    double d0, d1, d2, e01, e02, e12;
+    {
+        const double w = qw, x = qx, y = qy, z = qz, x2 = 2.f * qx, y2 = 2.f * qy, z2 = 2.f * qz;
+        const double ww = w * w, xx = x * x, yy = y * y, zz = z * z;   // exact: 24-bit factors
+        const double a = ww + xx, b = yy + zz, cd = ww - xx, dd = yy - zz;
+        const double wz = w * z2, wy = w * y2, wx = w * x2;
+        const double R[3][3] = {{a - b, fma(x, y2, -wz), fma(x, z2, wy)},
+                                {fma(x, y2, wz), cd + dd, fma(y, z2, -wx)},
+                                {fma(x, z2, -wy), fma(y, z2, wx), cd - dd}};
+        const double eps = (a + b) - 1.0;                          // |q|^2 - 1, FP32 rounding only
+        const double f = fma(eps, fma(3.0, eps, -2.0), 1.0);       // |q|^-4
+        double C[3][3];   // A R
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            C[0][j] = fma(a02, R[2][j], fma(a01, R[1][j], a00 * R[0][j]));
+            C[1][j] = fma(a12, R[2][j], fma(a11, R[1][j], a01 * R[0][j]));
+            C[2][j] = fma(a22, R[2][j], fma(a12, R[1][j], a02 * R[0][j]));
+        }
+        auto dot = [&](int i, int j) { return f * fma(R[2][i], C[2][j], fma(R[1][i], C[1][j], R[0][i] * C[0][j])); };
+        d0 = dot(0, 0), d1 = dot(1, 1), d2 = dot(2, 2), e01 = dot(0, 1), e02 = dot(0, 2), e12 = dot(1, 2);
+    }
+    const float rm = __fdividef(1.f, m);
+    for (int sweep = 0; sweep < 4; ++sweep) {
+        bool turned = false;
+#pragma unroll
+        for (int pq = 0; pq < 3; ++pq) {
+            double& e = pq == 0 ? e01 : pq == 1 ? e02 : e12;
+            double& dp = pq == 2 ? d1 : d0;
+            double& dq = pq == 0 ? d1 : d2;
+            double& x = pq == 0 ? e02 : e01;
+            double& y = pq == 2 ? e02 : e12;
+            const double h = dq - dp;
+            const float ef = float(e), hf = float(h), en = ef * rm;
+            if (!(en * en > 1e-18f * fabsf(hf * rm)) || fabsf(en) < 1e-16f) continue;
+            turned = true;
+            const float tf = tan_rotation(hf, ef), yf = rsqrtf(fmaf(tf, tf, 1.f));
+            const double t = tf, y0 = yf, t2 = t * t;
+            const double r = fma(-(t2 + 1.0), y0 * y0, 1.0);
+            const double c = fma(y0 * r, fma(0.375, r, 0.5), y0), sn = t * c, c2 = c * c;
+            const double dl = t * (c2 * fma(t, h, -2.0 * e));   // a_pp' - a_pp for any t
+            e = c2 * fma(-t, h, fma(-t2, e, e));
+            dp += dl;
+            dq -= dl;
+            const double x0 = x, y1 = y;
+            x = fma(c, x0, -sn * y1);
+            y = fma(sn, x0, c * y1);
+        }
+        if (!turned) break;
+    }
+    double tmp;
+    if (d0 < d1) tmp = d0, d0 = d1, d1 = tmp;
+    if (d1 < d2) tmp = d1, d1 = d2, d2 = tmp;
+    if (d0 < d1) tmp = d0, d0 = d1, d1 = tmp;
+    p1 = d0;
+    p2 = d1;
+    p3 = d2;
+}
+
+// 1 / k for the element counts of a hex mesh's nodes (the same quotients as the division)
+__constant__ double kInverse[17] = {0.0,      1.0 / 1,  1.0 / 2,  1.0 / 3,  1.0 / 4,  1.0 / 5,
+                                    1.0 / 6,  1.0 / 7,  1.0 / 8,  1.0 / 9,  1.0 / 10, 1.0 / 11,
+                                    1.0 / 12, 1.0 / 13, 1.0 / 14, 1.0 / 15, 1.0 / 16};
+
 __global__ void __launch_bounds__(256) k_stress_node(int64_t n_node, const int32_t* __restrict__ ne_ptr,
                                                      const int32_t* __restrict__ ne_list,
                                                      const int32_t* __restrict__ co_elem,
@@ -235,25 +355,40 @@ __global__ void __launch_bounds__(256) k_stress_node(int64_t n_node, const int32
     if (i >= n_node) return;
     double v[6] = {0, 0, 0, 0, 0, 0};
     const int ks = ne_ptr[i], ke = ne_ptr[i + 1];
-    for (int k = ks; k < ke; ++k) {
-        const int ent = __ldg(ne_list + k);
-        const double* r = rec + (int64_t(ent >> 3) * 8 + (ent & 7)) * 6;
+    if (ks < ke) {
+        const double2* r = reinterpret_cast<const double2*>(rec + int64_t(__ldg(ne_list + ks)) * 6);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) v[c] += __ldg(r + c);
+        for (int c = 0; c < 3; ++c) {
+            const double2 x = __ldg(r + c);
+            v[2 * c] = x.x;
+            v[2 * c + 1] = x.y;
+        }
     }
-    const double rce = 1.0 / double(co_elem[i]);
+#pragma unroll 4
+    for (int k = ks + 1; k < ke; ++k) {
+        const double2* r = reinterpret_cast<const double2*>(rec + int64_t(__ldg(ne_list + k)) * 6);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double2 x = __ldg(r + c);
+            v[2 * c] += x.x;
+            v[2 * c + 1] += x.y;
+        }
+    }
+    const int ce = co_elem[i];
+    const double rce = ce > 0 && ce <= 16 ? kInverse[ce] : 1.0 / double(ce);
 #pragma unroll
     for (int c = 0; c < 6; ++c) v[c] *= rce;
     double p1, p2, p3;
     // vector order [xx, yy, zz, xy, yz, xz] (POST_process.py:79-86)
     sym3_eig_desc(v[0], v[1], v[2], v[3], v[4], v[5], p1, p2, p3);
-    double* o = out + 10 * i;
+    double* o = out + 10 * i;   // the caller's: 8-byte alignment only
 #pragma unroll
     for (int c = 0; c < 6; ++c) o[c] = v[c];
     o[6] = p1;
     o[7] = p2;
     o[8] = p3;
-    o[9] = sqrt((p1 - p2) * (p1 - p2) + (p2 - p3) * (p2 - p3) + (p3 - p2) * (p3 - p2));
+    const double d12 = p1 - p2, d23 = p2 - p3;
+    o[9] = sqrt(fma(d12, d12, 2.0 * (d23 * d23)));
 }
 
 }  // namespace
@@ -296,9 +431,8 @@ extern "C" int fem_stress_ex(const fem_mesh* mesh, const fem_material* mat, cons
         sp.n_elem = mesh->n_elem;
         sp.rec = static_cast<double*>(workspace);
         const double EX = mat->EX, PO = mat->PO;
-        sp.D0d = EX * (1 - PO) / (1 + PO) / (1 - 2 * PO);  // POST_process.py:292-302
-        sp.lam = EX * PO / (1 + PO) / (1 - 2 * PO);
-        sp.mu = EX / 2 / (1 + PO);                          // :304-306
+        sp.lm = 2 * PO / (1 - 2 * PO);   // D0 of POST_process.py:292-302 = lam + 2 mu, lam; lam / mu
+        sp.mu = EX / 2 / (1 + PO);       // :304-306
         // distinct rows of the table (exactly equal rows share one)
         std::memset(sp.W, 0, sizeof(sp.W));
         sp.nrow = 0;

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreadsT) k_hex8_tangent(const TangentParams 
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
             const double o = __shfl_xor_sync(full, c[i], m);
-            c[i] = (t & m) ? o - c[i] : o + c[i];
+            c[i] = o + flip_sign(c[i], t & m);
         }
     const double eighth = (t & 4) ? -0.125 : 0.125;
 #pragma unroll
