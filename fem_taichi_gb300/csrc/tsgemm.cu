@@ -4,17 +4,22 @@
 // n x b blocks (b <= 32).  No reference counterpart on the GPU (the reference runs these as
 // numpy GEMMs on the host).
 //
-//  k_ts_tn_partial / k_ts_tn_reduce: C (m x b) = Q^T X, m <= 256.  Persistent CTAs step over
-//    chunks of kChunk rows (a fixed assignment for a given n); a CTA stages the chunk's X rows
-//    in shared memory and thread j accumulates column j of Q (coalesced loads along a row of
-//    Q) against all b columns of X; the per-CTA partials are summed in CTA order by the
-//    reduce kernel (deterministic).
-//  k_ts_nn: W = beta W + alpha Q C (C m x b staged in shared memory): one warp per row, lanes
-//    over the columns of Q's row (coalesced), per-lane partial sums for every output column,
-//    then a butterfly over the warp.
-// FP64 throughout and bound by the FP64 pipe, so the column count of X / W is a template
-// width close to b (4, 8, 10, 12, 16, 24, 32) rather than a power of two: padded columns
-// would be FMAs on zeros.
+//  k_ts_tn_partial / k_ts_tn_reduce: C (m x b) = Q^T X, m <= 256.  CTA k of G takes the rows
+//    [k n / G, (k + 1) n / G) -- the same number to within one, so no SM runs a chunk more than the
+//    others -- in chunks of kChunk; it stages a chunk's X rows in shared memory and thread j
+//    accumulates column j of Q (coalesced loads along a row of Q) against all b columns of X.  The
+//    per-CTA partials are summed in a fixed order (deterministic): kSeg warps of a block each sum
+//    a consecutive share of the CTAs for 32 outputs, loads running ahead, then the shares in order.
+//  k_ts_nn: W = beta W + alpha Q C (C m x b staged in shared memory): one thread per row of Q, which
+//    a warp reads 32 x 32 values at a time, coalesced, into its own shared-memory tile, the next
+//    tile's loads in flight; the row's sums over the columns are b independent chains.
+// FP64 throughout and bound by the FP64 pipe (n m b FMAs each: 199 us at 65,559 x 190 x 10), so the
+// column count of X / W is a template width close to b (4, 8, 10, 12, 16, 24, 32) rather than a
+// power of two: padded columns would be FMAs on zeros.  At that size the products took 251 + 84 us
+// (whole chunks per CTA: 4 on some SMs, 3 on others; one thread summing 513 partials) and 479 us
+// (a warp per row, lanes over the columns: the butterfly adds of 10 sums were as many FP64
+// instructions as the FMAs); now 215 + 15 and
+// 253 us.
 #include <algorithm>
 
 #include "fem_common.cuh"
@@ -22,9 +27,11 @@
 namespace fem {
 namespace {
 
-constexpr int kChunk = 128;    // rows per step of the transposed product
+constexpr int kChunk = 64;     // rows per step of the transposed product
 constexpr int kTsThreads = 256;
 constexpr int kMaxCols = 256;  // columns of Q per launch (one per thread)
+constexpr int kSeg = 8;        // warps that share the sum over the CTAs of one output
+constexpr int kNnThreads = 64;
 
 template <int B>
 __global__ void __launch_bounds__(kTsThreads) k_ts_tn_partial(int64_t n, int m, int b, const double* __restrict__ Q,
@@ -35,8 +42,9 @@ __global__ void __launch_bounds__(kTsThreads) k_ts_tn_partial(int64_t n, int m, 
     double acc[B];
 #pragma unroll
     for (int c = 0; c < B; ++c) acc[c] = 0.0;
-    for (int64_t r0 = int64_t(blockIdx.x) * kChunk; r0 < n; r0 += int64_t(gridDim.x) * kChunk) {
-        const int rows = int(std::min<int64_t>(kChunk, n - r0));
+    const int64_t end = n * (int64_t(blockIdx.x) + 1) / gridDim.x;
+    for (int64_t r0 = n * int64_t(blockIdx.x) / gridDim.x; r0 < end; r0 += kChunk) {
+        const int rows = int(std::min<int64_t>(kChunk, end - r0));
         __syncthreads();
         for (int i = threadIdx.x; i < kChunk * B; i += kTsThreads) {
             const int r = i / B, c = i % B;
@@ -45,6 +53,7 @@ __global__ void __launch_bounds__(kTsThreads) k_ts_tn_partial(int64_t n, int m, 
         __syncthreads();
         if (j < m) {
             const double* q = Q + r0 * ldq + j;
+#pragma unroll 4
             for (int r = 0; r < rows; ++r) {
                 const double qv = __ldg(q + int64_t(r) * ldq);
 #pragma unroll
@@ -59,54 +68,75 @@ __global__ void __launch_bounds__(kTsThreads) k_ts_tn_partial(int64_t n, int m, 
     }
 }
 
-// C[j][c] = sum over CTAs (in order) of the partials
+// C[j][c] = sum over CTAs of the partials: warp w of a block adds the CTAs [w, w + 1) nblocks / kSeg in
+// order for 32 consecutive outputs, then the kSeg sums are added in order.
 template <int B>
-__global__ void k_ts_tn_reduce(int m, int b, int nblocks, const double* __restrict__ part, double* C, int64_t ldc) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m * b) return;
-    const int j = i / b, c = i % b;
+__global__ void __launch_bounds__(kSeg * 32) k_ts_tn_reduce(int m, int b, int nblocks, const double* __restrict__ part,
+                                                             double* C, int64_t ldc) {
+    __shared__ double seg[kSeg][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t total = int64_t(m) * B, i = int64_t(blockIdx.x) * 32 + lane;
     double s = 0.0;
-    for (int k = 0; k < nblocks; ++k) s += part[(int64_t(k) * m + j) * B + c];
+    if (i < total) {
+        const int k1 = nblocks * (w + 1) / kSeg;
+#pragma unroll 8
+        for (int k = nblocks * w / kSeg; k < k1; ++k) s += __ldg(part + int64_t(k) * total + i);
+    }
+    seg[w][lane] = s;
+    __syncthreads();
+    const int j = int(i / B), c = int(i - int64_t(j) * B);
+    if (w || i >= total || c >= b) return;
+#pragma unroll
+    for (int k = 1; k < kSeg; ++k) s += seg[k][lane];
     C[int64_t(j) * ldc + c] = s;
 }
 
 template <int B>
-__global__ void __launch_bounds__(kTsThreads) k_ts_nn(int64_t n, int m, int b, const double* __restrict__ Q,
+__global__ void __launch_bounds__(kNnThreads) k_ts_nn(int64_t n, int m, int b, const double* __restrict__ Q,
                                                         int64_t ldq, const double* __restrict__ C, int64_t ldc,
                                                         double alpha, double beta, double* W, int64_t ldw) {
-    extern __shared__ double cs[];  // [m][B]
-    for (int i = threadIdx.x; i < m * B; i += kTsThreads) {
+    extern __shared__ double cs[];  // [m][B], then a 32 x 33 tile per warp
+    for (int i = threadIdx.x; i < m * B; i += kNnThreads) {
         const int j = i / B, c = i % B;
         cs[i] = c < b ? C[int64_t(j) * ldc + c] : 0.0;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int64_t warp = (int64_t(blockIdx.x) * kTsThreads + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * kTsThreads) >> 5;
-    for (int64_t r = warp; r < n; r += nwarps) {
-        double acc[B];
+    double* tile = cs + m * B + (threadIdx.x >> 5) * (32 * 33);
+    const int64_t groups = (n + 31) / 32, nwarps = (int64_t(gridDim.x) * kNnThreads) >> 5;
+    for (int64_t gr = (int64_t(blockIdx.x) * kNnThreads + threadIdx.x) >> 5; gr < groups; gr += nwarps) {
+        const int64_t r0 = gr * 32;
+        const int rows = int(std::min<int64_t>(32, n - r0));
+        double acc[B], q[32];
 #pragma unroll
         for (int c = 0; c < B; ++c) acc[c] = 0.0;
-        const double* q = Q + r * ldq;
-        for (int j = lane; j < m; j += 32) {
-            const double qv = __ldg(q + j);
+        auto load = [&](int j0) {
+            const double* p = Q + r0 * ldq + j0 + lane;
 #pragma unroll
-            for (int c = 0; c < B; ++c) acc[c] = fma(qv, cs[j * B + c], acc[c]);
+            for (int r = 0; r < 32; ++r) q[r] = r < rows && j0 + lane < m ? __ldg(p + int64_t(r) * ldq) : 0.0;
+        };
+        load(0);
+        for (int j0 = 0; j0 < m; j0 += 32) {
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 32; ++r) tile[r * 33 + lane] = q[r];
+            __syncwarp();
+            if (j0 + 32 < m) load(j0 + 32);
+            const double* cj = cs + j0 * B;
+            const double* tl = tile + lane * 33;
+            const int nj = min(32, m - j0);
+#pragma unroll 2
+            for (int j = 0; j < nj; ++j) {
+                const double qv = tl[j];
+#pragma unroll
+                for (int c = 0; c < B; ++c) acc[c] = fma(qv, cj[j * B + c], acc[c]);
+            }
         }
+        if (lane < rows) {
+            double* w = W + (r0 + lane) * ldw;
 #pragma unroll
-        for (int c = 0; c < B; ++c) {
-            double v = acc[c];
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            acc[c] = v;
-        }
-        if (lane < b) {
-            double v = acc[0];
-#pragma unroll
-            for (int c = 1; c < B; ++c)
-                if (lane == c) v = acc[c];
-            double* w = W + r * ldw + lane;
-            *w = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *w);
+            for (int c = 0; c < B; ++c)
+                if (c < b) w[c] = beta == 0.0 ? alpha * acc[c] : fma(alpha, acc[c], beta * w[c]);
         }
     }
 }
@@ -114,7 +144,8 @@ __global__ void __launch_bounds__(kTsThreads) k_ts_nn(int64_t n, int m, int b, c
 int tn_grid(int64_t n) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return int(std::max<int64_t>(1, std::min<int64_t>((n + kChunk - 1) / kChunk, int64_t(sms) * 4)));
+    // four CTAs an SM; short problems take CTAs of at least 16 rows
+    return int(std::max<int64_t>(1, std::min<int64_t>((n + 15) / 16, int64_t(sms) * 4)));
 }
 
 template <int B>
@@ -123,7 +154,7 @@ int ts_tn(int64_t n, int m, int b, const double* Q, int64_t ldq, const double* X
     const int blocks = tn_grid(n);
     k_ts_tn_partial<B><<<unsigned(blocks), kTsThreads, 0, st>>>(n, m, b, Q, ldq, X, ldx, ws);
     FEM_LAUNCH_CHECK("k_ts_tn_partial");
-    k_ts_tn_reduce<B><<<(m * b + 255) / 256, 256, 0, st>>>(m, b, blocks, ws, C, ldc);
+    k_ts_tn_reduce<B><<<unsigned((int64_t(m) * B + 31) / 32), kSeg * 32, 0, st>>>(m, b, blocks, ws, C, ldc);
     FEM_LAUNCH_CHECK("k_ts_tn_reduce");
     return FEM_OK;
 }
@@ -131,14 +162,12 @@ int ts_tn(int64_t n, int m, int b, const double* Q, int64_t ldq, const double* X
 template <int B>
 int ts_nn(int64_t n, int m, int b, const double* Q, int64_t ldq, const double* C, int64_t ldc, double alpha,
           double beta, double* W, int64_t ldw, cudaStream_t st) {
-    const size_t smem = size_t(m) * B * sizeof(double);
+    const size_t smem = (size_t(m) * B + (kNnThreads / 32) * 32 * 33) * sizeof(double);
     FEM_CUDA(cudaFuncSetAttribute(k_ts_nn<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int dev = 0, sms = 0;
-    FEM_CUDA(cudaGetDevice(&dev));
-    FEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t need = (n * 32 + kTsThreads - 1) / kTsThreads;
-    const unsigned grid = unsigned(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 8)));
-    k_ts_nn<B><<<grid, kTsThreads, smem, st>>>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw);
+    // a warp per 32 rows; every group of rows in one wave where they fit
+    const int64_t need = (n + kNnThreads - 1) / kNnThreads;
+    const unsigned grid = unsigned(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(1) << 20)));
+    k_ts_nn<B><<<grid, kNnThreads, smem, st>>>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw);
     FEM_LAUNCH_CHECK("k_ts_nn");
     return FEM_OK;
 }
