@@ -7,11 +7,12 @@
 //     entries e*8+a, then each node's short list sorted ascending (so the order does not
 //     depend on the atomics); co_elem = distinct elements per node.
 //  2. pattern: one warp per block row gathers the corner nodes of the row's incident
-//     elements (8 per element) into shared memory, sorts them (bitonic, padded to a power of
-//     two) and keeps the distinct ones -> row length; scan -> indptr; the sorted rows are then
-//     compacted into indices.
+//     elements (8 per element), sorts them (bitonic, padded to a power of two; in registers up
+//     to 64, i.e. 8 incident elements, in shared memory beyond) and keeps the distinct ones -> row
+//     length; scan -> indptr; the sorted rows are then compacted into indices.
 //  3. gather map: ne_inv by scatter; slot_map by binary search of each corner's node in the
 //     row of the entry's node.
+// Bound by instruction issue and latency, not bytes (271 MB for 960,000 elements, 40 us).
 #include <climits>
 
 #include "fem_common.cuh"
@@ -132,19 +133,63 @@ __global__ void k_scan_add(int64_t n, const int64_t* __restrict__ tile_sum, int3
         out[i] = int32_t(out[i] + tile_sum[i / kScanTile]);
 }
 
+// Bitonic sort of 64 keys of a warp, element lane in a and element lane + 32 in b.
+__device__ __forceinline__ void sort64(int32_t& a, int32_t& b, int lane) {
+#pragma unroll
+    for (int size = 2; size <= 64; size <<= 1)
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride == 32) {   // the last merge: ascending, both ends in this lane
+                const int32_t lo = min(a, b);
+                b = max(a, b);
+                a = lo;
+            } else {
+                const int32_t oa = __shfl_xor_sync(0xffffffffu, a, stride);
+                const int32_t ob = __shfl_xor_sync(0xffffffffu, b, stride);
+                const bool low = (lane & stride) == 0;
+                // ascending blocks have bit `size` of the element index clear
+                const bool upa = size == 64 || (lane & size) == 0;
+                const bool upb = size == 64 || ((lane + 32) & size) == 0;
+                a = upa == low ? min(a, oa) : max(a, oa);
+                b = upb == low ? min(b, ob) : max(b, ob);
+            }
+        }
+}
+
 // Sorted distinct corner nodes of row i's incident elements -> rows[8 * ne_ptr[i] ...],
 // count -> len[i].  One warp per row.  status bit 1: a row has more than kMaxCand candidates.
+// (All rows sorted in shared memory took 942 us on 1,010,025 nodes, 21 passes of loads, stores and
+// barriers; the register sort of the usual 8-element rows 325 us.)
 __global__ void __launch_bounds__(kRowWarps * 32) k_row_nodes(int64_t n, const int32_t* __restrict__ conn,
                                                               const int32_t* __restrict__ ne_ptr,
                                                               const int32_t* __restrict__ ne_list, int32_t* rows,
                                                               int32_t* len, int* status) {
     __shared__ int32_t buf[kRowWarps][kMaxCand];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
     int32_t* b = buf[w];
     const int64_t nwarps = int64_t(gridDim.x) * kRowWarps;
     for (int64_t i = int64_t(blockIdx.x) * kRowWarps + w; i < n; i += nwarps) {
         const int32_t k0 = ne_ptr[i], k1 = ne_ptr[i + 1];
         const int m = 8 * (k1 - k0);
+        int32_t* out = rows + 8 * int64_t(k0);
+        if (m <= 64) {
+            const int ja = lane, jb = lane + 32;
+            int32_t va = INT_MAX, vb = INT_MAX;
+            if (ja < m) va = __ldg(conn + 8 * int64_t(__ldg(ne_list + k0 + (ja >> 3)) >> 3) + (ja & 7));
+            if (jb < m) vb = __ldg(conn + 8 * int64_t(__ldg(ne_list + k0 + (jb >> 3)) >> 3) + (jb & 7));
+            sort64(va, vb, lane);
+            const int32_t pa = __shfl_up_sync(full, va, 1);
+            const int32_t pb = __shfl_up_sync(full, vb, 1);
+            const int32_t last_a = __shfl_sync(full, va, 31);
+            const bool keep_a = va != INT_MAX && (lane == 0 || va != pa);
+            const bool keep_b = vb != INT_MAX && vb != (lane == 0 ? last_a : pb);
+            const unsigned ma = __ballot_sync(full, keep_a), mb = __ballot_sync(full, keep_b);
+            if (keep_a) out[__popc(ma & below)] = va;
+            if (keep_b) out[__popc(ma) + __popc(mb & below)] = vb;
+            if (lane == 0) len[i] = __popc(ma) + __popc(mb);
+            continue;
+        }
         if (m > kMaxCand) {
             if (lane == 0) {
                 atomicOr(status, 1);
@@ -152,7 +197,7 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_row_nodes(int64_t n, const i
             }
             continue;
         }
-        int p2 = 32;
+        int p2 = 128;
         while (p2 < m) p2 <<= 1;
         for (int j = lane; j < p2; j += 32)
             b[j] = j < m ? __ldg(conn + 8 * int64_t(ne_list[k0 + (j >> 3)] >> 3) + (j & 7)) : INT_MAX;
@@ -175,13 +220,12 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_row_nodes(int64_t n, const i
             }
         }
         // keep the distinct values, in order
-        int32_t* out = rows + 8 * int64_t(k0);
         int written = 0;
         for (int base = 0; base < m; base += 32) {
             const int j = base + lane;
             const bool keep = j < m && (j == 0 || b[j] != b[j - 1]);
-            const unsigned mask = __ballot_sync(0xffffffffu, keep);
-            if (keep) out[written + __popc(mask & ((1u << lane) - 1u))] = b[j];
+            const unsigned mask = __ballot_sync(full, keep);
+            if (keep) out[written + __popc(mask & below)] = b[j];
             written += __popc(mask);
         }
         if (lane == 0) len[i] = written;
@@ -189,40 +233,72 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_row_nodes(int64_t n, const i
     }
 }
 
-__global__ void k_compact_rows(int64_t n, const int32_t* __restrict__ ne_ptr, const int32_t* __restrict__ rows,
-                               const int32_t* __restrict__ indptr, int32_t* indices) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t i = warp0; i < n; i += nw) {
-        const int32_t* src = rows + 8 * int64_t(ne_ptr[i]);
-        const int32_t s = indptr[i], L = indptr[i + 1] - s;
-        for (int l = lane; l < L; l += 32) indices[s + l] = src[l];
+// Rows into indices, 8 lanes a row, four entries a lane in flight (a warp a row left most lanes
+// waiting on one load each: 180 -> 57 us on 1,010,025 nodes).
+__global__ void __launch_bounds__(256) k_compact_rows(int64_t n, const int32_t* __restrict__ ne_ptr,
+                                                      const int32_t* __restrict__ rows,
+                                                      const int32_t* __restrict__ indptr, int32_t* indices) {
+    const int sub = threadIdx.x & 7;
+    const int64_t row0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
+    const int64_t nr = (int64_t(gridDim.x) * blockDim.x) >> 3;
+    for (int64_t i = row0; i < n; i += nr) {
+        const int32_t* src = rows + 8 * int64_t(__ldg(ne_ptr + i));
+        const int32_t s = __ldg(indptr + i), L = __ldg(indptr + i + 1) - s;
+        for (int l0 = sub; l0 < L; l0 += 32) {
+            int32_t v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = l0 + 8 * q < L ? __ldg(src + l0 + 8 * q) : 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (l0 + 8 * q < L) indices[s + l0 + 8 * q] = v[q];
+        }
     }
 }
 
 // ne_inv[e*8+a] = k; slot_map[8k+b] = slot of conn[e][b] in row conn[e][a].  status bit 4:
-// a pair is missing from the pattern or a row has more than 256 blocks.
-__global__ void k_gather_map(int64_t n8, const int32_t* __restrict__ conn, const int32_t* __restrict__ ne_list,
-                             const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, int32_t* ne_inv,
-                             uint8_t* slot_map, int* status) {
+// a pair is missing from the pattern or a row has more than 256 blocks.  One thread per entry; its
+// eight searches run side by side, one load of each in flight per step (one after the other they took
+// 190 us on 960,000 elements, 145 side by side; a warp per row with the row in shared memory,
+// measured too, 326: its per-row work is more instructions than the searches).
+__global__ void __launch_bounds__(256) k_gather_map(int64_t n8, const int32_t* __restrict__ conn,
+                                                    const int32_t* __restrict__ ne_list,
+                                                    const int32_t* __restrict__ indptr,
+                                                    const int32_t* __restrict__ indices, int32_t* ne_inv,
+                                                    uint8_t* slot_map, int packed, int* status) {
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n8; k += int64_t(gridDim.x) * blockDim.x) {
-        const int32_t ent = ne_list[k];
+        const int32_t ent = __ldg(ne_list + k);
         ne_inv[ent] = int32_t(k);
-        const int64_t e = ent >> 3;
-        const int32_t row = conn[ent];
-        const int32_t s = indptr[row], L = indptr[row + 1] - s;
+        const int64_t e8 = ent & ~7;
+        const int32_t row = __ldg(conn + ent);
+        const int32_t s = __ldg(indptr + row), L = __ldg(indptr + row + 1) - s;
+        const int32_t* __restrict__ r = indices + s;
+        int32_t col[8];
+        int lo[8];
+#pragma unroll
         for (int b = 0; b < 8; ++b) {
-            const int32_t col = conn[8 * e + b];
-            int lo = 0, hi = L;  // first position with indices >= col
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (indices[s + mid] < col) lo = mid + 1;
-                else hi = mid;
-            }
-            const bool ok = lo < L && indices[s + lo] == col && lo <= 255;
-            if (!ok) atomicOr(status, 4);
-            slot_map[8 * k + b] = ok ? uint8_t(lo) : uint8_t(0);
+            col[b] = __ldg(conn + e8 + b);
+            lo[b] = 0;
+        }
+        // lower bound: the answer stays in [lo, lo + len)
+        for (int len = L; len > 1;) {
+            const int half = len >> 1;
+#pragma unroll
+            for (int b = 0; b < 8; ++b) lo[b] += __ldg(r + lo[b] + half - 1) < col[b] ? half : 0;
+            len -= half;
+        }
+        unsigned long long out = 0ull;
+        bool bad = false;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const bool ok = L > 0 && __ldg(r + lo[b]) == col[b] && lo[b] <= 255;
+            bad |= !ok;
+            out |= static_cast<unsigned long long>(ok ? lo[b] : 0) << (8 * b);
+        }
+        if (bad) atomicOr(status, 4);
+        if (packed) {  // slot_map on an 8-byte boundary
+            reinterpret_cast<unsigned long long*>(slot_map)[k] = out;
+        } else {
+            for (int b = 0; b < 8; ++b) slot_map[8 * k + b] = uint8_t(out >> (8 * b));
         }
     }
 }
@@ -371,13 +447,15 @@ extern "C" int fem_topology_fill_gpu(int64_t n_node, int64_t n_elem, const int32
     int* status = reinterpret_cast<int*>(ws + L.status);
     const int32_t* rows = reinterpret_cast<const int32_t*>(ws + L.rows);
     if (n_node) {
-        k_compact_rows<<<grid_for(n_node * 32, 256), 256, 0, st>>>(n_node, ne_ptr, rows, indptr, indices);
+        k_compact_rows<<<grid_for(n_node * 8, 256), 256, 0, st>>>(n_node, ne_ptr, rows, indptr, indices);
         FEM_LAUNCH_CHECK("k_compact_rows");
     }
     const int64_t n8 = 8 * n_elem;
     if (n8 && ne_inv && slot_map) {
         FEM_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
-        k_gather_map<<<grid_for(n8, 256), 256, 0, st>>>(n8, conn, ne_list, indptr, indices, ne_inv, slot_map, status);
+        const int packed = (reinterpret_cast<uintptr_t>(slot_map) & 7) == 0;
+        k_gather_map<<<grid_for(n8, 256), 256, 0, st>>>(n8, conn, ne_list, indptr, indices, ne_inv, slot_map, packed,
+                                                         status);
         FEM_LAUNCH_CHECK("k_gather_map");
         int h = 0;
         int rc = read_status(status, st, h);
