@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kThreads) k_l0_1(const BsrView<float> A, const
     spmv1_rows_epi<float, LPR>(A, x, epi);
 }
 template <int R, typename Epi>
-__global__ void __launch_bounds__(kThreads) k_l0_R(const BsrView<float> A, const float* __restrict__ x, const Epi epi,
+__global__ void __launch_bounds__(kThreads, spmm_ctas<float, R>()) k_l0_R(const BsrView<float> A, const float* __restrict__ x, const Epi epi,
                                                     const PcgState* __restrict__ st) {
     if (st->done) return;
     spmm_rows_epi<float, R>(A, x, epi);
@@ -488,7 +488,7 @@ int launch_l0(const BsrView<float>& A, const float* x, const Epi& epi, const Pcg
     if (R == 1) {
         run(k_l0_1<8, Epi>, (kThreads / 32) * 4);
     } else {
-        const int rpc = (kThreads / 32) * (32 / R);
+        const int rpc = (kThreads / 32) * (A.rsoa == 2 ? 1 : 32 / R);
         switch (R) {
             case 2: run(k_l0_R<2, Epi>, rpc); break;
             case 4: run(k_l0_R<4, Epi>, rpc); break;

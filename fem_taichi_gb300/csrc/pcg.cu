@@ -1,8 +1,11 @@
 // Device-resident block-preconditioned conjugate gradients on the 3x3-block BSR matrix.
 // Replaces pardisoSolver(KL, mtype=2).factor()/solve(F) of SOLVE_static.py:31-33.
 //
-// One PCG iteration is three kernels (p = z + beta p;  q = A p with p.q;  x += alpha p,
-// r -= alpha q, z = M r with r.z and r.r).  All scalars live in a device state block:
+// One PCG iteration is three kernels (x += alpha p, p = M r + beta p;  q = A p with p.q;
+// r -= alpha q with r.M r and r.r).  z = M r is formed where it is used (nine values of M per node
+// against three of z per node and right-hand side) and x waits for the kernel that reads p anyway,
+// so an iteration streams 8 vectors beside the product instead of 10; one more kernel after the last
+// iteration adds the pending alpha p.  All scalars live in a device state block:
 // every reduction writes per-CTA partials and the last CTA to finish (atomic ticket) sums
 // them in CTA order, so results are bitwise reproducible, and computes alpha / beta /
 // convergence on the device.  Each kernel returns immediately once the state says the
@@ -29,11 +32,10 @@ namespace {
 
 using namespace pcgd;
 
-// x = 0, r = b, z = M r; rz, rr -> state (bb = rr, tol2 = rtol^2 bb).
+// x = 0, r = b; rz = r.M r, rr -> state (bb = rr, tol2 = rtol^2 bb).
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restrict__ M, const T* __restrict__ b,
-                                                    T* x, T* r, T* z, double* part, PcgState* st, double rtol,
-                                                    int maxit) {
+                                                    T* x, T* r, double* part, PcgState* st, double rtol, int maxit) {
     double v[2] = {0.0, 0.0};
     Dot<T> d_rz, d_rr;
     const int64_t total_t = n * R;
@@ -52,9 +54,6 @@ __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restric
             r[o] = r0;
             r[o + R] = r1;
             r[o + 2 * R] = r2;
-            z[o] = z0;
-            z[o + R] = z1;
-            z[o + 2 * R] = z2;
             d_rz.add(r0, z0);
             d_rz.add(r1, z1);
             d_rz.add(r2, z2);
@@ -96,6 +95,63 @@ __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restric
     }
 }
 
+// x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration).  One
+// thread per node and V right-hand sides (rows of r, x and p on V * sizeof(T)-byte boundaries).
+template <typename T, int V>
+struct alignas(V * sizeof(T)) Pack {
+    T v[V];
+};
+template <typename T, int R, int V>
+__global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __restrict__ M, const T* __restrict__ r,
+                                                         T* x, T* p, const PcgState* __restrict__ st) {
+    if (st->done) return;
+    using P = Pack<T, V>;
+    const bool first = st->it == 0;
+    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n * (R / V);
+         t += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t node = t / (R / V);
+        const int k = int(t % (R / V)) * V;
+        const int64_t o = 3 * node * R + k;
+        P rv[3], xv[3], pv[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            rv[j] = *reinterpret_cast<const P*>(r + o + j * R);
+            if (!first) {
+                xv[j] = *reinterpret_cast<const P*>(x + o + j * R);
+                pv[j] = *reinterpret_cast<const P*>(p + o + j * R);
+            }
+        }
+        T m[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) m[q] = __ldg(M + 9 * node + q);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            T z[3];
+            apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], z[0], z[1], z[2]);
+            const T a = T(st->alpha[k + i]), b = T(st->beta[k + i]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                if (!first) xv[j].v[i] += a * pv[j].v[i];
+                pv[j].v[i] = first ? z[j] : T(z[j] + b * pv[j].v[i]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            if (!first) *reinterpret_cast<P*>(x + o + j * R) = xv[j];
+            *reinterpret_cast<P*>(p + o + j * R) = pv[j];
+        }
+    }
+}
+
+// The last iteration's x += alpha p, whatever ended the solve (nothing pending when it took no step).
+template <typename T, int R>
+__global__ void __launch_bounds__(kThreads) k_x_finish(int64_t nv, const T* __restrict__ p, T* x,
+                                                        const PcgState* __restrict__ st) {
+    if (st->it == 0) return;
+    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < nv; e += int64_t(gridDim.x) * blockDim.x)
+        x[e] += T(st->alpha[e % R]) * p[e];
+}
+
 // p = z + beta p  (p = z on the first iteration)
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_p_update(int64_t nv, const T* __restrict__ z, T* p,
@@ -111,26 +167,18 @@ __global__ void __launch_bounds__(kThreads) k_p_update(int64_t nv, const T* __re
 // q = A p and p.q -> alpha = rz / pq on the device.  (Folding p = z + beta p into this
 // kernel as q = A z + beta q was measured slower: the row epilogue's extra loads sit on the
 // product's critical path, and the recurrence drifts from A p in FP32.)
-template <typename T, int LPR_OR_R>
-__global__ void __launch_bounds__(kThreads) k_spmv_pq(const BsrView<T> A, const T* __restrict__ p, T* __restrict__ q,
-                                                       double* part, PcgState* st, int R) {
+template <typename T, int R, int LPR>
+__global__ void __launch_bounds__(kThreads, spmm_ctas<T, R>())
+    k_spmv_pq(const BsrView<T> A, const T* __restrict__ p, T* __restrict__ q, double* part, PcgState* st) {
     if (st->done) return;
     double v[1];
-    if (R == 1)
-        v[0] = spmv1_rows<T, LPR_OR_R>(A, p, q, true);
+    if constexpr (R == 1)
+        v[0] = spmv1_rows<T, LPR>(A, p, q, true);
     else
-        v[0] = spmm_rows<T, LPR_OR_R>(A, p, q, true);
-    constexpr int RR = LPR_OR_R;
+        v[0] = spmm_rows<T, R>(A, p, q, true);
     __shared__ double tot[1][kMaxR];
-    bool last;
-    if (R == 1) {
-        last = block_partials<1, 1>(v, part, &st->ticket);
-        if (last) last_block_totals<1, 1>(part, gridDim.x, tot);
-    } else {
-        last = block_partials<RR, 1>(v, part, &st->ticket);
-        if (last) last_block_totals<RR, 1>(part, gridDim.x, tot);
-    }
-    if (last) {
+    if (block_partials<R, 1>(v, part, &st->ticket)) {
+        last_block_totals<R, 1>(part, gridDim.x, tot);
         const int k = threadIdx.x;
         if (k < R) {
             if (st->active[k]) {
@@ -152,11 +200,10 @@ __global__ void __launch_bounds__(kThreads) k_spmv_pq(const BsrView<T> A, const 
     }
 }
 
-// x += alpha p; r -= alpha q; z = M r; rz, rr -> beta, convergence, iteration count.
+// r -= alpha q; z = M r; rz, rr -> beta, convergence, iteration count.
 template <typename T, int R>
-__global__ void __launch_bounds__(kThreads) k_update(int64_t n, const T* __restrict__ M, const T* __restrict__ p,
-                                                      const T* __restrict__ q, T* x, T* r, T* z, double* part,
-                                                      PcgState* st) {
+__global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __restrict__ M, const T* __restrict__ q,
+                                                        T* r, double* part, PcgState* st) {
     if (st->done) return;
     double v[2] = {0.0, 0.0};
     Dot<T> d_rz, d_rr;
@@ -168,18 +215,12 @@ __global__ void __launch_bounds__(kThreads) k_update(int64_t n, const T* __restr
             const int k = int(t % R);
             const int64_t o = 3 * node * R + k;
             const T a = T(st->alpha[k]);
-            x[o] += a * p[o];
-            x[o + R] += a * p[o + R];
-            x[o + 2 * R] += a * p[o + 2 * R];
             const T r0 = r[o] - a * q[o], r1 = r[o + R] - a * q[o + R], r2 = r[o + 2 * R] - a * q[o + 2 * R];
             r[o] = r0;
             r[o + R] = r1;
             r[o + 2 * R] = r2;
             T z0, z1, z2;
             apply_block(M + 9 * node, r0, r1, r2, z0, z1, z2);
-            z[o] = z0;
-            z[o + R] = z1;
-            z[o + 2 * R] = z2;
             d_rz.add(r0, z0);
             d_rz.add(r1, z1);
             d_rz.add(r2, z2);
@@ -200,7 +241,10 @@ __global__ void __launch_bounds__(kThreads) k_update(int64_t n, const T* __restr
             st->rz[k] = rz;
             st->rr[k] = rr;
             st->iters[k] += 1;
-            if (!(rr > st->tol2[k])) st->active[k] = 0;
+            if (!(rr > st->tol2[k])) {
+                st->active[k] = 0;
+                st->beta[k] = 0.0;   // a frozen system's p stays M r
+            }
             if (!isfinite(rr)) {
                 st->active[k] = 0;
                 st->status = FEM_ERR_BREAKDOWN;
@@ -524,35 +568,40 @@ unsigned vec_grid(Kernel kernel, int64_t work) {
 // dot-product partial sums.
 template <typename T, int R>
 void launch_spmv_pq(const BsrView<T>& A, const T* p, T* q, double* part, PcgState* st, int variant, cudaStream_t s) {
-    auto run = [&](auto kernel, int64_t rows_per_cta, int64_t cap, int r) {
+    auto run = [&](auto kernel, int64_t rows_per_cta, int64_t cap) {
         const unsigned g = resident_grid(reinterpret_cast<const void*>(kernel), kThreads,
                                          (A.n + rows_per_cta - 1) / rows_per_cta, std::min<int64_t>(cap, kMaxCtas));
-        kernel<<<g, kThreads, 0, s>>>(A, p, q, part, st, r);
+        kernel<<<g, kThreads, 0, s>>>(A, p, q, part, st);
     };
-    if (R > 1) {
-        run(k_spmv_pq<T, R>, int64_t(kThreads / 32) * (32 / R), int64_t(sm_count()) * 8, R);
-        return;
-    }
-    const SpmvVariant v = spmv_variant(variant);
-    const int64_t rows_per_cta = int64_t(kThreads / 32) * (32 / v.lpr);
-    const int64_t cap = int64_t(sm_count()) * (v.ctas_per_sm * v.threads / kThreads);
-    switch (v.lpr) {
-        case 32: run(k_spmv_pq<T, 32>, rows_per_cta, cap, 1); break;
-        case 16: run(k_spmv_pq<T, 16>, rows_per_cta, cap, 1); break;
-        case 8: run(k_spmv_pq<T, 8>, rows_per_cta, cap, 1); break;
-        case 4: run(k_spmv_pq<T, 4>, rows_per_cta, cap, 1); break;
-        default: run(k_spmv_pq<T, 2>, rows_per_cta, cap, 1); break;
+    if constexpr (R > 1) {
+        run(k_spmv_pq<T, R, 0>, int64_t(kThreads / 32) * (A.rsoa == 2 ? 1 : 32 / R), int64_t(sm_count()) * 8);
+    } else {
+        const SpmvVariant v = spmv_variant(variant);
+        const int64_t rows_per_cta = int64_t(kThreads / 32) * (32 / v.lpr);
+        const int64_t cap = int64_t(sm_count()) * (v.ctas_per_sm * v.threads / kThreads);
+        switch (v.lpr) {
+            case 32: run(k_spmv_pq<T, 1, 32>, rows_per_cta, cap); break;
+            case 16: run(k_spmv_pq<T, 1, 16>, rows_per_cta, cap); break;
+            case 8: run(k_spmv_pq<T, 1, 8>, rows_per_cta, cap); break;
+            case 4: run(k_spmv_pq<T, 1, 4>, rows_per_cta, cap); break;
+            default: run(k_spmv_pq<T, 1, 2>, rows_per_cta, cap); break;
+        }
     }
 }
 
 template <typename T, int R>
-int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* z, T* p, T* q, double* part, PcgState* st,
-                      int variant, int count, cudaStream_t s) {
-    const int64_t nv = 3 * A.n * R;
+int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* p, T* q, double* part, PcgState* st, int variant,
+                      int count, cudaStream_t s) {
+    // 16-byte packs of right-hand sides where the rows of r, p and x (the caller's U in the FP64 solve)
+    // start on 16-byte boundaries
+    constexpr int V = R % (16 / int(sizeof(T))) == 0 ? 16 / int(sizeof(T)) : 1;
     for (int i = 0; i < count; ++i) {
-        k_p_update<T, R><<<vec_grid(k_p_update<T, R>, nv), kThreads, 0, s>>>(nv, z, p, st);
+        if (aligned16(x))
+            k_xp_update<T, R, V><<<vec_grid(k_xp_update<T, R, V>, A.n * (R / V)), kThreads, 0, s>>>(A.n, M, r, x, p, st);
+        else
+            k_xp_update<T, R, 1><<<vec_grid(k_xp_update<T, R, 1>, A.n * R), kThreads, 0, s>>>(A.n, M, r, x, p, st);
         launch_spmv_pq<T, R>(A, p, q, part, st, variant, s);
-        k_update<T, R><<<vec_grid(k_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, p, q, x, r, z, part, st);
+        k_r_update<T, R><<<vec_grid(k_r_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, q, r, part, st);
     }
     FEM_LAUNCH_CHECK("pcg iteration");
     return FEM_OK;
@@ -623,20 +672,25 @@ int pcg_drive(const Init& init, const Iters& iters, PcgState* st, int maxit, int
     return FEM_OK;
 }
 
-// Runs PCG on (A, M) with right-hand side b into x; vectors r z p q are workspace.
+// Runs PCG on (A, M) with right-hand side b into x; vectors r p q are workspace (16-byte aligned).
 template <typename T, int R>
-int pcg_core(const BsrView<T>& A, const T* M, const T* b, T* x, T* r, T* z, T* p, T* q, double* part, PcgState* st,
+int pcg_core(const BsrView<T>& A, const T* M, const T* b, T* x, T* r, T* p, T* q, double* part, PcgState* st,
              double rtol, int maxit, int variant, int use_graph, int unroll, cudaStream_t s, InnerResult* res,
              int stall = 0) {
     auto init = [&](cudaStream_t ss) -> int {
-        k_init<T, R><<<vec_grid(k_init<T, R>, A.n * R), kThreads, 0, ss>>>(A.n, M, b, x, r, z, part, st, rtol, maxit);
+        k_init<T, R><<<vec_grid(k_init<T, R>, A.n * R), kThreads, 0, ss>>>(A.n, M, b, x, r, part, st, rtol, maxit);
         FEM_LAUNCH_CHECK("k_init");
         return FEM_OK;
     };
     auto iters = [&](int count, cudaStream_t ss) -> int {
-        return launch_iterations<T, R>(A, M, x, r, z, p, q, part, st, variant, count, ss);
+        return launch_iterations<T, R>(A, M, x, r, p, q, part, st, variant, count, ss);
     };
-    return pcg_drive(init, iters, st, maxit, use_graph, unroll, s, res, stall);
+    int rc = pcg_drive(init, iters, st, maxit, use_graph, unroll, s, res, stall);
+    if (rc) return rc;
+    const int64_t nv = 3 * A.n * R;
+    k_x_finish<T, R><<<vec_grid(k_x_finish<T, R>, nv), kThreads, 0, s>>>(nv, p, x, st);
+    FEM_LAUNCH_CHECK("k_x_finish");
+    return FEM_OK;
 }
 
 // The same with the multigrid V-cycle as the preconditioner.  T = float: the FP32 inner
@@ -755,7 +809,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
                 return pcg_core_amg<double, R>(K64, K32, amg, b, x, r, z, p, q, part, st, tol, cap, o->spmv_variant,
                                                o->use_graph, o->unroll, s, &ir, o->stall_window);
             }
-            return pcg_core<double, R>(K64, M64, b, x, r, z, p, q, part, st, tol, cap, o->spmv_variant,
+            return pcg_core<double, R>(K64, M64, b, x, r, p, q, part, st, tol, cap, o->spmv_variant,
                                        o->use_graph, o->unroll, s, &ir, o->stall_window);
         };
         int rc = core(F, U, o->rtol, maxit);
@@ -822,7 +876,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
                                             std::max(1, o->inner_maxit), o->spmv_variant32, o->use_graph, o->unroll,
                                             s, &ir, o->stall_window);
             else
-                rc = pcg_core<float, R>(K32, M32, b32, d32, rr, zz, pp, qq, part, st, o->inner_rtol,
+                rc = pcg_core<float, R>(K32, M32, b32, d32, rr, pp, qq, part, st, o->inner_rtol,
                                         std::max(1, o->inner_maxit), o->spmv_variant32, o->use_graph, o->unroll, s,
                                         &ir, o->stall_window);
             if (rc) return rc;

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(512) k_spmv(const BsrView<T> A, const T* __res
 }
 
 template <typename T, int R>
-__global__ void __launch_bounds__(256) k_spmm(const BsrView<T> A, const T* __restrict__ x, T* __restrict__ y) {
+__global__ void __launch_bounds__(256, spmm_ctas<T, R>()) k_spmm(const BsrView<T> A, const T* __restrict__ x, T* __restrict__ y) {
     spmm_rows<T, R>(A, x, y, false);
 }
 
@@ -168,7 +168,7 @@ int launch_spmv(const BsrView<T>& A, int nrhs, const T* x, T* y, int variant, cu
             default: run(k_spmv<T, 2>, v.threads, rows_per_cta, cap); break;
         }
     } else {
-        const int64_t rows_per_cta = 8 * (32 / nrhs);
+        const int64_t rows_per_cta = 8 * (A.rsoa == 2 ? 1 : 32 / nrhs);
         const int64_t cap = int64_t(sms) * 8;
         switch (nrhs) {
             case 2: run(k_spmm<T, 2>, 256, rows_per_cta, cap); break;

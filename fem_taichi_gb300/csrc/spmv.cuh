@@ -5,7 +5,8 @@
 //  * nrhs == 1: LPR lanes cooperate on one block row (lane = block slot), followed by an
 //    xor-shuffle reduction of the three row sums; 32/LPR rows per warp.
 //  * nrhs  > 1: lanes map to right-hand sides (32/nrhs rows per warp); each block's nine
-//    values are loaded once per row group (broadcast) and applied to all RHS.
+//    values are loaded once per row group (broadcast) and applied to all RHS (the padded FP32
+//    layout: spmm4_rows_epi).
 // Rows are visited with a grid-stride loop so the grid can be sized in multiples of the SM
 // count; a fixed grid gives a fixed row -> CTA mapping, hence deterministic partial sums.
 #pragma once
@@ -187,47 +188,180 @@ __device__ __forceinline__ double spmv1_rows_epi(const BsrView<T>& A, const T* _
     return dot.value();
 }
 
-// Many right-hand sides on the padded row-SoA FP32 copy: one block row per warp, lane =
-// (slot group g, right-hand side k) with 32 / R slot groups; each lane takes 4 consecutive
-// slots per step (one 16-byte load per value, the same address for the R lanes of a group),
-// then the groups' partial sums are combined by xor-shuffles.
+// Many right-hand sides on the padded row-SoA FP32 copy, one block row per warp (256 threads a CTA).
+// A row's values and columns are one contiguous piece each; cp.async brings them into the warp's
+// shared-memory ring kStage - 1 rows ahead, so only the gathers of x wait on memory.  Lane = (slot group
+// g of G, vector sub of LP): it takes 4 consecutive slots a step and V right-hand sides of them, so
+// one load instruction fetches x of G blocks and one shared-memory load a value of 4 G slots.  At the end
+// of a row the groups' sums are exchanged so that a lane adds only the right-hand sides it keeps
+// (reduce-scatter), and right-hand side k's totals move to lane k.  A CTA takes eight consecutive rows
+// at a time, for the x lines they share in L1.
+// Bound by L1 (84 lines of x per 27-block row at R = 32) and the latency of the gathers.  Product of
+// 137,781 rows at R = 32: 207 us with one right-hand side per lane and values loaded in line (1,188
+// instructions a row, most of them addresses); 190 us with vectors of right-hand sides (560, every step
+// waiting on values from HBM); 125 us staged.  L1 capacity decides the rest: 2 rows staged and 2 CTAs an SM
+// leave it 192 KB (3 rows: 156 us; 3 CTAs with p.q: 339 instead of 268 us an iteration of the solve);
+// fewer right-hand sides gather less and take 3 CTAs (R = 8: 59 against 69 us).  V and G: 4-slot groups of a 28-slot row in 2 x 4 or 8
+// groups leave 1 in 8 idle, more groups would idle half.
+template <int V>
+struct alignas(4 * V) FloatVec {
+    float v[V];
+};
+constexpr int kStage = 2;          // rows of a warp in shared memory
+constexpr int kStageSlots = 32;    // longest staged row; longer ones are read in place
+// CTAs per SM of the kernels around spmm_rows_epi (see spmm4_rows_epi)
+template <typename T, int R>
+constexpr int spmm_ctas() {
+    return sizeof(T) != 4 || R == 1 ? 1 : R == 32 ? 2 : 3;
+}
+
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(dst))), "l"(src));
+}
+
 template <int R, typename Epi>
 __device__ __forceinline__ double spmm4_rows_epi(const BsrView<float>& A, const float* __restrict__ x, const Epi& epi) {
-    constexpr int G = 32 / R;
-    const int lane = threadIdx.x & 31;
-    const int g = lane / R, rhs = lane % R;
-    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    constexpr int V = R >= 16 ? 4 : R == 8 ? 2 : 1, LP = R / V, G = 32 / LP, CS = 4 * G;
+    constexpr unsigned full = 0xffffffffu;
+    constexpr int kWarps = 8;
+    struct Stage {
+        float val[9 * kStageSlots];
+        int32_t col[kStageSlots];
+    };
+    __shared__ __align__(16) Stage ring[kWarps][kStage];
+    using X = FloatVec<V>;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int g = lane / LP, sub = lane % LP;
     Dot<float> dot;
-    for (int64_t row = warp; row < A.n; row += nwarps) {
-        const int64_t rs = __ldg(A.indptr + row);
-        const int Lp = __ldg(A.indptr + row + 1) - int(rs);
-        const float* v0 = A.vals + 9 * rs;
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-        for (int s = 4 * g; s < Lp; s += 4 * G) {
-            const int4 c = __ldg(reinterpret_cast<const int4*>(A.indices + rs + s));
-            float4 w[9];
+    const int64_t first = int64_t(blockIdx.x) * kWarps + wid, stride = int64_t(gridDim.x) * kWarps;
+    const int steps = first < A.n ? int((A.n - first + stride - 1) / stride) : 0;
+
+    int32_t rp = 0, rp1 = 0;  // row pointers of the warp's rows, 32 steps at a time
+    int64_t rs[kStage];
+    int len[kStage];
 #pragma unroll
-            for (int q = 0; q < 9; ++q) w[q] = __ldg(reinterpret_cast<const float4*>(v0 + int64_t(q) * Lp + s));
-            const int cc[4] = {c.x, c.y, c.z, c.w};
+    for (int d = 0; d < kStage; ++d) rs[d] = 0, len[d] = 0;
+    // row of step t into slot t % kStage of the ring; rs / len are shifted by the caller
+    auto fetch = [&](int t, int64_t& r0, int& L) {
+        r0 = 0;
+        L = 0;
+        if (t < steps) {
+            if ((t & 31) == 0) {
+                const int64_t row = first + stride * (t + lane);
+                rp = rp1 = 0;
+                if (row < A.n) {
+                    rp = __ldg(A.indptr + row);
+                    rp1 = __ldg(A.indptr + row + 1);
+                }
+            }
+            r0 = __shfl_sync(full, rp, t & 31);
+            L = __shfl_sync(full, rp1, t & 31) - int(r0);
+            if (L <= kStageSlots) {
+                Stage& st = ring[wid][t % kStage];
+                const float* v = A.vals + 9 * r0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                auto wq = [&](int q) { return j == 0 ? w[q].x : j == 1 ? w[q].y : j == 2 ? w[q].z : w[q].w; };
-                const float* xc = x + 3 * int64_t(cc[j]) * R + rhs;
-                const float x0 = xc[0], x1 = xc[R], x2 = xc[2 * R];
-                a0 += wq(0) * x0 + wq(1) * x1 + wq(2) * x2;
-                a1 += wq(3) * x0 + wq(4) * x1 + wq(5) * x2;
-                a2 += wq(6) * x0 + wq(7) * x1 + wq(8) * x2;
+                for (int i = 0; i < 9 * kStageSlots / 4; i += 32)
+                    if (i + lane < 9 * L / 4) copy_async16(st.val + 4 * (i + lane), v + 4 * (i + lane));
+                if (lane < L / 4) copy_async16(st.col + 4 * lane, A.indices + r0 + 4 * lane);
             }
         }
+        asm volatile("cp.async.commit_group;");
+    };
 #pragma unroll
-        for (int off = R; off < 32; off <<= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-            a2 += __shfl_xor_sync(0xffffffffu, a2, off);
+    for (int d = 0; d < kStage - 1; ++d) fetch(d, rs[d], len[d]);
+    for (int t = 0; t < steps; ++t) {
+        fetch(t + kStage - 1, rs[kStage - 1], len[kStage - 1]);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStage - 1));
+        __syncwarp();   // every lane's copies of this row have landed
+        const int64_t row = first + stride * t;
+        const int Lp = len[0];
+        const Stage& st = ring[wid][t % kStage];
+        float acc[3][V];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[j][i] = 0.f;
+        // one step: 4 slots of every group, values and columns from `val` and `col`
+        auto step = [&](int c0, const float* val, const int32_t* col) {
+            const int s = c0 + 4 * g;
+            const bool in = s < Lp;
+            // slots beyond the row: the row's own x times 0
+            const int4 idx = in ? *reinterpret_cast<const int4*>(col + s)
+                                : make_int4(int(row), int(row), int(row), int(row));
+            X xv[4][3];
+            const int cc[4] = {idx.x, idx.y, idx.z, idx.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float* xc = x + int64_t(cc[u]) * (3 * R) + sub * V;
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    if constexpr (V == 4) {
+                        const float4 f = __ldg(reinterpret_cast<const float4*>(xc + j * R));
+                        xv[u][j].v[0] = f.x, xv[u][j].v[1] = f.y, xv[u][j].v[2] = f.z, xv[u][j].v[3] = f.w;
+                    } else if constexpr (V == 2) {
+                        const float2 f = __ldg(reinterpret_cast<const float2*>(xc + j * R));
+                        xv[u][j].v[0] = f.x, xv[u][j].v[1] = f.y;
+                    } else {
+                        xv[u][j].v[0] = __ldg(xc + j * R);
+                    }
+                }
+            }
+            const float* vs = val + s;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const float4 w = in ? *reinterpret_cast<const float4*>(vs + (3 * j + c) * Lp)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int i = 0; i < V; ++i) {
+                        acc[j][i] = fmaf(w.x, xv[0][c].v[i], acc[j][i]);
+                        acc[j][i] = fmaf(w.y, xv[1][c].v[i], acc[j][i]);
+                        acc[j][i] = fmaf(w.z, xv[2][c].v[i], acc[j][i]);
+                        acc[j][i] = fmaf(w.w, xv[3][c].v[i], acc[j][i]);
+                    }
+                }
+        };
+        if (Lp <= kStageSlots) {
+#pragma unroll 1
+            for (int c0 = 0; c0 < Lp; c0 += CS) step(c0, st.val, st.col);
+        } else {
+#pragma unroll 1
+            for (int c0 = 0; c0 < Lp; c0 += CS) step(c0, A.vals + 9 * rs[0], A.indices + rs[0]);
         }
-        if (g == 0) epi(3 * row * R + rhs, R, rhs, a0, a1, a2, dot);
+        __syncwarp();   // the ring slot may be refilled
+        // reduce-scatter: after a level with offset off, lane keeps half of its right-hand sides
+        int off = LP;
+#pragma unroll
+        for (int keep = V / 2; keep >= 1; keep >>= 1, off <<= 1) {
+            const bool hi = (lane & off) != 0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < keep; ++i) {
+                    const float send = hi ? acc[j][i] : acc[j][i + keep];
+                    const float mine = hi ? acc[j][i + keep] : acc[j][i];
+                    acc[j][i] = mine + __shfl_xor_sync(full, send, off);
+                }
+        }
+        float a[3] = {acc[0][0], acc[1][0], acc[2][0]};
+#pragma unroll
+        for (; off < 32; off <<= 1)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) a[j] += __shfl_xor_sync(full, a[j], off);
+        // right-hand side k stays with vector k / V, on the lane whose scatter bits (high half first) are
+        // the bits of k % V
+        const int k = lane % R;
+        if constexpr (V > 1) {
+            const int src = (V == 4 ? ((k >> 1) & 1) + 2 * (k & 1) : k & 1) * LP + k / V;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) a[j] = __shfl_sync(full, a[j], src);
+        }
+        if (lane < R) epi(3 * row * R + k, R, k, a[0], a[1], a[2], dot);
+#pragma unroll
+        for (int d = 0; d < kStage - 1; ++d) rs[d] = rs[d + 1], len[d] = len[d + 1];
     }
+    asm volatile("cp.async.wait_all;");
     return dot.value();
 }
 
@@ -236,7 +370,8 @@ __device__ __forceinline__ double spmm4_rows_epi(const BsrView<float>& A, const 
 template <typename T, int R, typename Epi>
 __device__ __forceinline__ double spmm_rows_epi(const BsrView<T>& A, const T* __restrict__ x, const Epi& epi) {
     if constexpr (sizeof(T) == 4) {
-        if (A.rsoa == 2) return spmm4_rows_epi<R>(A, x, epi);
+        // the vector loads of x need its rows on 16-byte boundaries (a caller's x may be a view)
+        if (A.rsoa == 2 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) return spmm4_rows_epi<R>(A, x, epi);
     }
     const int lane = threadIdx.x & 31;
     const int sub = lane / R, rhs = lane % R;
