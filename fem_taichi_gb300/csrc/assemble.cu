@@ -2,27 +2,32 @@
 //
 // Two kernels, both deterministic and free of floating-point atomics:
 //
-//  1. k_hex8_element -- 8 threads per element.  Thread t first forms coefficient t of the
-//     element's trilinear map x(xi) = sum_k c_k m_k(xi) (m = 1, xi, eta, zeta, xi eta,
-//     eta zeta, xi zeta, xi eta zeta; c_k = 1/8 sum_a m_k(corner a) x_a) and W x_t, where W is
-//     the centrifugal operator of UnitVectorF (FEM_model_bsr.py:291-300).  Phase A: thread g
-//     handles Gauss point g (Jacobian from the coefficients, 27 FMA instead of 72; adjugate,
-//     determinant, the 8 scaled gradients R_a = dN_a/dxi . adj(J)); results are staged in
+//  1. k_hex8_element -- 8 threads per element, an element's threads in one warp (no block barrier
+//     but for the shape table).  Thread t loads corner t; a Walsh transform over the 8 lanes gives
+//     8 times the coefficients of the element's trilinear map x(xi) = sum_k c_k m_k(xi) (m = 1, xi,
+//     eta, zeta, xi eta, eta zeta, xi zeta, xi eta zeta; c_k = 1/8 sum_a m_k(corner a) x_a); the powers of two
+//     go into mu and DE.  Phase A: thread g handles Gauss point g (Jacobian from the coefficients --
+//     a column d/dxi does not depend on xi, so the two lanes that share it split its three components
+//     -- adjugate, determinant, the 8 scaled gradients R_a = dN_a/dxi . adj(J)); results are staged in
 //     shared memory.  Phase B: the 36 node pairs (a <= b) are split across the 8 threads;
-//     each accumulates the Gram matrix P_ab = sum_g R_a R_b^T / det_g and turns it into the
-//     3x3 stiffness block  K_ab[p][q] = lam P[p][q] + mu P[q][p],
-//     K_ab[p][p] = D0d P[p][p] + mu (tr P - P[p][p]), which equals sum_g det (B1_a^T D0 B1_b +
+//     each accumulates the Gram matrix P_ab = mu sum_g R_a R_b^T / det_g and turns it into the
+//     3x3 stiffness block  K_ab[p][q] = (lam/mu) P[p][q] + P[q][p],
+//     K_ab[p][p] = (lam/mu + 1) P[p][p] + tr P, which equals sum_g det (B1_a^T D0 B1_b +
 //     B2_a^T D1 B2_b) of the reference (FEM_model_bsr.py:262-274, 303-347) with a different
-//     summation order.  The consistent mass M_ab = DE sum_g det_g N_a N_b
+//     summation order.  The 28 off-diagonal pairs are 3.5 per thread: two threads share each of the
+//     last four, four Gauss points a thread.  The consistent mass M_ab = DE sum_g det_g N_a N_b
 //     (FEM_model_bsr.py:276-287) is sum-factorised: N_a(g) is a product of one 1D factor per
 //     axis, so M_ab depends only on the per-axis class of (a, b) and the 8 det_g are contracted
-//     axis by axis (27 classes, 141 FP64 operations per element instead of 288).  The centrifugal
+//     axis by axis (27 classes, 114 FP64 operations per element instead of 288).  The centrifugal
 //     load (FEM_model_bsr.py:229-245) is F_a = sum_g DE det_g N_a(g) W x(g); W x is linear and
 //     the isoparametric map reproduces it at the Gauss points, W x(g) = sum_b N_b(g) W x_b, so
 //     F_a = sum_b M_ab W x_b: the same quantity from the mass blocks, with no per-Gauss-point
 //     load density.  Each element writes one 2,944-byte record: 28 off-diagonal pairs as
 //     K (3x3) + M, 8 diagonal pairs as the 6 distinct values of the symmetric K + M (8-double
-//     slots), 8 x F(3).
+//     slots), 8 x F(3).  Bound by the FP64 pipe (one warp instruction per 16 cycles per SM): what
+//     shuffles, sign flips and prescaled constants save shows in full.  960,000 elements: 8.85 ms with
+//     a summed Jacobian per lane, lam and mu applied per block and half of a fourth round of pairs
+//     idle; 7.4 ms in this form.
 //
 //  2. k_gather -- one warp per block row i.  Lane l owns slot l of the row (column node
 //     indices[indptr[i] + l]).  The warp walks the incident (element, corner) list of
@@ -63,26 +68,26 @@ struct ElemParams {
     const int4* conn4;
     int64_t e_begin, e_end;  // elements [e_begin, e_end) of this launch
     double* rec;
-    double DE, D0d, lam, mu;
+    double lm;         // lam / mu
+    double mu8;        // mu / 8
     double wc[3][3];   // centrifugal operator: f = wc . x (UnitVectorF)
     DevTables tab;
     // tm[s][c]: product of the 1D shape factors of two corners along one axis at a Gauss point
     // on the negative (s = 0) or positive (s = 1) side: c = 0 both corners negative, 1 mixed,
-    // 2 both positive
-    double tm[2][3];
+    // 2 both positive; tmx the same times DE / 512 (x is contracted first)
+    double tm[2][3], tmx[2][3];
 };
 
 struct ElemSmem {
     double dnr[8][kRPad];       // dN_a/dxi_i at Gauss point g at [g][3a+i]; padded row: the 8 rows
                                 // start in 8 different bank pairs (a 24-double row put every
                                 // even g in one bank and every odd g in another)
-    double x[kEpc][8][3];       // corner coordinates; later the first mass contraction (D1)
-    double xl[kEpc][8][3];      // corner coordinates relative to corner 0; later D2
-    double cf[kEpc][8][3];      // trilinear coefficients c_k of the element map (c_0 unused)
+    double cf[kEpc][8][3];      // Walsh sums of the element-local coordinates; later D1
     double wx[kEpc][8][3];      // W x_a: centrifugal density per unit mass at corner a
-    double R[kEpc][8][kRPad];   // R_a(g)[i] at [el][g][3a+i]
-    double Rs[kEpc][8][kRPad];  // R_a(g)[i] / det_g
-    double det[kEpc][8];
+    double R[kEpc][8][kRPad];   // R_a(g)[i] (x 64) at [el][g][3a+i]
+    double Rs[kEpc][8][kRPad];  // mu R_a(g)[i] / det_g, scaled so that the products have no factor
+    double det[kEpc][8];        // x 512
+    double d2[kEpc][18];        // second mass contraction
     double m[kEpc][36];         // mass by corner-pair class (27 used, DE included), see mass_class
 };
 
@@ -95,17 +100,7 @@ __device__ __forceinline__ int mass_class(int a, int b) {
     return cx * 9 + cy * 3 + cz;
 }
 
-// m_k(corner a) for the trilinear monomials 1, xi, eta, zeta, xi eta, eta zeta, xi zeta,
-// xi eta zeta; corner signs in the reference's node order (FEM_model_bsr.py:371-382):
-// xi < 0 at corners 1, 2, 5, 6 (mask 0x66), eta < 0 at 2, 3, 6, 7 (0xCC), zeta < 0 at 0-3
-// (0x0F); monomial k contains xi for k in {1, 4, 6, 7} (0xD2), eta for {2, 4, 5, 7} (0xB4),
-// zeta for {3, 5, 6, 7} (0xE8).
-__device__ __forceinline__ double monomial_sign(int k, int a) {
-    const int neg = (((0xD2 >> k) & (0x66 >> a)) ^ ((0xB4 >> k) & (0xCC >> a)) ^ ((0xE8 >> k) & (0x0F >> a))) & 1;
-    return neg ? -1.0 : 1.0;
-}
-
-// Off-diagonal pair list (a < b), 28 entries; thread t takes entries t, t+8, t+16, t+24.
+// Off-diagonal pair list (a < b), 28 entries.
 __device__ __forceinline__ void offdiag_pair(int q, int& a, int& b) {
     // q -> (a, b) for row-major enumeration of a < b
     int aa = 0, rem = q;
@@ -117,58 +112,83 @@ __device__ __forceinline__ void offdiag_pair(int q, int& a, int& b) {
     b = aa + 1 + rem;
 }
 
+// P += sum over Gauss points g0 .. g0 + ng - 1 of Rs_a R_b^T
+__device__ __forceinline__ void gram(const ElemSmem& s, int el, int a, int b, int g0, int ng, double (&P)[9]) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) P[i] = 0.0;
+#pragma unroll 4
+    for (int g = g0; g < g0 + ng; ++g) {
+        const double* q = s.Rs[el][g] + 3 * a;
+        const double* r = s.R[el][g] + 3 * b;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) P[3 * i + j] = fma(q[i], r[j], P[3 * i + j]);
+    }
+}
+
 __global__ void __launch_bounds__(kElemThreads, 3) k_hex8_element(const ElemParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ElemSmem& s = *reinterpret_cast<ElemSmem*>(smem_raw);
+    const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x;
     const int el = tid >> 3;
     const int t = tid & 7;
-    const int64_t e = p.e_begin + int64_t(blockIdx.x) * kEpc + el;
-    const bool valid = e < p.e_end;
+    const int64_t e_raw = p.e_begin + int64_t(blockIdx.x) * kEpc + el;
+    const bool valid = e_raw < p.e_end;
+    const int64_t e = valid ? e_raw : p.e_end - 1;   // the lanes of absent elements repeat the last one
 
     for (int k = tid; k < 8 * 8 * 3; k += kElemThreads) s.dnr[k / 24][k % 24] = (&p.tab.dnr[0][0][0])[k];
-    if (valid) {
-        const int* cn = reinterpret_cast<const int*>(p.conn4) + 8 * e;
-        const int node = __ldg(cn + t);
-        s.x[el][t][0] = __ldg(p.xyz + 3 * int64_t(node) + 0);
-        s.x[el][t][1] = __ldg(p.xyz + 3 * int64_t(node) + 1);
-        s.x[el][t][2] = __ldg(p.xyz + 3 * int64_t(node) + 2);
+    double c[3];
+    {
+        const int64_t node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = __ldg(p.xyz + 3 * node + i);
     }
-    __syncthreads();
-
-    // ---- coefficient t of the trilinear map, and W x_t ---------------------------------
-    if (valid) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s.wx[el][t][i] = p.wc[i][0] * c[0] + p.wc[i][1] * c[1] + p.wc[i][2] * c[2];
+    // element-local coordinates (no offset to cancel), then Walsh sums over the corners,
+    // W_s = sum_a (-1)^popc(s & a) x_a on lane s.  The natural coordinates are negative at corners
+    // {1,2,5,6} (xi), {2,3,6,7} (eta), {0,1,2,3} (zeta) (FEM_model_bsr.py:371-382), so 8 c_k is W_3 for xi,
+    // W_2 for eta, -W_4 for zeta, W_1 for xi eta, -W_6 for eta zeta, -W_7 for xi zeta, -W_5 for xi eta zeta.
+#pragma unroll
+    for (int i = 0; i < 3; ++i) c[i] -= __shfl_sync(full, c[i], tid & 24);
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1)
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            s.wx[el][t][i] = p.wc[i][0] * s.x[el][t][0] + p.wc[i][1] * s.x[el][t][1] + p.wc[i][2] * s.x[el][t][2];
-            s.xl[el][t][i] = s.x[el][t][i] - s.x[el][0][i];   // element-local: no offset to cancel
+            const double o = __shfl_xor_sync(full, c[i], m);
+            c[i] = o + flip_sign(c[i], t & m);
         }
-    }
-    __syncthreads();
-    if (valid) {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            double acc = 0.0;
-#pragma unroll
-            for (int a = 1; a < 8; ++a) acc = fma(monomial_sign(t, a), s.xl[el][a][i], acc);
-            s.cf[el][t][i] = 0.125 * acc;
-        }
-    }
-    __syncthreads();
+    for (int i = 0; i < 3; ++i) s.cf[el][t][i] = flip_sign(c[i], t & 4);
+    __syncthreads();  // the shape table is shared by the block's warps
 
     // ---- phase A: Gauss point g = t ------------------------------------------------
-    if (valid) {
+    {
         const int g = t;
         // Gauss point coordinates in the reference's order (zeta fastest, FEM_model_bsr.py:425-432)
         const double xi = (g & 4) ? kGS1 : -kGS1, et = (g & 2) ? kGS1 : -kGS1, ze = (g & 1) ? kGS1 : -kGS1;
+        const double(*f)[3] = s.cf[el];
+        // 8 J: of the two lanes that share column d the one on the negative side of direction d forms
+        // components 0 and 1, the other 2
         double J[3][3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double c1 = s.cf[el][1][i], c2 = s.cf[el][2][i], c3 = s.cf[el][3][i], c4 = s.cf[el][4][i];
-            const double c5 = s.cf[el][5][i], c6 = s.cf[el][6][i], c7 = s.cf[el][7][i];
-            J[i][0] = fma(ze, fma(et, c7, c6), fma(et, c4, c1));   // dx/dxi
-            J[i][1] = fma(ze, fma(xi, c7, c5), fma(xi, c4, c2));   // dx/deta
-            J[i][2] = fma(et, fma(xi, c7, c5), fma(xi, c6, c3));   // dx/dzeta
+        for (int d = 0; d < 3; ++d) {
+            const int bit = d == 0 ? 4 : d == 1 ? 2 : 1;
+            const bool up = (g & bit) != 0;
+            double v[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int i = up ? 2 : k;
+                if (d == 0) v[k] = fma(ze, fma(et, f[5][i], f[7][i]), fma(et, f[1][i], f[3][i]));        // dx/dxi
+                else if (d == 1) v[k] = fma(ze, fma(xi, f[5][i], f[6][i]), fma(xi, f[1][i], f[2][i]));   // dx/deta
+                else v[k] = fma(et, fma(xi, f[5][i], f[6][i]), fma(xi, f[7][i], f[4][i]));               // dx/dzeta
+            }
+            const double o0 = __shfl_xor_sync(full, v[0], bit), o1 = __shfl_xor_sync(full, v[1], bit);
+            J[0][d] = up ? o0 : v[0];
+            J[1][d] = up ? o1 : v[1];
+            J[2][d] = up ? v[0] : o0;
         }
         double A[3][3];  // adjugate: inverse(J) = A / det
 #pragma unroll
@@ -179,54 +199,51 @@ __global__ void __launch_bounds__(kElemThreads, 3) k_hex8_element(const ElemPara
                 A[j][i] = J[i1][j1] * J[i2][j2] - J[i2][j1] * J[i1][j2];
             }
         const double det = J[0][0] * A[0][0] + J[1][0] * A[0][1] + J[2][0] * A[0][2];
-        const double inv = 1.0 / det;
+        const double sc = p.mu8 / det;
 #pragma unroll
         for (int a = 0; a < 8; ++a)
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                const double r =
-                    s.dnr[g][3 * a] * A[0][i] + s.dnr[g][3 * a + 1] * A[1][i] + s.dnr[g][3 * a + 2] * A[2][i];
+                const double r = fma(s.dnr[g][3 * a + 2], A[2][i],
+                                     fma(s.dnr[g][3 * a + 1], A[1][i], s.dnr[g][3 * a] * A[0][i]));
                 s.R[el][g][3 * a + i] = r;
-                s.Rs[el][g][3 * a + i] = r * inv;
+                s.Rs[el][g][3 * a + i] = r * sc;
             }
         s.det[el][g] = det;
     }
-    __syncthreads();
+    __syncwarp();
 
     // ---- mass, M_ab = DE sum_g det_g N_a(g) N_b(g), by sum factorisation ------------------
     // N_a(g) is a product of one 1D factor per axis, so M_ab depends on the class of (a, b) per
     // axis only: contract the 8 det_g along x (D1: 3 classes x 4 (y, z) points), y (D2: 9 x 2),
-    // z (D3: 27 classes), 141 FP64 operations instead of 36 pairs x 8 Gauss points.
+    // z (D3: 27 classes), 114 FP64 operations instead of 36 pairs x 8 Gauss points.
     {
-        double* D1 = &s.x[el][0][0];
-        double* D2 = &s.xl[el][0][0];
-        double* D3 = &s.m[el][0];
-        if (valid)
-            for (int i = t; i < 12; i += 8) {
-                const int c = i >> 2, gyz = i & 3;
-                D1[i] = fma(s.det[el][4 + gyz], p.tm[1][c], s.det[el][gyz] * p.tm[0][c]);
-            }
-        __syncthreads();
-        if (valid)
-            for (int i = t; i < 18; i += 8) {
-                const int cx = i / 6, r = i - 6 * cx, cy = r >> 1, gz = r & 1;
-                D2[i] = fma(D1[cx * 4 + 2 + gz], p.tm[1][cy], D1[cx * 4 + gz] * p.tm[0][cy]);
-            }
-        __syncthreads();
-        if (valid)
-            for (int i = t; i < 27; i += 8) {
-                const int cxy = i / 3, cz = i - 3 * cxy;
-                D3[i] = p.DE * fma(D2[cxy * 2 + 1], p.tm[1][cz], D2[cxy * 2] * p.tm[0][cz]);
-            }
-        __syncthreads();
+        double* D1 = &s.cf[el][0][0];
+        double* D2 = s.d2[el];
+        double* D3 = s.m[el];
+        for (int i = t; i < 12; i += 8) {
+            const int cx = i >> 2, gyz = i & 3;
+            D1[i] = fma(s.det[el][4 + gyz], p.tmx[1][cx], s.det[el][gyz] * p.tmx[0][cx]);
+        }
+        __syncwarp();
+        for (int i = t; i < 18; i += 8) {
+            const int cx = i / 6, r = i - 6 * cx, cy = r >> 1, gz = r & 1;
+            D2[i] = fma(D1[cx * 4 + 2 + gz], p.tm[1][cy], D1[cx * 4 + gz] * p.tm[0][cy]);
+        }
+        __syncwarp();
+        for (int i = t; i < 27; i += 8) {
+            const int cxy = i / 3, cz = i - 3 * cxy;
+            D3[i] = fma(D2[cxy * 2 + 1], p.tm[1][cz], D2[cxy * 2] * p.tm[0][cz]);
+        }
+        __syncwarp();
     }
 
     // ---- phase B: node pairs -----------------------------------------------------------
-    double* rec = p.rec + (valid ? e : 0) * kRec;
-    const double lam = p.lam, mu = p.mu, D0d = p.D0d;
+    double* rec = p.rec + e * kRec;
+    const double lm = p.lm, lm1 = p.lm + 1.0;
     // diagonal pair (t, t): P symmetric
-    if (valid) {
-        const int a = t, pi = pair_index(a, a);
+    {
+        const int a = t;
         double P00 = 0, P11 = 0, P22 = 0, P01 = 0, P02 = 0, P12 = 0;
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
@@ -239,52 +256,42 @@ __global__ void __launch_bounds__(kElemThreads, 3) k_hex8_element(const ElemPara
             P02 = fma(q0, r2, P02);
             P12 = fma(q1, r2, P12);
         }
-        const double lm = lam + mu;
-        double* o = rec + kPairStride * pi - 2 * a;  // pair_offset(a, a)
-        o[0] = D0d * P00 + mu * (P11 + P22);
-        o[1] = D0d * P11 + mu * (P00 + P22);
-        o[2] = D0d * P22 + mu * (P00 + P11);
-        o[3] = lm * P01;
-        o[4] = lm * P02;
-        o[5] = lm * P12;
-        o[6] = s.m[el][mass_class(a, a)];
-        o[7] = 0.0;  // the unused slot: whole 32-byte sectors written, none read back from DRAM
+        const double tr = P00 + P11 + P22;
+        if (valid) {
+            double2* o = reinterpret_cast<double2*>(rec + kPairStride * pair_index(a, a) - 2 * a);  // pair_offset(a, a)
+            o[0] = make_double2(fma(lm1, P00, tr), fma(lm1, P11, tr));
+            o[1] = make_double2(fma(lm1, P22, tr), lm1 * P01);
+            o[2] = make_double2(lm1 * P02, lm1 * P12);
+            // the unused slot: whole 32-byte sectors written, none read back from DRAM
+            o[3] = make_double2(s.m[el][mass_class(a, a)], 0.0);
+        }
     }
     // off-diagonal pairs
-    for (int q = t; q < 28 && valid; q += 8) {
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const bool shared_pair = i == 3;   // the last four pairs: two threads, four Gauss points each
         int a, b;
-        offdiag_pair(q, a, b);
-        const int pi = pair_index(a, b);
-        double P[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        offdiag_pair(shared_pair ? 24 + (t >> 1) : 8 * i + t, a, b);
+        double P[9];
+        if (shared_pair) {
+            gram(s, el, a, b, 4 * (t & 1), 4, P);
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-            const double q0 = s.Rs[el][g][3 * a], q1 = s.Rs[el][g][3 * a + 1], q2 = s.Rs[el][g][3 * a + 2];
-            const double r0 = s.R[el][g][3 * b], r1 = s.R[el][g][3 * b + 1], r2 = s.R[el][g][3 * b + 2];
-            P[0][0] = fma(q0, r0, P[0][0]);
-            P[0][1] = fma(q0, r1, P[0][1]);
-            P[0][2] = fma(q0, r2, P[0][2]);
-            P[1][0] = fma(q1, r0, P[1][0]);
-            P[1][1] = fma(q1, r1, P[1][1]);
-            P[1][2] = fma(q1, r2, P[1][2]);
-            P[2][0] = fma(q2, r0, P[2][0]);
-            P[2][1] = fma(q2, r1, P[2][1]);
-            P[2][2] = fma(q2, r2, P[2][2]);
+            for (int k = 0; k < 9; ++k) P[k] += __shfl_xor_sync(full, P[k], 1);
+        } else {
+            gram(s, el, a, b, 0, 8, P);
         }
-        double* o = rec + kPairStride * pi - 2 * (a + 1);  // pair_offset(a, b), a < b
-        o[0] = D0d * P[0][0] + mu * (P[1][1] + P[2][2]);
-        o[4] = D0d * P[1][1] + mu * (P[0][0] + P[2][2]);
-        o[8] = D0d * P[2][2] + mu * (P[0][0] + P[1][1]);
-        o[1] = lam * P[0][1] + mu * P[1][0];
-        o[2] = lam * P[0][2] + mu * P[2][0];
-        o[3] = lam * P[1][0] + mu * P[0][1];
-        o[5] = lam * P[1][2] + mu * P[2][1];
-        o[6] = lam * P[2][0] + mu * P[0][2];
-        o[7] = lam * P[2][1] + mu * P[1][2];
-        o[9] = s.m[el][mass_class(a, b)];
+        const double tr = P[0] + P[4] + P[8];
+        if (valid && !(shared_pair && (t & 1))) {
+            double2* o = reinterpret_cast<double2*>(rec + kPairStride * pair_index(a, b) - 2 * (a + 1));  // pair_offset
+            o[0] = make_double2(fma(lm1, P[0], tr), fma(lm, P[1], P[3]));
+            o[1] = make_double2(fma(lm, P[2], P[6]), fma(lm, P[3], P[1]));
+            o[2] = make_double2(fma(lm1, P[4], tr), fma(lm, P[5], P[7]));
+            o[3] = make_double2(fma(lm, P[6], P[2]), fma(lm, P[7], P[5]));
+            o[4] = make_double2(fma(lm1, P[8], tr), s.m[el][mass_class(a, b)]);
+        }
     }
     // element load for corner t: F_t = sum_b M_tb W x_b (the mass blocks of the other threads'
     // pairs come through shared memory)
-    __syncthreads();
     if (valid) {
         double f0 = 0, f1 = 0, f2 = 0;
 #pragma unroll
@@ -819,10 +826,8 @@ int launch_hex8_element(const fem_mesh* mesh, const fem_material* mat, void* wor
     ep.e_end = e_end;
     ep.rec = static_cast<double*>(workspace);
     const double EX = mat->EX, PO = mat->PO;
-    ep.DE = mat->DE;
-    ep.D0d = EX * (1 - PO) / (1 + PO) / (1 - 2 * PO);  // FEM_model_bsr.py:435-437
-    ep.lam = EX * PO / (1 + PO) / (1 - 2 * PO);         // :439-445
-    ep.mu = EX / 2 / (1 + PO);                          // :447-449
+    ep.lm = 2 * PO / (1 - 2 * PO);   // FEM_model_bsr.py:435-449: D0 = lam + 2 mu and lam, D1 = mu
+    ep.mu8 = EX / 2 / (1 + PO) / 8;
     {
         const double w0 = mat->omega[0], w1 = mat->omega[1], w2 = mat->omega[2];
         const double wc[3][3] = {{w1 * w1 + w2 * w2, -w0 * w1, -w0 * w2},   // UnitVectorF, FEM_model_bsr.py:291-300
@@ -838,7 +843,10 @@ int launch_hex8_element(const fem_mesh* mesh, const fem_material* mat, void* wor
         const double al = 0.5 * (1.0 + kGS1), be = 0.5 * (1.0 - kGS1);
         const double tm[2][3] = {{al * al, al * be, be * be}, {be * be, al * be, al * al}};
         for (int sd = 0; sd < 2; ++sd)
-            for (int c = 0; c < 3; ++c) ep.tm[sd][c] = tm[sd][c];
+            for (int c = 0; c < 3; ++c) {
+                ep.tm[sd][c] = tm[sd][c];
+                ep.tmx[sd][c] = mat->DE / 512 * tm[sd][c];
+            }
     }
     const size_t smem = sizeof(ElemSmem);
     FEM_CUDA(cudaFuncSetAttribute(k_hex8_element, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
