@@ -315,7 +315,8 @@ class DeviceSystem:
         if self._ws is None or self._ws.numel() < nbytes:
             self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         opts = FemPcgOpts(Rp, int(mixed), float(rtol), int(maxit), float(inner_rtol), int(inner_maxit),
-                          int(max_outer), int(use_graph), int(unroll), self.variant(False, Rp),
+                          int(max_outer), int(use_graph), int(unroll),
+                          0 if mixed else self.variant(False, Rp),   # a mixed solve has no FP64 product to tune
                           self.variant(True, Rp) if mixed else 0,
                           _lib.RESIDUAL_EXTRA if residual == "extra" else _lib.RESIDUAL_FP64, int(stall_window))
         st = FemPcgStats()
