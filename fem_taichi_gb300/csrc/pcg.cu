@@ -36,8 +36,8 @@ using namespace pcgd;
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restrict__ M, const T* __restrict__ b,
                                                     T* x, T* r, double* part, PcgState* st, double rtol, int maxit) {
-    double v[2] = {0.0, 0.0};
-    Dot<T> d_rz, d_rr;
+    Dot<T> v[2];
+    Dot<T>&d_rz = v[0], &d_rr = v[1];
     const int64_t total_t = n * R;
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < ((total_t + 31) / 32) * 32;
          t += int64_t(gridDim.x) * blockDim.x) {
@@ -62,8 +62,6 @@ __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restric
             d_rr.add(r2, r2);
         }
     }
-    v[0] = d_rz.value();
-    v[1] = d_rr.value();
     if (!block_partials<R, 2>(v, part, &st->ticket)) return;
     __shared__ double tot[2][kMaxR];
     last_block_totals<R, 2>(part, gridDim.x, tot);
@@ -143,6 +141,40 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
     }
 }
 
+// The same for one FP32 right-hand side with p of 4 floats a node.
+__global__ void __launch_bounds__(kThreads) k_xp_update_pad(int64_t n, const float* __restrict__ M,
+                                                             const float* __restrict__ r, float* x, float4* p,
+                                                             const PcgState* __restrict__ st) {
+    if (st->done) return;
+    const bool first = st->it == 0;
+    const float a = float(st->alpha[0]), b = float(st->beta[0]);
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        float z0, z1, z2;
+        apply_block(M + 9 * i, r[3 * i], r[3 * i + 1], r[3 * i + 2], z0, z1, z2);
+        if (!first) {
+            const float4 o = p[i];
+            x[3 * i] += a * o.x;
+            x[3 * i + 1] += a * o.y;
+            x[3 * i + 2] += a * o.z;
+            z0 += b * o.x;
+            z1 += b * o.y;
+            z2 += b * o.z;
+        }
+        p[i] = make_float4(z0, z1, z2, 0.f);
+    }
+}
+__global__ void __launch_bounds__(kThreads) k_x_finish_pad(int64_t n, const float4* __restrict__ p, float* x,
+                                                            const PcgState* __restrict__ st) {
+    if (st->it == 0) return;
+    const float a = float(st->alpha[0]);
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        const float4 o = p[i];
+        x[3 * i] += a * o.x;
+        x[3 * i + 1] += a * o.y;
+        x[3 * i + 2] += a * o.z;
+    }
+}
+
 // The last iteration's x += alpha p, whatever ended the solve (nothing pending when it took no step).
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_x_finish(int64_t nv, const T* __restrict__ p, T* x,
@@ -167,12 +199,15 @@ __global__ void __launch_bounds__(kThreads) k_p_update(int64_t nv, const T* __re
 // q = A p and p.q -> alpha = rz / pq on the device.  (Folding p = z + beta p into this
 // kernel as q = A z + beta q was measured slower: the row epilogue's extra loads sit on the
 // product's critical path, and the recurrence drifts from A p in FP32.)
-template <typename T, int R, int LPR>
+// kPad (FP32, one right-hand side, padded row-SoA matrix): p holds 4 floats a node.
+template <typename T, int R, int LPR, bool kPad>
 __global__ void __launch_bounds__(kThreads, spmm_ctas<T, R>())
     k_spmv_pq(const BsrView<T> A, const T* __restrict__ p, T* __restrict__ q, double* part, PcgState* st) {
     if (st->done) return;
-    double v[1];
-    if constexpr (R == 1)
+    Dot<T> v[1];
+    if constexpr (kPad)
+        v[0] = spmv4_rows_epi<(LPR > 8 ? 8 : LPR), true>(A, p, StoreYPad{p, q});
+    else if constexpr (R == 1)
         v[0] = spmv1_rows<T, LPR>(A, p, q, true);
     else
         v[0] = spmm_rows<T, R>(A, p, q, true);
@@ -205,8 +240,8 @@ template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __restrict__ M, const T* __restrict__ q,
                                                         T* r, double* part, PcgState* st) {
     if (st->done) return;
-    double v[2] = {0.0, 0.0};
-    Dot<T> d_rz, d_rr;
+    Dot<T> v[2];
+    Dot<T>&d_rz = v[0], &d_rr = v[1];
     const int64_t total_t = n * R;
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < ((total_t + 31) / 32) * 32;
          t += int64_t(gridDim.x) * blockDim.x) {
@@ -229,8 +264,6 @@ __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __res
             d_rr.add(r2, r2);
         }
     }
-    v[0] = d_rz.value();
-    v[1] = d_rr.value();
     if (block_partials<R, 2>(v, part, &st->ticket)) {
         __shared__ double tot[2][kMaxR];
         last_block_totals<R, 2>(part, gridDim.x, tot);
@@ -274,8 +307,8 @@ __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __res
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_init_r(int64_t nv, const T* __restrict__ b, T* x, T* r, float* r32,
                                                       double* part, PcgState* st, double rtol, int maxit) {
-    double v[1];
-    Dot<T> d_rr;
+    Dot<T> v[1];
+    Dot<T>& d_rr = v[0];
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
          e += int64_t(gridDim.x) * blockDim.x) {
         if (e < nv) {
@@ -286,7 +319,6 @@ __global__ void __launch_bounds__(kThreads) k_init_r(int64_t nv, const T* __rest
             d_rr.add(b0, b0);
         }
     }
-    v[0] = d_rr.value();
     if (!block_partials<R, 1>(v, part, &st->ticket)) return;
     __shared__ double tot[1][kMaxR];
     last_block_totals<R, 1>(part, gridDim.x, tot);
@@ -318,8 +350,8 @@ template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_update_r(int64_t nv, const T* __restrict__ p, const T* __restrict__ q,
                                                         T* x, T* r, float* r32, double* part, PcgState* st) {
     if (st->done) return;
-    double v[1];
-    Dot<T> d_rr;
+    Dot<T> v[1];
+    Dot<T>& d_rr = v[0];
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
          e += int64_t(gridDim.x) * blockDim.x) {
         if (e < nv) {
@@ -331,7 +363,6 @@ __global__ void __launch_bounds__(kThreads) k_update_r(int64_t nv, const T* __re
             d_rr.add(r0, r0);
         }
     }
-    v[0] = d_rr.value();
     if (block_partials<R, 1>(v, part, &st->ticket)) {
         __shared__ double tot[1][kMaxR];
         last_block_totals<R, 1>(part, gridDim.x, tot);
@@ -366,8 +397,8 @@ template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_rz(int64_t nv, const T* __restrict__ r, T* z, const float* z32,
                                                   const T* __restrict__ q, double* part, PcgState* st) {
     if (st->done) return;
-    double v[2];
-    Dot<T> d_rz, d_qz;
+    Dot<T> v[2];
+    Dot<T>&d_rz = v[0], &d_qz = v[1];
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
          e += int64_t(gridDim.x) * blockDim.x) {
         if (e < nv) {
@@ -382,8 +413,6 @@ __global__ void __launch_bounds__(kThreads) k_rz(int64_t nv, const T* __restrict
             if (q) d_qz.add(q[e], ze);
         }
     }
-    v[0] = d_rz.value();
-    v[1] = d_qz.value();
     if (block_partials<R, 2>(v, part, &st->ticket)) {
         __shared__ double tot[2][kMaxR];
         last_block_totals<R, 2>(part, gridDim.x, tot);
@@ -409,29 +438,6 @@ __global__ void __launch_bounds__(kThreads) k_rz(int64_t nv, const T* __restrict
 }
 
 // ---- FP64 refinement helpers --------------------------------------------------------------
-// r = b - y (y = A u computed by the SpMV), norms of r per RHS -> st->norm2.
-template <int R>
-__global__ void __launch_bounds__(kThreads) k_residual(int64_t nv, const double* __restrict__ b,
-                                                        const double* __restrict__ y, double* r, double* part,
-                                                        PcgState* st) {
-    double v[1] = {0.0};
-    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
-         e += int64_t(gridDim.x) * blockDim.x) {
-        if (e < nv) {
-            const double d = b[e] - y[e];
-            r[e] = d;
-            v[0] += d * d;
-        }
-    }
-    if (block_partials<R, 1>(v, part, &st->ticket)) {
-        __shared__ double tot[1][kMaxR];
-        last_block_totals<R, 1>(part, gridDim.x, tot);
-        if (threadIdx.x < R) st->norm2[threadIdx.x] = tot[0][threadIdx.x];
-        __syncthreads();
-        if (threadIdx.x == 0) st->ticket = 0;
-    }
-}
-
 // True residual r = F - A u per scalar row with its rounding scale |F| + |A||u|; per RHS
 // ||r||^2 -> st->norm2 and || |F| + |A||u| ||^2 -> st->anorm2.  kExtra: each row sum is the
 // compensated dot product "Dot2" of Ogita, Rump and Oishi (SIAM J. Sci. Comput. 26 (2005)
@@ -444,7 +450,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
                                                           const double* __restrict__ u, double* r, double* part,
                                                           PcgState* st) {
     const int64_t nv = 3 * A.n * R;
-    double v[2] = {0.0, 0.0};
+    Dot<double> v[2];
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
          e += int64_t(gridDim.x) * blockDim.x) {
         if (e < nv) {
@@ -479,8 +485,8 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
             }
             const double rv = kExtra ? __dadd_rn(s, comp) : s;
             r[e] = rv;
-            v[0] = fma(rv, rv, v[0]);
-            v[1] = fma(sc, sc, v[1]);
+            v[0].add(rv, rv);
+            v[1].add(sc, sc);
         }
     }
     if (block_partials<R, 2>(v, part, &st->ticket)) {
@@ -490,6 +496,29 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
             st->norm2[threadIdx.x] = tot[0][threadIdx.x];
             st->anorm2[threadIdx.x] = tot[1][threadIdx.x];
         }
+        __syncthreads();
+        if (threadIdx.x == 0) st->ticket = 0;
+    }
+}
+
+// The true residual of u = 0: r = F (r may be F itself), and its norms as k_residual_ex gives them
+// with an empty row.
+template <int R>
+__global__ void __launch_bounds__(kThreads) k_residual_zero(int64_t nv, const double* __restrict__ F, double* r,
+                                                            double* part, PcgState* st) {
+    Dot<double> v[1];
+    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
+         e += int64_t(gridDim.x) * blockDim.x) {
+        if (e < nv) {
+            const double f = F[e];
+            if (r) r[e] = f;
+            v[0].add(f, f);
+        }
+    }
+    if (block_partials<R, 1>(v, part, &st->ticket)) {
+        __shared__ double tot[1][kMaxR];
+        last_block_totals<R, 1>(part, gridDim.x, tot);
+        if (threadIdx.x < R) st->norm2[threadIdx.x] = st->anorm2[threadIdx.x] = tot[0][threadIdx.x];
         __syncthreads();
         if (threadIdx.x == 0) st->ticket = 0;
     }
@@ -548,7 +577,8 @@ Layout layout(int64_t n, int R, int mixed) {
     L.state = take(sizeof(PcgState));
     L.part = take(sizeof(double) * kMaxCtas * kSlots * kMaxR);
     for (int i = 0; i < 6; ++i) L.v64[i] = take(mixed ? (i < 2 ? sizeof(double) * nv : 0) : sizeof(double) * nv);
-    for (int i = 0; i < 6; ++i) L.v32[i] = take(mixed ? sizeof(float) * nv : 0);
+    // v32[4], the search direction: 4 floats a node for one right-hand side
+    for (int i = 0; i < 6; ++i) L.v32[i] = take(mixed ? sizeof(float) * (R == 1 && i == 4 ? size_t(4) * n : nv) : 0);
     L.m32 = take(mixed ? sizeof(float) * 9 * n : 0);
     L.scale = take(sizeof(double) * kMaxR);
     L.total = off;
@@ -566,7 +596,7 @@ unsigned vec_grid(Kernel kernel, int64_t work) {
 // Grid of the product kernel: one wave of resident CTAs (grid-stride rows), at most kMaxCtas
 // (the size of the partial-sum buffer).  The grid fixes each row's CTA, hence the order of the
 // dot-product partial sums.
-template <typename T, int R>
+template <typename T, int R, bool kPad = false>
 void launch_spmv_pq(const BsrView<T>& A, const T* p, T* q, double* part, PcgState* st, int variant, cudaStream_t s) {
     auto run = [&](auto kernel, int64_t rows_per_cta, int64_t cap) {
         const unsigned g = resident_grid(reinterpret_cast<const void*>(kernel), kThreads,
@@ -574,20 +604,23 @@ void launch_spmv_pq(const BsrView<T>& A, const T* p, T* q, double* part, PcgStat
         kernel<<<g, kThreads, 0, s>>>(A, p, q, part, st);
     };
     if constexpr (R > 1) {
-        run(k_spmv_pq<T, R, 0>, int64_t(kThreads / 32) * (A.rsoa == 2 ? 1 : 32 / R), int64_t(sm_count()) * 8);
+        run(k_spmv_pq<T, R, 0, false>, int64_t(kThreads / 32) * (A.rsoa == 2 ? 1 : 32 / R), int64_t(sm_count()) * 8);
     } else {
         const SpmvVariant v = spmv_variant(variant);
         const int64_t rows_per_cta = int64_t(kThreads / 32) * (32 / v.lpr);
         const int64_t cap = int64_t(sm_count()) * (v.ctas_per_sm * v.threads / kThreads);
         switch (v.lpr) {
-            case 32: run(k_spmv_pq<T, 1, 32>, rows_per_cta, cap); break;
-            case 16: run(k_spmv_pq<T, 1, 16>, rows_per_cta, cap); break;
-            case 8: run(k_spmv_pq<T, 1, 8>, rows_per_cta, cap); break;
-            case 4: run(k_spmv_pq<T, 1, 4>, rows_per_cta, cap); break;
-            default: run(k_spmv_pq<T, 1, 2>, rows_per_cta, cap); break;
+            case 32: run(k_spmv_pq<T, 1, 32, kPad>, rows_per_cta, cap); break;
+            case 16: run(k_spmv_pq<T, 1, 16, kPad>, rows_per_cta, cap); break;
+            case 8: run(k_spmv_pq<T, 1, 8, kPad>, rows_per_cta, cap); break;
+            case 4: run(k_spmv_pq<T, 1, 4, kPad>, rows_per_cta, cap); break;
+            default: run(k_spmv_pq<T, 1, 2, kPad>, rows_per_cta, cap); break;
         }
     }
 }
+
+// One FP32 right-hand side on the padded row-SoA copy: the search direction has 4 floats a node.
+inline bool pad_direction(const BsrView<float>& A) { return A.rsoa == 2; }
 
 template <typename T, int R>
 int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* p, T* q, double* part, PcgState* st, int variant,
@@ -596,6 +629,15 @@ int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* p, T* q, d
     // start on 16-byte boundaries
     constexpr int V = R % (16 / int(sizeof(T))) == 0 ? 16 / int(sizeof(T)) : 1;
     for (int i = 0; i < count; ++i) {
+        if constexpr (sizeof(T) == 4 && R == 1) {
+            if (pad_direction(A)) {
+                k_xp_update_pad<<<vec_grid(k_xp_update_pad, A.n), kThreads, 0, s>>>(A.n, M, r, x,
+                                                                                      reinterpret_cast<float4*>(p), st);
+                launch_spmv_pq<T, R, true>(A, p, q, part, st, variant, s);
+                k_r_update<T, R><<<vec_grid(k_r_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, q, r, part, st);
+                continue;
+            }
+        }
         if (aligned16(x))
             k_xp_update<T, R, V><<<vec_grid(k_xp_update<T, R, V>, A.n * (R / V)), kThreads, 0, s>>>(A.n, M, r, x, p, st);
         else
@@ -687,6 +729,14 @@ int pcg_core(const BsrView<T>& A, const T* M, const T* b, T* x, T* r, T* p, T* q
     };
     int rc = pcg_drive(init, iters, st, maxit, use_graph, unroll, s, res, stall);
     if (rc) return rc;
+    if constexpr (sizeof(T) == 4 && R == 1) {
+        if (pad_direction(A)) {
+            k_x_finish_pad<<<vec_grid(k_x_finish_pad, A.n), kThreads, 0, s>>>(A.n, reinterpret_cast<const float4*>(p), x,
+                                                                               st);
+            FEM_LAUNCH_CHECK("k_x_finish");
+            return FEM_OK;
+        }
+    }
     const int64_t nv = 3 * A.n * R;
     k_x_finish<T, R><<<vec_grid(k_x_finish<T, R>, nv), kThreads, 0, s>>>(nv, p, x, st);
     FEM_LAUNCH_CHECK("k_x_finish");
@@ -761,13 +811,10 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
     FEM_CUDA(cudaMemsetAsync(st, 0, sizeof(PcgState), s));
     double bnorm[kMaxR];
     {
-        // ||F_k||: the residual of u = 0
-        double* z0 = reinterpret_cast<double*>(ws + L.v64[0]);
-        double* r0 = reinterpret_cast<double*>(ws + L.v64[1]);
-        k_zero<<<vec_grid(k_zero, nv), kThreads, 0, s>>>(nv, z0);
-        FEM_LAUNCH_CHECK("k_zero");
-        k_residual_ex<R, false><<<vec_grid(k_residual_ex<R, false>, nv), kThreads, 0, s>>>(K64, F, z0, r0, part, st);
-        FEM_LAUNCH_CHECK("k_residual_ex");
+        // ||F_k||; a mixed solve starts from u = 0, whose residual F goes to its r64
+        double* r0 = o->mixed ? reinterpret_cast<double*>(ws + L.v64[1]) : nullptr;
+        k_residual_zero<R><<<vec_grid(k_residual_zero<R>, nv), kThreads, 0, s>>>(nv, F, r0, part, st);
+        FEM_LAUNCH_CHECK("k_residual_zero");
         FEM_CUDA(cudaMemcpyAsync(&h, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
         FEM_CUDA(cudaStreamSynchronize(s));
         for (int k = 0; k < R; ++k) bnorm[k] = sqrt(h.norm2[k]);
@@ -859,9 +906,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
         if (rc) return rc;
         k_zero<<<vec_grid(k_zero, nv), kThreads, 0, s>>>(nv, U);
         FEM_LAUNCH_CHECK("k_zero");
-        rc = true_residual(U, r64);
-        if (rc) return rc;
-        double prev = 1e300;
+        double prev = 1e300;   // h and r64 hold the residual of u = 0
         for (outer = 0; outer < max_outer; ++outer) {
             double sc[kMaxR];
             if (!set_active(sc)) break;

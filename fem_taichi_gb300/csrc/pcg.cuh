@@ -22,22 +22,14 @@ struct PcgState {
     unsigned ticket;
 };
 
-// Sum of v over the lanes of this warp that hold the same right-hand side (lane % R).
-template <int R>
-__device__ __forceinline__ double warp_rhs_sum(double v) {
-#pragma unroll
-    for (int off = 16; off >= R; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
-
 // This CTA's sums of v[s] (per RHS) into part[blockIdx.x] slots slot0 .. slot0 + NS - 1.
-template <int R, int NS>
-__device__ void write_partials(const double (&v)[NS], double* part, int slot0) {
+template <int R, int NS, typename T>
+__device__ void write_partials(const Dot<T> (&v)[NS], double* part, int slot0) {
     __shared__ double sm[kThreads / 32][NS][kMaxR];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-        const double w = warp_rhs_sum<R>(v[s]);
+        const double w = rhs_sum<R>(v[s]);
         if (lane < R) sm[warp][s][lane] = w;
     }
     __syncthreads();
@@ -53,10 +45,10 @@ __device__ void write_partials(const double (&v)[NS], double* part, int slot0) {
 
 // Block-level reduction of up to kSlots values per RHS into part[blockIdx.x]; returns true
 // in every thread of the CTA that finished last (after which part[] is complete).
-template <int R, int NS>
-__device__ bool block_partials(const double (&v)[NS], double* part, unsigned* ticket) {
+template <int R, int NS, typename T>
+__device__ bool block_partials(const Dot<T> (&v)[NS], double* part, unsigned* ticket) {
     __shared__ bool last;
-    write_partials<R, NS>(v, part, 0);
+    write_partials<R, NS, T>(v, part, 0);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
@@ -76,6 +68,7 @@ __device__ void last_block_totals(const double* part, int nblocks, double (&tot)
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         double acc = 0.0;
+#pragma unroll 4
         for (int b = g; b < nblocks; b += G) acc += __ldcg(part + (int64_t(b) * kSlots + slot0 + s) * kMaxR + k);
         red[s][t] = acc;
     }

@@ -50,6 +50,31 @@ struct Dot<float> {
     __device__ __forceinline__ double value() const { return double(s) + double(c); }
 };
 
+// Sum of d over the lanes of a warp that hold the same right-hand side (lane % R), as a double.  FP32
+// pairs are added as pairs (two-sums on the FP32 pipes; the FP64 form's five adds and the
+// conversions cost 16 FP64 cycles each per warp and SM).
+template <int R>
+__device__ __forceinline__ double rhs_sum(const Dot<double>& d) {
+    double v = d.value();
+#pragma unroll
+    for (int off = 16; off >= R; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+template <int R>
+__device__ __forceinline__ double rhs_sum(const Dot<float>& d) {
+    float s = d.s, c = d.c;
+#pragma unroll
+    for (int off = 16; off >= R; off >>= 1) {
+        const float s2 = __shfl_xor_sync(0xffffffffu, s, off), c2 = __shfl_xor_sync(0xffffffffu, c, off);
+        const float t = __fadd_rn(s, s2);
+        const float b = __fsub_rn(t, s);
+        const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(s2, b));
+        s = t;
+        c = __fadd_rn(__fadd_rn(c, c2), err);
+    }
+    return double(s) + double(c);
+}
+
 // BsrView::rsoa for a fem_bsr layout code
 inline int rsoa_kind(int layout) {
     return layout == FEM_LAYOUT_RSOA ? 1 : layout == FEM_LAYOUT_RSOA4 ? 2 : 0;
@@ -107,57 +132,112 @@ struct StoreY {
     }
 };
 
+// The same with x of 4 floats a node (y of 3).
+struct StoreYPad {
+    const float* x;
+    float* y;
+    __device__ __forceinline__ void operator()(int64_t o, int, int, float a0, float a1, float a2, Dot<float>& dot) const {
+        const float4 xr = __ldg(reinterpret_cast<const float4*>(x) + o / 3);
+        y[o] = a0;
+        y[o + 1] = a1;
+        y[o + 2] = a2;
+        dot.add(xr.x, a0);
+        dot.add(xr.y, a1);
+        dot.add(xr.z, a2);
+    }
+};
+
 // Padded row-SoA FP32 product: each lane takes 4 consecutive slots of its row per step and
 // reads each of the 9 values of those 4 blocks with one 16-byte load (rows, values and
-// slot groups all start on 16-byte boundaries); padding blocks hold zeros.
-template <int LPR, typename Epi>
-__device__ __forceinline__ double spmv4_rows_epi(const BsrView<float>& A, const float* __restrict__ x, const Epi& epi) {
+// slot groups all start on 16-byte boundaries); padding blocks hold zeros.  kPad: x holds 4 floats a
+// node, one 16-byte load per gather instead of three of 4 bytes.
+// Bound by HBM once the row pointer, the columns and the gathers no longer wait for one another: the
+// next row's columns and the pointer of the row after load while a row is summed (in line, 214,221 nodes took
+// 45.6 us of 34 us of HBM time whatever the occupancy; the solve of which it is two thirds went from 69.5 to
+// 66.3 us an iteration).
+template <int LPR, bool kPad, typename Epi>
+__device__ __forceinline__ Dot<float> spmv4_rows_epi(const BsrView<float>& A, const float* __restrict__ x,
+                                                     const Epi& epi) {
     const int lane = threadIdx.x & 31;
     const int sub = lane / LPR, sl = lane % LPR;
     constexpr int RPW = 32 / LPR;
     const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    const int64_t stride = ((int64_t(gridDim.x) * blockDim.x) >> 5) * RPW;
     Dot<float> dot;
-    for (int64_t base = warp * RPW; base < A.n; base += nwarps * RPW) {
-        const int64_t row = base + sub;
-        const bool valid = row < A.n;
+    auto pointers = [&](int64_t row, int& rs, int& L) {
+        rs = L = 0;
+        if (row < A.n) {
+            rs = __ldg(A.indptr + row);
+            L = __ldg(A.indptr + row + 1) - rs;
+        }
+    };
+    auto columns = [&](int rs, int L, int s) {
+        return s < L ? __ldg(reinterpret_cast<const int4*>(A.indices + rs + s)) : make_int4(0, 0, 0, 0);
+    };
+    int rs, L, rs_next, L_next;
+    int64_t row = warp * RPW + sub;
+    pointers(row, rs, L);
+    pointers(row + stride, rs_next, L_next);
+    int4 c = columns(rs, L, 4 * sl);
+    for (int64_t base = warp * RPW; base < A.n; base += stride, row += stride) {
         float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-        if (valid) {
-            const int64_t rs = __ldg(A.indptr + row);
-            const int Lp = __ldg(A.indptr + row + 1) - int(rs);
-            const float* v0 = A.vals + 9 * rs;
-            for (int s = 4 * sl; s < Lp; s += 4 * LPR) {
-                const int4 c = __ldg(reinterpret_cast<const int4*>(A.indices + rs + s));
-                float4 w[9];
+        auto step = [&](int s, const int4& cc4) {
+            const float* v0 = A.vals + 9 * int64_t(rs) + s;
+            const int cc[4] = {cc4.x, cc4.y, cc4.z, cc4.w};
+            float4 w[9], xv[4];
 #pragma unroll
-                for (int q = 0; q < 9; ++q) w[q] = __ldg(reinterpret_cast<const float4*>(v0 + int64_t(q) * Lp + s));
-                const int cc[4] = {c.x, c.y, c.z, c.w};
+            for (int j = 0; j < 4; ++j) {
+                if constexpr (kPad) {
+                    xv[j] = __ldg(reinterpret_cast<const float4*>(x) + cc[j]);
+                } else {
+                    const float* xc = x + 3 * int64_t(cc[j]);
+                    xv[j] = make_float4(xc[0], xc[1], xc[2], 0.f);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 9; ++q) w[q] = __ldg(reinterpret_cast<const float4*>(v0 + int64_t(q) * L));
+            return [=](float& b0, float& b1, float& b2) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     // component j of each value's float4 = slot s + j
                     auto wq = [&](int q) { return j == 0 ? w[q].x : j == 1 ? w[q].y : j == 2 ? w[q].z : w[q].w; };
-                    const float* xc = x + 3 * int64_t(cc[j]);
-                    const float x0 = xc[0], x1 = xc[1], x2 = xc[2];
-                    a0 += wq(0) * x0 + wq(1) * x1 + wq(2) * x2;
-                    a1 += wq(3) * x0 + wq(4) * x1 + wq(5) * x2;
-                    a2 += wq(6) * x0 + wq(7) * x1 + wq(8) * x2;
+                    b0 = fmaf(wq(0), xv[j].x, fmaf(wq(1), xv[j].y, fmaf(wq(2), xv[j].z, b0)));
+                    b1 = fmaf(wq(3), xv[j].x, fmaf(wq(4), xv[j].y, fmaf(wq(5), xv[j].z, b1)));
+                    b2 = fmaf(wq(6), xv[j].x, fmaf(wq(7), xv[j].y, fmaf(wq(8), xv[j].z, b2)));
                 }
-            }
+            };
+        };
+        int rs2, L2;
+        int4 c_next;
+        if (4 * sl < L) {
+            const auto add = step(4 * sl, c);   // loads issued
+            c_next = columns(rs_next, L_next, 4 * sl);
+            pointers(row + 2 * stride, rs2, L2);
+            add(a0, a1, a2);
+        } else {
+            c_next = columns(rs_next, L_next, 4 * sl);
+            pointers(row + 2 * stride, rs2, L2);
         }
+        for (int s = 4 * sl + 4 * LPR; s < L; s += 4 * LPR) step(s, columns(rs, L, s))(a0, a1, a2);
         a0 = group_sum<LPR>(a0);
         a1 = group_sum<LPR>(a1);
         a2 = group_sum<LPR>(a2);
-        if (valid && sl == 0) epi(3 * row, 1, 0, a0, a1, a2, dot);
+        if (row < A.n && sl == 0) epi(3 * row, 1, 0, a0, a1, a2, dot);
+        c = c_next;
+        rs = rs_next;
+        L = L_next;
+        rs_next = rs2;
+        L_next = L2;
     }
-    return dot.value();
+    return dot;
 }
 
 // One pass of A x over the rows assigned to this thread (LPR lanes per block row; one RHS);
 // returns this lane's share of the epilogue's dot product.
 template <typename T, int LPR, typename Epi>
-__device__ __forceinline__ double spmv1_rows_epi(const BsrView<T>& A, const T* __restrict__ x, const Epi& epi) {
+__device__ __forceinline__ Dot<T> spmv1_rows_epi(const BsrView<T>& A, const T* __restrict__ x, const Epi& epi) {
     if constexpr (sizeof(T) == 4) {
-        if (A.rsoa == 2) return spmv4_rows_epi<(LPR > 8 ? 8 : LPR)>(A, x, epi);
+        if (A.rsoa == 2) return spmv4_rows_epi<(LPR > 8 ? 8 : LPR), false>(A, x, epi);
     }
     const int lane = threadIdx.x & 31;
     const int sub = lane / LPR, sl = lane % LPR;
@@ -185,7 +265,7 @@ __device__ __forceinline__ double spmv1_rows_epi(const BsrView<T>& A, const T* _
         a2 = group_sum<LPR>(a2);
         if (valid && sl == 0) epi(3 * row, 1, 0, a0, a1, a2, dot);
     }
-    return dot.value();
+    return dot;
 }
 
 // Many right-hand sides on the padded row-SoA FP32 copy, one block row per warp (256 threads a CTA).
@@ -220,7 +300,7 @@ __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
 }
 
 template <int R, typename Epi>
-__device__ __forceinline__ double spmm4_rows_epi(const BsrView<float>& A, const float* __restrict__ x, const Epi& epi) {
+__device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, const float* __restrict__ x, const Epi& epi) {
     constexpr int V = R >= 16 ? 4 : R == 8 ? 2 : 1, LP = R / V, G = 32 / LP, CS = 4 * G;
     constexpr unsigned full = 0xffffffffu;
     constexpr int kWarps = 8;
@@ -362,13 +442,13 @@ __device__ __forceinline__ double spmm4_rows_epi(const BsrView<float>& A, const 
         for (int d = 0; d < kStage - 1; ++d) rs[d] = rs[d + 1], len[d] = len[d + 1];
     }
     asm volatile("cp.async.wait_all;");
-    return dot.value();
+    return dot;
 }
 
 // Many right-hand sides: lane = RHS (32 / R rows per warp), each block's values loaded once
 // per row group and applied to every RHS.
 template <typename T, int R, typename Epi>
-__device__ __forceinline__ double spmm_rows_epi(const BsrView<T>& A, const T* __restrict__ x, const Epi& epi) {
+__device__ __forceinline__ Dot<T> spmm_rows_epi(const BsrView<T>& A, const T* __restrict__ x, const Epi& epi) {
     if constexpr (sizeof(T) == 4) {
         // the vector loads of x need its rows on 16-byte boundaries (a caller's x may be a view)
         if (A.rsoa == 2 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) return spmm4_rows_epi<R>(A, x, epi);
@@ -395,18 +475,18 @@ __device__ __forceinline__ double spmm_rows_epi(const BsrView<T>& A, const T* __
         }
         epi(3 * row * R + rhs, R, rhs, a0, a1, a2, dot);
     }
-    return dot.value();
+    return dot;
 }
 
 // y = A x forms of the three products (dot: sum_rows x_i . y_i when want_dot).
 template <typename T, int LPR>
-__device__ __forceinline__ double spmv1_rows(const BsrView<T>& A, const T* __restrict__ x, T* __restrict__ y,
+__device__ __forceinline__ Dot<T> spmv1_rows(const BsrView<T>& A, const T* __restrict__ x, T* __restrict__ y,
                                              bool want_dot) {
     return spmv1_rows_epi<T, LPR>(A, x, StoreY<T>{x, y, want_dot});
 }
 
 template <typename T, int R>
-__device__ __forceinline__ double spmm_rows(const BsrView<T>& A, const T* __restrict__ x, T* __restrict__ y,
+__device__ __forceinline__ Dot<T> spmm_rows(const BsrView<T>& A, const T* __restrict__ x, T* __restrict__ y,
                                             bool want_dot) {
     return spmm_rows_epi<T, R>(A, x, StoreY<T>{x, y, want_dot});
 }
