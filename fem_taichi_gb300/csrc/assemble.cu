@@ -127,7 +127,7 @@ __device__ __forceinline__ void gram(const ElemSmem& s, int el, int a, int b, in
     }
 }
 
-__global__ void __launch_bounds__(kElemThreads, 3) k_hex8_element(const ElemParams p) {
+__global__ void __launch_bounds__(kElemThreads, 48 / kEpc) k_hex8_element(const ElemParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ElemSmem& s = *reinterpret_cast<ElemSmem*>(smem_raw);
     const unsigned full = 0xffffffffu;
@@ -304,6 +304,183 @@ __global__ void __launch_bounds__(kElemThreads, 3) k_hex8_element(const ElemPara
         rec[kFOff + 3 * t + 0] = f0;
         rec[kFOff + 3 * t + 1] = f1;
         rec[kFOff + 3 * t + 2] = f2;
+    }
+}
+
+// The same records with a warp per element, for meshes too small to fill the SMs: one SMSP takes a
+// FP64 warp instruction every 64 cycles, so the 566 of k_hex8_element are 18 us however few warps
+// there are; spread over 32 lanes they are about 230 (the 28 off-diagonal pairs in one round; gradients,
+// diagonal pairs and loads in quarters; the geometry of a Gauss point repeated by 4 lanes).  In total
+// that is 1.6 times the work, so the rule of launch_hex8_element stops where the device is full.
+// Lane = (quarter h, corner or Gauss point t).
+constexpr int kWideEpc = 4;
+constexpr int kWidePerSm = 16;   // elements per SM up to which it is taken (see launch_hex8_element)
+struct WideSmem {
+    double dnr[8][kRPad];
+    double cf[kWideEpc][8][3];
+    double wx[kWideEpc][8][3];
+    double R[kWideEpc][8][kRPad];
+    double Rs[kWideEpc][8][kRPad];
+    double det[kWideEpc][8];
+    double d1[kWideEpc][12], d2[kWideEpc][18];
+    double m[kWideEpc][36];
+};
+
+__global__ void __launch_bounds__(kWideEpc * 32) k_hex8_element_wide(const ElemParams p) {
+    __shared__ WideSmem s;
+    const unsigned full = 0xffffffffu;
+    const int tid = threadIdx.x, el = tid >> 5, lane = tid & 31, t = lane & 7, h = lane >> 3;
+    const int64_t e_raw = p.e_begin + int64_t(blockIdx.x) * kWideEpc + el;
+    const bool valid = e_raw < p.e_end;
+    const int64_t e = valid ? e_raw : p.e_end - 1;
+    for (int k = tid; k < 8 * 8 * 3; k += kWideEpc * 32) s.dnr[k / 24][k % 24] = (&p.tab.dnr[0][0][0])[k];
+    double c[3];
+    {
+        const int64_t node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = __ldg(p.xyz + 3 * node + i);
+    }
+    if (h < 3) s.wx[el][t][h] = p.wc[h][0] * c[0] + p.wc[h][1] * c[1] + p.wc[h][2] * c[2];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) c[i] -= __shfl_sync(full, c[i], lane & 24);
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double o = __shfl_xor_sync(full, c[i], m);
+            c[i] = o + flip_sign(c[i], t & m);
+        }
+    if (h == 0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) s.cf[el][t][i] = flip_sign(c[i], t & 4);
+    }
+    __syncthreads();
+    {
+        const int g = t;
+        const double xi = (g & 4) ? kGS1 : -kGS1, et = (g & 2) ? kGS1 : -kGS1, ze = (g & 1) ? kGS1 : -kGS1;
+        const double(*f)[3] = s.cf[el];
+        // 8 J: quarter h < 3 forms component h
+        double d[3];
+        {
+            const int i = h < 3 ? h : 0;
+            const double m = fma(xi, f[5][i], f[6][i]);
+            d[0] = fma(ze, fma(et, f[5][i], f[7][i]), fma(et, f[1][i], f[3][i]));
+            d[1] = fma(ze, m, fma(xi, f[1][i], f[2][i]));
+            d[2] = fma(et, m, fma(xi, f[7][i], f[4][i]));
+        }
+        double J[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) J[i][k] = __shfl_sync(full, d[k], 8 * i + t);
+        double A[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+                A[j][i] = J[i1][j1] * J[i2][j2] - J[i2][j1] * J[i1][j2];
+            }
+        const double det = J[0][0] * A[0][0] + J[1][0] * A[0][1] + J[2][0] * A[0][2];
+        const double sc = p.mu8 / det;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int a = 2 * h + k;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double r = fma(s.dnr[g][3 * a + 2], A[2][i],
+                                     fma(s.dnr[g][3 * a + 1], A[1][i], s.dnr[g][3 * a] * A[0][i]));
+                s.R[el][g][3 * a + i] = r;
+                s.Rs[el][g][3 * a + i] = r * sc;
+            }
+        }
+        if (h == 0) s.det[el][g] = det;
+    }
+    __syncwarp();
+    // mass by sum factorisation, as k_hex8_element
+    if (lane < 12) {
+        const int cx = lane >> 2, gyz = lane & 3;
+        s.d1[el][lane] = fma(s.det[el][4 + gyz], p.tmx[1][cx], s.det[el][gyz] * p.tmx[0][cx]);
+    }
+    __syncwarp();
+    if (lane < 18) {
+        const int cx = lane / 6, r = lane - 6 * cx, cy = r >> 1, gz = r & 1;
+        s.d2[el][lane] = fma(s.d1[el][cx * 4 + 2 + gz], p.tm[1][cy], s.d1[el][cx * 4 + gz] * p.tm[0][cy]);
+    }
+    __syncwarp();
+    if (lane < 27) {
+        const int cxy = lane / 3, cz = lane - 3 * cxy;
+        s.m[el][lane] = fma(s.d2[el][cxy * 2 + 1], p.tm[1][cz], s.d2[el][cxy * 2] * p.tm[0][cz]);
+    }
+    __syncwarp();
+    double* rec = p.rec + e * kRec;
+    const double lm = p.lm, lm1 = p.lm + 1.0;
+    // diagonal pair (t, t): two Gauss points a quarter
+    {
+        const int a = t;
+        double P[6] = {0, 0, 0, 0, 0, 0};  // 00, 11, 22, 01, 02, 12
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double* r = s.R[el][2 * h + k] + 3 * a;
+            const double* q = s.Rs[el][2 * h + k] + 3 * a;
+            P[0] = fma(q[0], r[0], P[0]);
+            P[1] = fma(q[1], r[1], P[1]);
+            P[2] = fma(q[2], r[2], P[2]);
+            P[3] = fma(q[0], r[1], P[3]);
+            P[4] = fma(q[0], r[2], P[4]);
+            P[5] = fma(q[1], r[2], P[5]);
+        }
+#pragma unroll
+        for (int off = 8; off < 32; off <<= 1)
+#pragma unroll
+            for (int i = 0; i < 6; ++i) P[i] += __shfl_xor_sync(full, P[i], off);
+        const double tr = P[0] + P[1] + P[2];
+        if (valid && h == 0) {
+            double2* o = reinterpret_cast<double2*>(rec + kPairStride * pair_index(a, a) - 2 * a);  // pair_offset(a, a)
+            o[0] = make_double2(fma(lm1, P[0], tr), fma(lm1, P[1], tr));
+            o[1] = make_double2(fma(lm1, P[2], tr), lm1 * P[3]);
+            o[2] = make_double2(lm1 * P[4], lm1 * P[5]);
+            o[3] = make_double2(s.m[el][mass_class(a, a)], 0.0);
+        }
+    }
+    // element load for corner t: two corners b a quarter
+    {
+        double f[3] = {0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int b = 2 * h + k;
+            const double mv = s.m[el][mass_class(t, b)];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) f[i] = fma(mv, s.wx[el][b][i], f[i]);
+        }
+#pragma unroll
+        for (int off = 8; off < 32; off <<= 1)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) f[i] += __shfl_xor_sync(full, f[i], off);
+        if (valid && h < 3) rec[kFOff + 3 * t + h] = h == 0 ? f[0] : h == 1 ? f[1] : f[2];
+    }
+    if (valid && lane < 28) {
+        int a, b;
+        offdiag_pair(lane, a, b);
+        double P[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) P[i] = 0.0;
+#pragma unroll 4
+        for (int g = 0; g < 8; ++g) {
+            const double* q = s.Rs[el][g] + 3 * a;
+            const double* r = s.R[el][g] + 3 * b;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) P[3 * i + j] = fma(q[i], r[j], P[3 * i + j]);
+        }
+        const double tr = P[0] + P[4] + P[8];
+        double2* o = reinterpret_cast<double2*>(rec + kPairStride * pair_index(a, b) - 2 * (a + 1));  // pair_offset
+        o[0] = make_double2(fma(lm1, P[0], tr), fma(lm, P[1], P[3]));
+        o[1] = make_double2(fma(lm, P[2], P[6]), fma(lm, P[3], P[1]));
+        o[2] = make_double2(fma(lm1, P[4], tr), fma(lm, P[5], P[7]));
+        o[3] = make_double2(fma(lm, P[6], P[2]), fma(lm, P[7], P[5]));
+        o[4] = make_double2(fma(lm1, P[8], tr), s.m[el][mass_class(a, b)]);
     }
 }
 
@@ -487,8 +664,9 @@ struct Gather64Params {
     const double* loads;
 };
 
+template <int W>
 struct Gather64Smem {
-    double acc[kG64Warps][kG64Rows][kG64RowStride];
+    double acc[W][kG64Rows][kG64RowStride];
 };
 
 // Lane-per-slot path for one row of any length (K and M; F is summed by the caller).
@@ -539,13 +717,14 @@ __device__ void gather_row_long64(const Gather64Params& p, int64_t row, int lane
     }
 }
 
-__global__ void __launch_bounds__(kG64Warps * 32, 6) k_gather64(const Gather64Params p) {
+template <int W>
+__global__ void __launch_bounds__(W * 32, 24 / W) k_gather64(const Gather64Params p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Gather64Smem& S = *reinterpret_cast<Gather64Smem*>(smem_raw);
+    Gather64Smem<W>& S = *reinterpret_cast<Gather64Smem<W>*>(smem_raw);
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane >> 3, b = lane & 7;
-    const int64_t row0 = p.row_begin + (int64_t(blockIdx.x) * kG64Warps + w) * kG64Rows;
+    const int64_t row0 = p.row_begin + (int64_t(blockIdx.x) * W + w) * kG64Rows;
     if (row0 >= p.row_end) return;  // uniform per warp
     const int64_t row = row0 + r;
     const bool vrow = row < p.row_end;
@@ -612,13 +791,24 @@ __global__ void __launch_bounds__(kG64Warps * 32, 6) k_gather64(const Gather64Pa
         }
     };
     load_chunk(0);
-    // F of this row on lanes b < 3: corner loads in element order, then the nodal loads
+    // F of this row on lanes b < 3: corner loads in element order, then the nodal loads.  Lane (r, j) loads
+    // entry 8c + j's three values, so a chunk's loads are in flight together; the sums walk the lanes.
     if (p.F) {
         double f = 0.0;
-        for (int k = 0; k < maxcnt; ++k) {
-            if (k > 0 && (k & 7) == 0) load_chunk(k >> 3);
-            const int ent = __shfl_sync(full, ent_reg, src | (k & 7));
-            if (b < 3 && k < cnt) f += __ldg(p.rec + int64_t(ent >> 3) * kRec + kFOff + 3 * (ent & 7) + b);
+        for (int c = 0; 8 * c < maxcnt; ++c) {
+            if (c) load_chunk(c);
+            double w[3] = {0.0, 0.0, 0.0};
+            if (8 * c + b < cnt) {
+                const double* q = p.rec + int64_t(ent_reg >> 3) * kRec + kFOff + 3 * (ent_reg & 7);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) w[i] = __ldg(q + i);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double w0 = __shfl_sync(full, w[0], src | j), w1 = __shfl_sync(full, w[1], src | j);
+                const double w2 = __shfl_sync(full, w[2], src | j);
+                if (8 * c + j < cnt) f += b == 0 ? w0 : b == 1 ? w1 : w2;
+            }
         }
         if (maxcnt > 8) load_chunk(0);
         if (b < 3 && vrow) {
@@ -807,6 +997,7 @@ int check_assembly_inputs(const fem_mesh* mesh, const fem_material* mat, void* w
 }  // namespace
 
 namespace fem {
+int sm_count();
 int launch_hex8_element_dd(const fem_mesh* mesh, const fem_material* mat, void* workspace, cudaStream_t st,
                            int64_t e_begin, int64_t e_end);
 int launch_gather_dd(const fem_mesh* mesh, const fem_assembly_out* out, const void* workspace, cudaStream_t st,
@@ -847,6 +1038,15 @@ int launch_hex8_element(const fem_mesh* mesh, const fem_material* mat, void* wor
                 ep.tm[sd][c] = tm[sd][c];
                 ep.tmx[sd][c] = mat->DE / 512 * tm[sd][c];
             }
+    }
+    // A warp per element up to 16 elements an SM (152 SMs): 12.3 against 26.7 us at 256 elements, 24.6
+    // against 26.7 at 1,536, 39.5 against 41.1 at 2,560, 55.1 against 42.4 at 4,000.  By the whole mesh,
+    // not the part: every split of an assembly gives the same bits.
+    if (mesh->n_elem <= int64_t(kWidePerSm) * sm_count()) {
+        const int64_t blocks = (e_end - e_begin + kWideEpc - 1) / kWideEpc;
+        k_hex8_element_wide<<<unsigned(blocks), kWideEpc * 32, 0, st>>>(ep);
+        FEM_LAUNCH_CHECK("k_hex8_element_wide");
+        return FEM_OK;
     }
     const size_t smem = sizeof(ElemSmem);
     FEM_CUDA(cudaFuncSetAttribute(k_hex8_element, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -901,11 +1101,12 @@ int launch_gather64(const fem_mesh* mesh, const fem_assembly_out* out, const voi
     gp.F = out->F;
     gp.fixed = out->fixed;
     gp.loads = out->loads;
-    const size_t smem = sizeof(Gather64Smem);
-    FEM_CUDA(cudaFuncSetAttribute(k_gather64, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int64_t rows_per_cta = int64_t(kG64Warps) * kG64Rows;
+    constexpr int W = kG64Warps;
+    const size_t smem = sizeof(Gather64Smem<W>);
+    FEM_CUDA(cudaFuncSetAttribute(k_gather64<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    const int64_t rows_per_cta = int64_t(W) * kG64Rows;
     const int64_t blocks = (row_end - row_begin + rows_per_cta - 1) / rows_per_cta;
-    k_gather64<<<unsigned(blocks), kG64Warps * 32, smem, st>>>(gp);
+    k_gather64<W><<<unsigned(blocks), W * 32, smem, st>>>(gp);
     FEM_LAUNCH_CHECK("k_gather64");
     return FEM_OK;
 }

@@ -1,5 +1,5 @@
-"""FP64 element kernel at the edges of its tiles (16 elements a block, 4 a warp): element counts off
-every multiple, the parts of a split assembly, far from the origin, an inverted element; K, M and F
+"""FP64 element kernels at the edges of their tiles (a warp per element up to 16 elements an SM, 16
+elements a block beyond) and where one takes over from the other: element counts off every multiple, the parts of a split assembly, far from the origin, an inverted element; K, M and F
 against the oracle with the suite's tolerances (1e-12 of the row's / vector's largest entry)."""
 import numpy as np
 import pytest
@@ -26,9 +26,18 @@ def test_element_counts_off_the_tile(shape):
     _check(F.hex_block(*shape, jitter=0.1, seed=4, twist_deg=30, fix="xmin"))
 
 
+@pytest.mark.parametrize("extra", [-1, 0, 1, 17])
+def test_where_the_kernels_meet(extra):
+    """16 x (SMs) elements and a few more or fewer, as a chain of bars of one element's section."""
+    import torch
+    n = 16 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    _check(F.hex_block(n, 1, 1, size=(float(n), 1.0, 1.0), jitter=0.0, seed=4, twist_deg=90, fix="xmin"))
+
+
+@pytest.mark.parametrize("shape", [(9, 7, 5), (31, 13, 7)])
 @pytest.mark.parametrize("parts", [1, 3, 50])
-def test_parts_off_the_tile(parts):
-    P = F.hex_block(9, 7, 5, jitter=0.1, seed=4, origin=(500.0, -200.0, 0.0), fix="zmin")
+def test_parts_off_the_tile(shape, parts):
+    P = F.hex_block(*shape, jitter=0.1, seed=4, origin=(500.0, -200.0, 0.0), fix="zmin")
     M = _check(P)
     K, Mm, Fv = M.assemble_host(n_parts=parts)
     K1, M1, F1 = M.assemble(k_layout="csr", m_layout="csr")
