@@ -130,6 +130,7 @@ struct MlpParams {
     float* out;         // [n][16]
     float* z1;          // [n][64] pre-activations (optional)
     float* z2;          // [n][64] (optional)
+    int wide;           // z1 and z2 on 16-byte boundaries
     int* err;           // device flag, set on a bounded-wait timeout
 };
 
@@ -142,9 +143,37 @@ struct MlpSmem {
     alignas(1024) unsigned char H1s[kTile * kHid * 2];   // 16 KB  A operand, layer 2
     alignas(1024) unsigned char H2s[kTile * kHid * 2];   // 16 KB  A operand, layer 3
     float b1[kHid], b2[kHid], b3[kOut];
+    alignas(16) float zs[kTile / 32][32][20];            // 10 KB  pre-activations on their way out
     alignas(8) uint64_t mbar;
     uint32_t tmem_base;
 };
+
+// Pre-activations z[16] = columns c0.. of this thread's node (row base + lane of a warp's 32) to dst
+// [n][64].  Through shared memory (rows of 20 floats: conflict-free 16-byte accesses), so that a
+// store instruction writes 64 contiguous bytes of 8 nodes; one 4-byte store per column wrote 32 sectors an
+// instruction and set the forward's pace (214,221 nodes with both pre-activations kept: 189 us,
+// 76 us here).
+__device__ __forceinline__ void store_preactivations(float* dst, int64_t base, int64_t n, int c0, const float (&z)[16],
+                                                     float (*stage)[20], int lane, int wide) {
+    if (!dst) return;
+    if (!wide) {
+        if (base + lane < n)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[(base + lane) * kHid + c0 + j] = z[j];
+        return;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4*>(&stage[lane][4 * q]) = make_float4(z[4 * q], z[4 * q + 1], z[4 * q + 2], z[4 * q + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), q = lane & 3;
+        if (base + r < n)
+            *reinterpret_cast<float4*>(dst + (base + r) * kHid + c0 + 4 * q) = *reinterpret_cast<const float4*>(&stage[r][4 * q]);
+    }
+}
 
 __device__ __forceinline__ void store_row_bf16(unsigned char* tile, int row, int k0, int K, const float (&v)[16]) {
     // 16 consecutive k values = two 16-byte core rows
@@ -225,11 +254,10 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_fwd(const MlpParams p) {
             float v[16];
             tmem_ld16(tmem + lane_base + uint32_t(c0), v);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float z = v[j] + s.b1[c0 + j];
-                if (p.z1 && valid) p.z1[node * kHid + c0 + j] = z;
-                v[j] = silu(z);
-            }
+            for (int j = 0; j < 16; ++j) v[j] += s.b1[c0 + j];
+            store_preactivations(p.z1, tile * kTile + 32 * warp, p.n, c0, v, s.zs[warp], tid & 31, p.wide);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = silu(v[j]);
             store_row_bf16(s.H1s, tid, c0, kHid, v);
         }
         fence_before();
@@ -253,11 +281,10 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_fwd(const MlpParams p) {
             float v[16];
             tmem_ld16(tmem + lane_base + uint32_t(64 + c0), v);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float z = v[j] + s.b2[c0 + j];
-                if (p.z2 && valid) p.z2[node * kHid + c0 + j] = z;
-                v[j] = silu(z);
-            }
+            for (int j = 0; j < 16; ++j) v[j] += s.b2[c0 + j];
+            store_preactivations(p.z2, tile * kTile + 32 * warp, p.n, c0, v, s.zs[warp], tid & 31, p.wide);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = silu(v[j]);
             store_row_bf16(s.H2s, tid, c0, kHid, v);
         }
         fence_before();
@@ -651,7 +678,11 @@ __global__ void __launch_bounds__(256) k_mlp_bwd(const BwdParams p) {
 
 // ---- backward on the tensor cores -------------------------------------------------------------
 //
-// k_mlp_bwd_tc: one persistent CTA of 128 threads per SM, 128 nodes per tile (thread = node).
+// k_mlp_bwd_tc: one persistent CTA of 512 threads per SM, 128 nodes per tile, four threads per node
+// (thread = node and 16 of its 64 columns; warp w holds nodes 32 (w mod 4).., the TMEM lanes it may read,
+// and columns 16 (w / 4)..).  The tile is a chain of loads, element-wise work, two products and their
+// waits, so its time is latency: with one thread per node, 4 warps an SM, 214,221 nodes took 343 us,
+// 161 us here.
 //  1. CUDA cores: h1 = bf16(silu(z1)), h2 = bf16(silu(z2)), s' = silu'(z), dz3 = dout[:6],
 //     dz2 = (dz3 W3[:6]) * s2' (K = 6 is too short for an MMA).
 //  2. tcgen05 (M = 128 nodes, N = 64, K = 64): D1 = bf16(dz2) W2 in TMEM columns [0, 64);
@@ -670,6 +701,7 @@ __global__ void __launch_bounds__(256) k_mlp_bwd(const BwdParams p) {
 // mlp_oracle.backward_bf16 states them).  Every mbarrier wait is bounded and TMEM is freed on
 // every exit.
 constexpr int kBwdCols = 256;  // TMEM columns allocated (176 used)
+constexpr int kBwdThreads = 4 * kTile;
 
 struct BwdTcParams {
     const float* W;      // FP32 master parameters (flat)
@@ -698,21 +730,21 @@ __device__ __forceinline__ void put_bf16(unsigned char* tile, int row, int k, in
     *reinterpret_cast<__nv_bfloat16*>(tile + core_off(row, k, K)) = __float2bfloat16_rn(v);
 }
 
-__global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
+__global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_bwd_tc(const BwdTcParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     BwdTcSmem& s = *reinterpret_cast<BwdTcSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid >> 5;
 
     // W2^T in the core-matrix layout: element (row k, col o) = W2[o][k], BF16 as the forward used it
-    for (int i = tid; i < kHid * kHid; i += kTile) {
+    for (int i = tid; i < kHid * kHid; i += kBwdThreads) {
         const int o = i / kHid, k = i % kHid;
         put_bf16(s.W2T, k, o, kHid, p.W[oW2 + i]);
     }
-    for (int i = tid; i < kOutUsed * kHid; i += kTile) s.W3[i / kHid][i % kHid] = bf16r(p.W[oW3 + i]);
+    for (int i = tid; i < kOutUsed * kHid; i += kBwdThreads) s.W3[i / kHid][i % kHid] = bf16r(p.W[oW3 + i]);
     // constant zero rows of the operands (rows 81-95 of Bg, 65-127 of A3, 6-15 of B3)
-    for (int i = tid; i < 15 * kTile; i += kTile) put_bf16(s.Bg, 81 + i / kTile, i % kTile, kTile, 0.f);
-    for (int i = tid; i < 63 * kTile; i += kTile) put_bf16(s.A3, 65 + i / kTile, i % kTile, kTile, 0.f);
-    for (int i = tid; i < 10 * kTile; i += kTile) put_bf16(s.B3, 6 + i / kTile, i % kTile, kTile, 0.f);
+    for (int i = tid; i < 15 * kTile; i += kBwdThreads) put_bf16(s.Bg, 81 + i / kTile, i % kTile, kTile, 0.f);
+    for (int i = tid; i < 63 * kTile; i += kBwdThreads) put_bf16(s.A3, 65 + i / kTile, i % kTile, kTile, 0.f);
+    for (int i = tid; i < 10 * kTile; i += kBwdThreads) put_bf16(s.B3, 6 + i / kTile, i % kTile, kTile, 0.f);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)),
                      "r"(uint32_t(kBwdCols)));
@@ -727,7 +759,9 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
     __syncthreads();
     fence_after();
     const uint32_t tmem = s.tmem_base;
-    const uint32_t lane_base = uint32_t(32 * warp) << 16;
+    const uint32_t lane_base = uint32_t(32 * (warp & 3)) << 16;
+    const int t = 32 * (warp & 3) + (tid & 31);  // this thread's node in the tile, its column (K index) in the transposed operands
+    const int cg = warp >> 2, c0 = 16 * cg;      // its columns
     const uint32_t id_d1 = idesc_bf16(kTile, kHid), id_g = idesc_bf16(kTile, 96), id_3 = idesc_bf16(kTile, 16);
     const uint32_t aDz2 = smem_u32(s.Dz2), aW2T = smem_u32(s.W2T);
     const uint32_t aAg = smem_u32(s.Ag), aBg = smem_u32(s.Bg), aA3 = smem_u32(s.A3), aB3 = smem_u32(s.B3);
@@ -736,19 +770,19 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
     bool first = true;
 
     for (int64_t tile = blockIdx.x; tile * kTile < p.n && ok; tile += gridDim.x) {
-        const int64_t node = tile * kTile + tid;
+        const int64_t node = tile * kTile + t;
         const bool valid = node < p.n;
-        const int t = tid;  // column (K index) of this node in the transposed operands
-        float s1g[kHid];
+        float s1g[16];
         {
             // dz3 and dz2 = (dz3 W3) s2'; h2^T, X^T, valid; dz3^T
             float d3[kOutUsed];
 #pragma unroll
             for (int o = 0; o < kOutUsed; ++o) d3[o] = valid ? p.dout[node * kOut + o] : 0.f;
+            if (cg == 0) {
 #pragma unroll
-            for (int o = 0; o < kOutUsed; ++o) put_bf16(s.B3, o, t, kTile, d3[o]);
-#pragma unroll
-            for (int c0 = 0; c0 < kHid; c0 += 16) {
+                for (int o = 0; o < kOutUsed; ++o) put_bf16(s.B3, o, t, kTile, d3[o]);
+            }
+            {
                 float a1v[16], a2v[16], v[16];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -771,25 +805,20 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
                     put_bf16(s.Ag, c, t, kTile, d);                            // dz2^T (rows 0-63)
                     put_bf16(s.A3, c, t, kTile, valid ? silu(a2v[j]) : 0.f);  // h2^T
                     put_bf16(s.Bg, c, t, kTile, valid ? silu(a1v[j]) : 0.f);  // h1^T
-                    s1g[c] = valid ? silu_grad(a1v[j]) : 0.f;
+                    s1g[j] = valid ? silu_grad(a1v[j]) : 0.f;
                 }
-                store_row_bf16(s.Dz2, tid, c0, kHid, v);                       // dz2, node-major
+                store_row_bf16(s.Dz2, t, c0, kHid, v);                       // dz2, node-major
             }
-            uint4 xa = make_uint4(0, 0, 0, 0), xb = make_uint4(0, 0, 0, 0);
-            if (valid) {
-                const uint4* src = reinterpret_cast<const uint4*>(p.X + node * kIn);
-                xa = src[0];
-                xb = src[1];
-            }
-            const uint16_t* xs = reinterpret_cast<const uint16_t*>(&xa);
-            const uint16_t* xt = reinterpret_cast<const uint16_t*>(&xb);
+            if (cg < 2) {  // X^T, 8 inputs each by two of the node's threads
+                uint4 xa = make_uint4(0, 0, 0, 0);
+                if (valid) xa = reinterpret_cast<const uint4*>(p.X + node * kIn)[cg];
+                const uint16_t* xs = reinterpret_cast<const uint16_t*>(&xa);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                *reinterpret_cast<uint16_t*>(s.Bg + core_off(64 + k, t, kTile)) = xs[k];
-                *reinterpret_cast<uint16_t*>(s.Bg + core_off(72 + k, t, kTile)) = xt[k];
+                for (int k = 0; k < 8; ++k) *reinterpret_cast<uint16_t*>(s.Bg + core_off(64 + 8 * cg + k, t, kTile)) = xs[k];
+            } else if (cg == 2) {
+                put_bf16(s.Bg, 80, t, kTile, valid ? 1.f : 0.f);
+                put_bf16(s.A3, 64, t, kTile, valid ? 1.f : 0.f);
             }
-            put_bf16(s.Bg, 80, t, kTile, valid ? 1.f : 0.f);
-            put_bf16(s.A3, 64, t, kTile, valid ? 1.f : 0.f);
         }
         fence_proxy_async();
         __syncthreads();
@@ -807,12 +836,11 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
         if (!ok) break;
         fence_after();
         // dz1 = D1 s1'  -> rows 64-127 of Ag (transposed)
-#pragma unroll
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
+        {
             float v[16];
             tmem_ld16(tmem + lane_base + uint32_t(c0), v);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) put_bf16(s.Ag, 64 + c0 + j, t, kTile, v[j] * s1g[c0 + j]);
+            for (int j = 0; j < 16; ++j) put_bf16(s.Ag, 64 + c0 + j, t, kTile, v[j] * s1g[j]);
         }
         fence_before();
         fence_proxy_async();
@@ -838,18 +866,17 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
     // ---- this CTA's partial gradient --------------------------------------------------------------
     float* out = p.part + int64_t(blockIdx.x) * kNParams;
     if (ok) {
-        const int r = tid;  // TMEM lane = row of the accumulators
+        const int r = t;  // TMEM lane = row of the accumulators
         if (first) {
             // no tile: zero partial
-            for (int i = tid; i < kNParams; i += kTile) out[i] = 0.f;
+            for (int i = tid; i < kNParams; i += kBwdThreads) out[i] = 0.f;
         } else {
-#pragma unroll
-            for (int c0 = 0; c0 < 96; c0 += 16) {
+            for (int k0 = c0; k0 < 96; k0 += kHid) {
                 float v[16];
-                tmem_ld16(tmem + lane_base + uint32_t(64 + c0), v);
+                tmem_ld16(tmem + lane_base + uint32_t(64 + k0), v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int c = c0 + j;
+                    const int c = k0 + j;
                     if (r < 64) {
                         if (c < 64) out[oW2 + r * kHid + c] = v[j];
                         else if (c == 80) out[ob2 + r] = v[j];
@@ -859,7 +886,7 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
                     }
                 }
             }
-            {
+            if (cg == 3) {
                 float v[16];
                 tmem_ld16(tmem + lane_base + 160u, v);
                 if (r < 64) {
@@ -870,7 +897,7 @@ __global__ void __launch_bounds__(kTile, 1) k_mlp_bwd_tc(const BwdTcParams p) {
                     for (int o = 0; o < kOutUsed; ++o) out[ob3 + o] = v[o];
                 }
             }
-            for (int i = kOutUsed * kHid + tid; i < kOut * kHid; i += kTile) out[oW3 + i] = 0.f;
+            for (int i = kOutUsed * kHid + tid; i < kOut * kHid; i += kBwdThreads) out[oW3 + i] = 0.f;
             if (tid < kOut - kOutUsed) out[ob3 + kOutUsed + tid] = 0.f;
         }
     } else if (tid == 0) {
@@ -1004,7 +1031,8 @@ extern "C" int fem_mlp_forward(const fem_mlp* net, const uint16_t* X, int64_t n,
     FEM_REQUIRE(n >= 0 && err && (n == 0 || (X && out)), "bad arguments");
     FEM_REQUIRE(n == 0 || aligned16(X), "X must be 16-byte aligned");
     if (n == 0) return FEM_OK;
-    MlpParams p{net->W1, net->b1, net->W2, net->b2, net->W3, net->b3, X, n, out, z1, z2, err};
+    MlpParams p{net->W1, net->b1, net->W2, net->b2, net->W3, net->b3, X, n, out, z1, z2,
+                aligned16(z1) && aligned16(z2), err};
     const size_t smem = sizeof(MlpSmem) + 1024;
     FEM_CUDA(cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const int64_t tiles = (n + kTile - 1) / kTile;
@@ -1078,7 +1106,7 @@ extern "C" int fem_mlp_backward_tc(const float* params, const uint16_t* X, const
     BwdTcParams p{params, X, z1, z2, dout, n, static_cast<float*>(workspace), err};
     const size_t smem = sizeof(BwdTcSmem) + 1024;
     FEM_CUDA(cudaFuncSetAttribute(k_mlp_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    k_mlp_bwd_tc<<<g, kTile, smem, st>>>(p);
+    k_mlp_bwd_tc<<<g, kBwdThreads, smem, st>>>(p);
     FEM_LAUNCH_CHECK("k_mlp_bwd_tc");
     k_sum_partials<<<(kNParams + 255) / 256, 256, 0, st>>>(static_cast<const float*>(workspace), g, kNParams, grad);
     FEM_LAUNCH_CHECK("k_sum_partials");
