@@ -141,28 +141,242 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
     }
 }
 
-// The same for one FP32 right-hand side with p of 4 floats a node.
-__global__ void __launch_bounds__(kThreads) k_xp_update_pad(int64_t n, const float* __restrict__ M,
-                                                             const float* __restrict__ r, float* x, float4* p,
-                                                             const PcgState* __restrict__ st) {
-    if (st->done) return;
-    const bool first = st->it == 0;
-    const float a = float(st->alpha[0]), b = float(st->beta[0]);
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        float z0, z1, z2;
-        apply_block(M + 9 * i, r[3 * i], r[3 * i + 1], r[3 * i + 2], z0, z1, z2);
-        if (!first) {
-            const float4 o = p[i];
-            x[3 * i] += a * o.x;
-            x[3 * i + 1] += a * o.y;
-            x[3 * i + 2] += a * o.z;
-            z0 += b * o.x;
-            z1 += b * o.y;
-            z2 += b * o.z;
-        }
-        p[i] = make_float4(z0, z1, z2, 0.f);
+// ---- one FP32 right-hand side, p of 4 floats a node --------------------------------------------
+// The iteration's sums without a last CTA: a kernel leaves one partial sum per CTA, and every CTA of the
+// kernel that needs the total adds them up itself, in the same order, while its first nodes load.  What
+// the last CTA did before (a fence, a ticket, the partial sums, a tree and alpha or beta, each waiting for
+// the one before) was 11 of the 17 us of the residual update and 4 of the product's 47 at 214,221 nodes: an
+// iteration took 68 us, 58 us here.  One CTA of 1,024 threads per SM keeps the partial sums few.
+// With more right-hand sides the sums would cost every CTA R times as much, and the vectors hide the rest.
+constexpr int kStepThreads = 1024;
+constexpr int kStepNodes = 2;    // nodes of a thread in flight
+constexpr int kPq = 0, kRz = 1;  // slots of kMaxCtas partial sums: p.q; r.z and r.r
+
+// The sums of v over this CTA's W warps to its entries of the slots slot0..
+template <int NS, int W>
+__device__ __forceinline__ void step_partials(const Dot<float> (&v)[NS], double* part, int slot0) {
+    __shared__ double sm[NS][W];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const double w = rhs_sum<1>(v[s]);
+        if (lane == 0) sm[s][warp] = w;
+    }
+    __syncthreads();
+    if (warp < NS) {
+        double a = lane < W ? sm[warp][lane] : 0.0;
+#pragma unroll
+        for (int off = W / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        if (lane == 0) part[(slot0 + warp) * kMaxCtas + blockIdx.x] = a;
     }
 }
+
+// Totals of NS slots with nb partial sums each: slot s's four parts in sm[4 s..], by warps 4 s.. (a
+// warp each on the four FP64 pipes of an SM); every thread of the CTA calls it.
+template <int NS>
+__device__ __forceinline__ void step_totals(const double* part, int slot0, int nb, double (&sm)[4 * NS]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 4 * NS) {
+        const double* src = part + (slot0 + warp / 4) * kMaxCtas;
+        double acc = 0.0;
+        for (int b0 = 32 * (warp % 4); b0 < nb; b0 += 1024) {
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = b0 + 128 * k + lane < nb ? __ldcg(src + b0 + 128 * k + lane) : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (b0 + 128 * k < nb) acc += v[k];
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if (lane == 0) sm[warp] = acc;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ double step_sum(const double* sm) { return (sm[0] + sm[1]) + (sm[2] + sm[3]); }
+
+// What the residual update's r.r says (one thread): whether the solve goes on; with `write`, the state.
+__device__ __forceinline__ bool step_goes_on(double rr, PcgState* st, bool write) {
+    const bool finite = isfinite(rr);
+    const bool active = rr > st->tol2[0] && finite;
+    const bool capped = active && st->it >= st->maxit;
+    if (write) {
+        st->iters[0] += 1;
+        st->rr[0] = rr;
+        st->active[0] = active;
+        if (!finite) st->status = FEM_ERR_BREAKDOWN;
+        if (capped && !st->status) st->status = FEM_ERR_MAXITER;
+        if (!active || capped) st->done = 1;
+    }
+    return active && !capped;
+}
+
+// Nodes of this thread: warps take 32 nodes at a time, in turn over the CTAs
+__device__ __forceinline__ int64_t step_node(int64_t& stride) {
+    stride = int64_t(gridDim.x) * kStepThreads;
+    return (int64_t(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+}
+
+// x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration).  CTA 0
+// records the iteration's outcome; the others form it for themselves and never read what it writes
+// (a CTA that sees `done` already set would have found the same).
+__global__ void __launch_bounds__(kStepThreads) k_step_p(int64_t n, const float* __restrict__ M,
+                                                          const float* __restrict__ r, float* x, float4* p,
+                                                          const double* part, int nb, PcgState* st) {
+    if (st->done) return;
+    const bool first = st->it == 0;
+    __shared__ double sm[8];
+    __shared__ float sa, sb;
+    __shared__ bool go;
+    float rv[kStepNodes][3], xv[kStepNodes][3], m[kStepNodes][9];
+    float4 pv[kStepNodes];
+    int64_t stride, i = step_node(stride);
+    auto load = [&]() {
+#pragma unroll
+        for (int h = 0; h < kStepNodes; ++h) {
+            const int64_t node = i + h * stride;
+            if (node >= n) continue;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) rv[h][j] = r[3 * node + j];
+#pragma unroll
+            for (int j = 0; j < 9; ++j) m[h][j] = __ldg(M + 9 * node + j);
+            if (first) continue;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) xv[h][j] = x[3 * node + j];
+            pv[h] = p[node];
+        }
+    };
+    load();
+    if (!first) {
+        step_totals<2>(part, kRz, nb, sm);
+        if (threadIdx.x == 0) {
+            const double rz = step_sum(sm), beta = rz / st->rz_old;
+            sb = float(beta);
+            if (blockIdx.x == 0) {
+                st->rz[0] = rz;
+                st->beta[0] = beta;
+            }
+        } else if (threadIdx.x == 32) {
+            go = step_goes_on(step_sum(sm + 4), st, blockIdx.x == 0);
+        } else if (threadIdx.x == 64) {
+            sa = float(st->alpha[0]);
+        }
+        __syncthreads();
+        if (!go) return;
+    }
+    const float a = first ? 0.f : sa, b = first ? 0.f : sb;
+    for (;;) {
+#pragma unroll
+        for (int h = 0; h < kStepNodes; ++h) {
+            const int64_t node = i + h * stride;
+            if (node >= n) continue;
+            float z0, z1, z2;
+            apply_block(m[h], rv[h][0], rv[h][1], rv[h][2], z0, z1, z2);
+            if (!first) {
+                x[3 * node] = xv[h][0] + a * pv[h].x;
+                x[3 * node + 1] = xv[h][1] + a * pv[h].y;
+                x[3 * node + 2] = xv[h][2] + a * pv[h].z;
+                z0 += b * pv[h].x;
+                z1 += b * pv[h].y;
+                z2 += b * pv[h].z;
+            }
+            p[node] = make_float4(z0, z1, z2, 0.f);
+        }
+        i += kStepNodes * stride;
+        if (i >= n) break;
+        load();
+    }
+}
+
+// alpha = r.z / p.q; r -= alpha q; partial sums of r.M r and r.r.  nb: CTAs of the product.
+__global__ void __launch_bounds__(kStepThreads) k_step_r(int64_t n, const float* __restrict__ M,
+                                                          const float* __restrict__ q, float* r, double* part, int nb,
+                                                          PcgState* st) {
+    if (st->done) return;
+    __shared__ double sm[4];
+    __shared__ float sa;
+    __shared__ bool go;
+    float rv[kStepNodes][3], qv[kStepNodes][3], m[kStepNodes][9];
+    int64_t stride, i = step_node(stride);
+    auto load = [&]() {
+#pragma unroll
+        for (int h = 0; h < kStepNodes; ++h) {
+            const int64_t node = i + h * stride;
+            if (node >= n) continue;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                rv[h][j] = r[3 * node + j];
+                qv[h][j] = q[3 * node + j];
+            }
+#pragma unroll
+            for (int j = 0; j < 9; ++j) m[h][j] = __ldg(M + 9 * node + j);
+        }
+    };
+    load();
+    step_totals<1>(part, kPq, nb, sm);
+    if (threadIdx.x == 0) {
+        const double pq = step_sum(sm), rz = st->rz[0];
+        const bool ok = pq > 0.0 && isfinite(pq);
+        const double alpha = ok ? rz / pq : 0.0;
+        sa = float(alpha);
+        go = ok;
+        if (blockIdx.x == 0) {
+            st->pq[0] = pq;
+            st->alpha[0] = alpha;
+            st->rz_old = rz;
+            st->it += 1;
+            if (!ok) {
+                st->active[0] = 0;
+                st->status = isfinite(pq) ? FEM_ERR_NOT_SPD : FEM_ERR_BREAKDOWN;
+                st->done = 1;
+            }
+        }
+    }
+    __syncthreads();
+    if (!go) return;
+    const float a = sa;
+    Dot<float> v[2];
+    for (;;) {
+#pragma unroll
+        for (int h = 0; h < kStepNodes; ++h) {
+            const int64_t node = i + h * stride;
+            if (node >= n) continue;
+            float z[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                rv[h][j] -= a * qv[h][j];
+                r[3 * node + j] = rv[h][j];
+            }
+            apply_block(m[h], rv[h][0], rv[h][1], rv[h][2], z[0], z[1], z[2]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                v[0].add(rv[h][j], z[j]);
+                v[1].add(rv[h][j], rv[h][j]);
+            }
+        }
+        i += kStepNodes * stride;
+        if (i >= n) break;
+        load();
+    }
+    step_partials<2, kStepThreads / 32>(v, part, kRz);
+}
+
+// The outcome of the last of the iterations launched together, for the host: what k_step_p would record
+// (which then finds the same, and records it, if the solve goes on).
+__global__ void __launch_bounds__(kThreads) k_step_check(const double* part, int nb, PcgState* st) {
+    if (st->done) return;
+    __shared__ double sm[8];
+    step_totals<2>(part, kRz, nb, sm);
+    if (threadIdx.x == 0) {
+        const double rr = step_sum(sm + 4);
+        st->rr[0] = rr;
+        if (!step_goes_on(rr, st, false)) {
+            st->rz[0] = step_sum(sm);
+            step_goes_on(rr, st, true);
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) k_x_finish_pad(int64_t n, const float4* __restrict__ p, float* x,
                                                             const PcgState* __restrict__ st) {
     if (st->it == 0) return;
@@ -199,7 +413,7 @@ __global__ void __launch_bounds__(kThreads) k_p_update(int64_t nv, const T* __re
 // q = A p and p.q -> alpha = rz / pq on the device.  (Folding p = z + beta p into this
 // kernel as q = A z + beta q was measured slower: the row epilogue's extra loads sit on the
 // product's critical path, and the recurrence drifts from A p in FP32.)
-// kPad (FP32, one right-hand side, padded row-SoA matrix): p holds 4 floats a node.
+// kPad (FP32, one right-hand side, padded row-SoA matrix): p holds 4 floats a node, and k_step_r forms alpha.
 template <typename T, int R, int LPR, bool kPad>
 __global__ void __launch_bounds__(kThreads, spmm_ctas<T, R>())
     k_spmv_pq(const BsrView<T> A, const T* __restrict__ p, T* __restrict__ q, double* part, PcgState* st) {
@@ -211,6 +425,10 @@ __global__ void __launch_bounds__(kThreads, spmm_ctas<T, R>())
         v[0] = spmv1_rows<T, LPR>(A, p, q, true);
     else
         v[0] = spmm_rows<T, R>(A, p, q, true);
+    if constexpr (kPad) {
+        step_partials<1, kThreads / 32>(v, part, kPq);
+        return;
+    }
     __shared__ double tot[1][kMaxR];
     if (block_partials<R, 1>(v, part, &st->ticket)) {
         last_block_totals<R, 1>(part, gridDim.x, tot);
@@ -597,9 +815,10 @@ unsigned vec_grid(Kernel kernel, int64_t work) {
 // (the size of the partial-sum buffer).  The grid fixes each row's CTA, hence the order of the
 // dot-product partial sums.
 template <typename T, int R, bool kPad = false>
-void launch_spmv_pq(const BsrView<T>& A, const T* p, T* q, double* part, PcgState* st, int variant, cudaStream_t s) {
+unsigned launch_spmv_pq(const BsrView<T>& A, const T* p, T* q, double* part, PcgState* st, int variant, cudaStream_t s) {
+    unsigned g = 0;
     auto run = [&](auto kernel, int64_t rows_per_cta, int64_t cap) {
-        const unsigned g = resident_grid(reinterpret_cast<const void*>(kernel), kThreads,
+        g = resident_grid(reinterpret_cast<const void*>(kernel), kThreads,
                                          (A.n + rows_per_cta - 1) / rows_per_cta, std::min<int64_t>(cap, kMaxCtas));
         kernel<<<g, kThreads, 0, s>>>(A, p, q, part, st);
     };
@@ -617,6 +836,12 @@ void launch_spmv_pq(const BsrView<T>& A, const T* p, T* q, double* part, PcgStat
             default: run(k_spmv_pq<T, 1, 2, kPad>, rows_per_cta, cap); break;
         }
     }
+    return g;
+}
+
+// Grid of the k_step kernels: a CTA per SM, fewer where the nodes would not give each one 8 warps
+inline unsigned step_grid(int64_t n) {
+    return unsigned(std::max<int64_t>(1, std::min<int64_t>(sm_count(), (n + 255) / 256)));
 }
 
 // One FP32 right-hand side on the padded row-SoA copy: the search direction has 4 floats a node.
@@ -628,16 +853,20 @@ int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* p, T* q, d
     // 16-byte packs of right-hand sides where the rows of r, p and x (the caller's U in the FP64 solve)
     // start on 16-byte boundaries
     constexpr int V = R % (16 / int(sizeof(T))) == 0 ? 16 / int(sizeof(T)) : 1;
-    for (int i = 0; i < count; ++i) {
-        if constexpr (sizeof(T) == 4 && R == 1) {
-            if (pad_direction(A)) {
-                k_xp_update_pad<<<vec_grid(k_xp_update_pad, A.n), kThreads, 0, s>>>(A.n, M, r, x,
-                                                                                      reinterpret_cast<float4*>(p), st);
-                launch_spmv_pq<T, R, true>(A, p, q, part, st, variant, s);
-                k_r_update<T, R><<<vec_grid(k_r_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, q, r, part, st);
-                continue;
+    if constexpr (sizeof(T) == 4 && R == 1) {
+        if (pad_direction(A)) {
+            const unsigned g = step_grid(A.n);
+            for (int i = 0; i < count; ++i) {
+                k_step_p<<<g, kStepThreads, 0, s>>>(A.n, M, r, x, reinterpret_cast<float4*>(p), part, int(g), st);
+                const unsigned gq = launch_spmv_pq<T, R, true>(A, p, q, part, st, variant, s);
+                k_step_r<<<g, kStepThreads, 0, s>>>(A.n, M, q, r, part, int(gq), st);
             }
+            k_step_check<<<1, kThreads, 0, s>>>(part, int(g), st);
+            FEM_LAUNCH_CHECK("pcg iteration");
+            return FEM_OK;
         }
+    }
+    for (int i = 0; i < count; ++i) {
         if (aligned16(x))
             k_xp_update<T, R, V><<<vec_grid(k_xp_update<T, R, V>, A.n * (R / V)), kThreads, 0, s>>>(A.n, M, r, x, p, st);
         else

@@ -15,6 +15,7 @@ constexpr int kSlots = 3;
 struct PcgState {
     double rz[kMaxR], pq[kMaxR], alpha[kMaxR], beta[kMaxR], bb[kMaxR], rr[kMaxR], tol2[kMaxR];
     double norm2[kMaxR];
+    double rz_old;         // r.z that the last step's alpha was formed with (k_step_r)
     double anorm2[kMaxR];  // || |F| + |A||u| ||^2 of the last true residual (its rounding scale)
     int active[kMaxR];
     int iters[kMaxR];
