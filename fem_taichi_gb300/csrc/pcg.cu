@@ -3,7 +3,8 @@
 //
 // One PCG iteration is three kernels (x += alpha p, p = M r + beta p;  q = A p with p.q;
 // r -= alpha q with r.M r and r.r).  z = M r is formed where it is used (nine values of M per node
-// against three of z per node and right-hand side) and x waits for the kernel that reads p anyway,
+// against three of z per node and right-hand side; the FP64 iteration, where forming it twice costs more
+// than the extra vector, keeps it) and x waits for the kernel that reads p anyway,
 // so an iteration streams 8 vectors beside the product instead of 10; one more kernel after the last
 // iteration adds the pending alpha p.  All scalars live in a device state block:
 // every reduction writes per-CTA partials and the last CTA to finish (atomic ticket) sums
@@ -35,7 +36,7 @@ using namespace pcgd;
 // x = 0, r = b; rz = r.M r, rr -> state (bb = rr, tol2 = rtol^2 bb).
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restrict__ M, const T* __restrict__ b,
-                                                    T* x, T* r, double* part, PcgState* st, double rtol, int maxit) {
+                                                    T* x, T* r, T* z, double* part, PcgState* st, double rtol, int maxit) {
     Dot<T> v[2];
     Dot<T>&d_rz = v[0], &d_rr = v[1];
     const int64_t total_t = n * R;
@@ -54,6 +55,11 @@ __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restric
             r[o] = r0;
             r[o + R] = r1;
             r[o + 2 * R] = r2;
+            if constexpr (sizeof(T) == 8) {
+                z[o] = z0;
+                z[o + R] = z1;
+                z[o + 2 * R] = z2;
+            }
             d_rz.add(r0, z0);
             d_rz.add(r1, z1);
             d_rz.add(r2, z2);
@@ -93,15 +99,17 @@ __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restric
     }
 }
 
-// x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration).  One
-// thread per node and V right-hand sides (rows of r, x and p on V * sizeof(T)-byte boundaries).
+// x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration; FP64: the
+// z of k_r_update: formed here again an iteration of 8 right-hand sides and 65,331 nodes took 304 us,
+// 297 with z read).  One thread per node and V right-hand sides (rows of r, z, x and p on V * sizeof(T)-byte
+// boundaries).
 template <typename T, int V>
 struct alignas(V * sizeof(T)) Pack {
     T v[V];
 };
 template <typename T, int R, int V>
 __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __restrict__ M, const T* __restrict__ r,
-                                                         T* x, T* p, const PcgState* __restrict__ st) {
+                                                         const T* __restrict__ zv, T* x, T* p, const PcgState* __restrict__ st) {
     if (st->done) return;
     using P = Pack<T, V>;
     const bool first = st->it == 0;
@@ -113,19 +121,20 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
         P rv[3], xv[3], pv[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            rv[j] = *reinterpret_cast<const P*>(r + o + j * R);
+            rv[j] = *reinterpret_cast<const P*>((sizeof(T) == 8 ? zv : r) + o + j * R);
             if (!first) {
                 xv[j] = *reinterpret_cast<const P*>(x + o + j * R);
                 pv[j] = *reinterpret_cast<const P*>(p + o + j * R);
             }
         }
         T m[9];
+        if constexpr (sizeof(T) == 4)
 #pragma unroll
-        for (int q = 0; q < 9; ++q) m[q] = __ldg(M + 9 * node + q);
+            for (int q = 0; q < 9; ++q) m[q] = __ldg(M + 9 * node + q);
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-            T z[3];
-            apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], z[0], z[1], z[2]);
+            T z[3] = {rv[0].v[i], rv[1].v[i], rv[2].v[i]};
+            if constexpr (sizeof(T) == 4) apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], z[0], z[1], z[2]);
             const T a = T(st->alpha[k + i]), b = T(st->beta[k + i]);
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
@@ -415,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) k_p_update(int64_t nv, const T* __re
 // product's critical path, and the recurrence drifts from A p in FP32.)
 // kPad (FP32, one right-hand side, padded row-SoA matrix): p holds 4 floats a node, and k_step_r forms alpha.
 template <typename T, int R, int LPR, bool kPad>
-__global__ void __launch_bounds__(kThreads, spmm_ctas<T, R>())
+__global__ void __launch_bounds__(kThreads, spmm_ctas<T, R, true>())
     k_spmv_pq(const BsrView<T> A, const T* __restrict__ p, T* __restrict__ q, double* part, PcgState* st) {
     if (st->done) return;
     Dot<T> v[1];
@@ -456,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, spmm_ctas<T, R>())
 // r -= alpha q; z = M r; rz, rr -> beta, convergence, iteration count.
 template <typename T, int R>
 __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __restrict__ M, const T* __restrict__ q,
-                                                        T* r, double* part, PcgState* st) {
+                                                        T* r, T* z, double* part, PcgState* st) {
     if (st->done) return;
     Dot<T> v[2];
     Dot<T>&d_rz = v[0], &d_rr = v[1];
@@ -474,6 +483,11 @@ __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __res
             r[o + 2 * R] = r2;
             T z0, z1, z2;
             apply_block(M + 9 * node, r0, r1, r2, z0, z1, z2);
+            if constexpr (sizeof(T) == 8) {
+                z[o] = z0;
+                z[o + R] = z1;
+                z[o + 2 * R] = z2;
+            }
             d_rz.add(r0, z0);
             d_rz.add(r1, z1);
             d_rz.add(r2, z2);
@@ -848,7 +862,7 @@ inline unsigned step_grid(int64_t n) {
 inline bool pad_direction(const BsrView<float>& A) { return A.rsoa == 2; }
 
 template <typename T, int R>
-int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* p, T* q, double* part, PcgState* st, int variant,
+int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* z, T* p, T* q, double* part, PcgState* st, int variant,
                       int count, cudaStream_t s) {
     // 16-byte packs of right-hand sides where the rows of r, p and x (the caller's U in the FP64 solve)
     // start on 16-byte boundaries
@@ -868,11 +882,11 @@ int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* p, T* q, d
     }
     for (int i = 0; i < count; ++i) {
         if (aligned16(x))
-            k_xp_update<T, R, V><<<vec_grid(k_xp_update<T, R, V>, A.n * (R / V)), kThreads, 0, s>>>(A.n, M, r, x, p, st);
+            k_xp_update<T, R, V><<<vec_grid(k_xp_update<T, R, V>, A.n * (R / V)), kThreads, 0, s>>>(A.n, M, r, z, x, p, st);
         else
-            k_xp_update<T, R, 1><<<vec_grid(k_xp_update<T, R, 1>, A.n * R), kThreads, 0, s>>>(A.n, M, r, x, p, st);
+            k_xp_update<T, R, 1><<<vec_grid(k_xp_update<T, R, 1>, A.n * R), kThreads, 0, s>>>(A.n, M, r, z, x, p, st);
         launch_spmv_pq<T, R>(A, p, q, part, st, variant, s);
-        k_r_update<T, R><<<vec_grid(k_r_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, q, r, part, st);
+        k_r_update<T, R><<<vec_grid(k_r_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, q, r, z, part, st);
     }
     FEM_LAUNCH_CHECK("pcg iteration");
     return FEM_OK;
@@ -943,18 +957,19 @@ int pcg_drive(const Init& init, const Iters& iters, PcgState* st, int maxit, int
     return FEM_OK;
 }
 
-// Runs PCG on (A, M) with right-hand side b into x; vectors r p q are workspace (16-byte aligned).
+// Runs PCG on (A, M) with right-hand side b into x; vectors r, z (FP64 only), p, q are workspace (16-byte
+// aligned).
 template <typename T, int R>
-int pcg_core(const BsrView<T>& A, const T* M, const T* b, T* x, T* r, T* p, T* q, double* part, PcgState* st,
+int pcg_core(const BsrView<T>& A, const T* M, const T* b, T* x, T* r, T* z, T* p, T* q, double* part, PcgState* st,
              double rtol, int maxit, int variant, int use_graph, int unroll, cudaStream_t s, InnerResult* res,
              int stall = 0) {
     auto init = [&](cudaStream_t ss) -> int {
-        k_init<T, R><<<vec_grid(k_init<T, R>, A.n * R), kThreads, 0, ss>>>(A.n, M, b, x, r, part, st, rtol, maxit);
+        k_init<T, R><<<vec_grid(k_init<T, R>, A.n * R), kThreads, 0, ss>>>(A.n, M, b, x, r, z, part, st, rtol, maxit);
         FEM_LAUNCH_CHECK("k_init");
         return FEM_OK;
     };
     auto iters = [&](int count, cudaStream_t ss) -> int {
-        return launch_iterations<T, R>(A, M, x, r, p, q, part, st, variant, count, ss);
+        return launch_iterations<T, R>(A, M, x, r, z, p, q, part, st, variant, count, ss);
     };
     int rc = pcg_drive(init, iters, st, maxit, use_graph, unroll, s, res, stall);
     if (rc) return rc;
@@ -1085,7 +1100,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
                 return pcg_core_amg<double, R>(K64, K32, amg, b, x, r, z, p, q, part, st, tol, cap, o->spmv_variant,
                                                o->use_graph, o->unroll, s, &ir, o->stall_window);
             }
-            return pcg_core<double, R>(K64, M64, b, x, r, p, q, part, st, tol, cap, o->spmv_variant,
+            return pcg_core<double, R>(K64, M64, b, x, r, z, p, q, part, st, tol, cap, o->spmv_variant,
                                        o->use_graph, o->unroll, s, &ir, o->stall_window);
         };
         int rc = core(F, U, o->rtol, maxit);
@@ -1150,7 +1165,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
                                             std::max(1, o->inner_maxit), o->spmv_variant32, o->use_graph, o->unroll,
                                             s, &ir, o->stall_window);
             else
-                rc = pcg_core<float, R>(K32, M32, b32, d32, rr, pp, qq, part, st, o->inner_rtol,
+                rc = pcg_core<float, R>(K32, M32, b32, d32, rr, nullptr, pp, qq, part, st, o->inner_rtol,
                                         std::max(1, o->inner_maxit), o->spmv_variant32, o->use_graph, o->unroll, s,
                                         &ir, o->stall_window);
             if (rc) return rc;

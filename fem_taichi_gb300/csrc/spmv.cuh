@@ -289,10 +289,14 @@ struct alignas(4 * V) FloatVec {
 };
 constexpr int kStage = 2;          // rows of a warp in shared memory
 constexpr int kStageSlots = 32;    // longest staged row; longer ones are read in place
-// CTAs per SM of the kernels around spmm_rows_epi (see spmm4_rows_epi)
-template <typename T, int R>
+// CTAs per SM of the kernels around the products, for the compiler's registers (FP32: see spmm4_rows_epi,
+// spmv4_rows_epi).  FP64 (bound by its pipe at 27 blocks a row): 4 for many right-hand sides with p.q, no bound
+// otherwise.  With 1 it unrolls to 136 registers (product of 66,411 rows, 32 right-hand sides: 1.76 ms against
+// 1.71); 65,331 rows, 8 right-hand sides: product 219 us without a bound and 222 with 4, solver iteration
+// 299 and 287.
+template <typename T, int R, bool kDot = false>
 constexpr int spmm_ctas() {
-    return sizeof(T) != 4 || R == 1 ? 1 : R == 32 ? 2 : 3;
+    return sizeof(T) == 8 ? (kDot && R > 1 ? 4 : 0) : R == 1 ? 1 : R == 32 ? 2 : 3;
 }
 
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
@@ -466,6 +470,7 @@ __device__ __forceinline__ Dot<T> spmm_rows_epi(const BsrView<T>& A, const T* __
         const int L = __ldg(A.indptr + row + 1) - int(rs);
         T a0 = 0, a1 = 0, a2 = 0;
         const int64_t vs = A.rsoa ? int64_t(L) : 1;
+#pragma unroll 3
         for (int l = 0; l < L; ++l) {
             const int64_t c = __ldg(A.indices + rs + l);
             const T* v = block_value(A, rs, L, l, 0);
