@@ -766,6 +766,6 @@ extern "C" int fem_amg_vcycle(fem_amg* h, const fem_bsr* A32, int nrhs, const fl
     int rc = ensure_vectors(h, nrhs);
     if (rc) return rc;
     const BsrView<float> A{A32->n_brow, A32->indptr, A32->indices, static_cast<const float*>(A32->vals),
-                           rsoa_kind(A32->layout)};
+                           rsoa_kind(A32->layout), value_stream(A32, nrhs, true)};
     return vcycle(h, A, r, z, static_cast<const pcgd::PcgState*>(h->d_state), nrhs, symmetric != 0, as_stream(stream));
 }

@@ -1096,7 +1096,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
         auto core = [&](const double* b, double* x, double tol, int cap) -> int {
             if (amg) {
                 const BsrView<float> K32{n, A32->indptr, A32->indices, static_cast<const float*>(A32->vals),
-                                         rsoa_kind(A32->layout)};
+                                         rsoa_kind(A32->layout), value_stream(A32, R, amg != nullptr)};
                 return pcg_core_amg<double, R>(K64, K32, amg, b, x, r, z, p, q, part, st, tol, cap, o->spmv_variant,
                                                o->use_graph, o->unroll, s, &ir, o->stall_window);
             }
@@ -1137,7 +1137,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
         }
     } else {
         BsrView<float> K32{n, A32->indptr, A32->indices, static_cast<const float*>(A32->vals),
-                           rsoa_kind(A32->layout)};
+                           rsoa_kind(A32->layout), value_stream(A32, R, amg != nullptr)};
         double* r64 = reinterpret_cast<double*>(ws + L.v64[1]);
         float* b32 = reinterpret_cast<float*>(ws + L.v32[0]);
         float* d32 = reinterpret_cast<float*>(ws + L.v32[1]);

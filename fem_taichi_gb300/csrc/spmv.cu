@@ -16,6 +16,13 @@ int sm_count() {
     return n;
 }
 
+int value_stream(const fem_bsr* A, int nrhs, bool multigrid) {
+    int dev = 0, l2 = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) return 0;
+    const int64_t values = 9 * 4 * A->nnzb, vectors = 4 * 3 * 4 * A->n_brow * nrhs;
+    return A->dtype == FEM_F32 && values * (multigrid ? 2 : 1) + vectors > int64_t(l2) / 8 * 5;
+}
+
 int resident_ctas(const void* kernel, int threads, size_t smem) {
     struct Entry {
         const void* kernel;
@@ -209,7 +216,7 @@ int bsr_spmv_any(const fem_bsr* A, int nrhs, const void* x, void* y, int variant
         return launch_spmv<double>(v, nrhs, static_cast<const double*>(x), static_cast<double*>(y), variant, st);
     }
     BsrView<float> v{A->n_brow, A->indptr, A->indices, static_cast<const float*>(A->vals),
-                     rsoa_kind(A->layout)};
+                     rsoa_kind(A->layout), value_stream(A, nrhs)};
     return launch_spmv<float>(v, nrhs, static_cast<const float*>(x), static_cast<float*>(y), variant, st);
 }
 

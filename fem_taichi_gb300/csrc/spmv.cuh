@@ -22,6 +22,7 @@ struct BsrView {
     const int32_t* indices; // [nnzb]
     const T* vals;          // [nnzb][3][3] (BSR) or, per block row, [9][row length] (row-SoA)
     int rsoa;               // 1: row-SoA value layout; 2: row-SoA padded to 4-block multiples (FP32)
+    int stream = 0;         // the values leave L2 first (value_stream; padded row-SoA only)
 };
 
 // Dot-product accumulator of the solver.  FP64 vectors: plain FP64 fused multiply-adds.
@@ -147,6 +148,29 @@ struct StoreYPad {
     }
 };
 
+// Whether A's values should be the first to leave L2 when it needs room.  An iteration reads them once and
+// a handful of vectors several times; a matrix that does not fit pushes those out as well, one that fits
+// would only be pushed out itself.  Microseconds an iteration of the FP32 solve with and without, one
+// right-hand side: 65,000 nodes (63 MB of values) 25.9 and 22.9, 86,000 29.0 and 28.9, 97,000 30.6 and 33.7,
+// 214,221 (200 MB) 50.5 and 58.3 (L2: 129 MB).  What else the iteration reads counts as well: at 65,000
+// nodes 66.5 and 72.3 with eight right-hand sides, 353 and 372 with multigrid, whose transfers and
+// coarse levels are about as large again.  The columns stay with the vectors: 52.3 with both streamed.
+int value_stream(const fem_bsr* A, int nrhs, bool multigrid = false);
+
+// The L2 policy of loads that are (first = 1) or are not the first to leave
+__device__ __forceinline__ uint64_t l2_policy(int first) {
+    uint64_t f, k;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(f));
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(k));
+    return first ? f : k;
+}
+__device__ __forceinline__ float4 load_l2(const float4* p, uint64_t pol) {
+    float4 v;
+    asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
+    return v;
+}
+
 // Padded row-SoA FP32 product: each lane takes 4 consecutive slots of its row per step and
 // reads each of the 9 values of those 4 blocks with one 16-byte load (rows, values and
 // slot groups all start on 16-byte boundaries); padding blocks hold zeros.  kPad: x holds 4 floats a
@@ -161,6 +185,7 @@ __device__ __forceinline__ Dot<float> spmv4_rows_epi(const BsrView<float>& A, co
     const int lane = threadIdx.x & 31;
     const int sub = lane / LPR, sl = lane % LPR;
     constexpr int RPW = 32 / LPR;
+    const uint64_t pol = l2_policy(A.stream);
     const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t stride = ((int64_t(gridDim.x) * blockDim.x) >> 5) * RPW;
     Dot<float> dot;
@@ -195,7 +220,7 @@ __device__ __forceinline__ Dot<float> spmv4_rows_epi(const BsrView<float>& A, co
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 9; ++q) w[q] = __ldg(reinterpret_cast<const float4*>(v0 + int64_t(q) * L));
+            for (int q = 0; q < 9; ++q) w[q] = load_l2(reinterpret_cast<const float4*>(v0 + int64_t(q) * L), pol);
             return [=](float& b0, float& b1, float& b2) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -299,6 +324,10 @@ constexpr int spmm_ctas() {
     return sizeof(T) == 8 ? (kDot && R > 1 ? 4 : 0) : R == 1 ? 1 : R == 32 ? 2 : 3;
 }
 
+__device__ __forceinline__ void copy_async16(void* dst, const void* src, uint64_t pol) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(
+                     unsigned(__cvta_generic_to_shared(dst))), "l"(src), "l"(pol));
+}
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(dst))), "l"(src));
 }
@@ -316,6 +345,7 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
     using X = FloatVec<V>;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = lane / LP, sub = lane % LP;
+    const uint64_t pol = l2_policy(A.stream);
     Dot<float> dot;
     const int64_t first = int64_t(blockIdx.x) * kWarps + wid, stride = int64_t(gridDim.x) * kWarps;
     const int steps = first < A.n ? int((A.n - first + stride - 1) / stride) : 0;
@@ -345,7 +375,7 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
                 const float* v = A.vals + 9 * r0;
 #pragma unroll
                 for (int i = 0; i < 9 * kStageSlots / 4; i += 32)
-                    if (i + lane < 9 * L / 4) copy_async16(st.val + 4 * (i + lane), v + 4 * (i + lane));
+                    if (i + lane < 9 * L / 4) copy_async16(st.val + 4 * (i + lane), v + 4 * (i + lane), pol);
                 if (lane < L / 4) copy_async16(st.col + 4 * lane, A.indices + r0 + 4 * lane);
             }
         }
