@@ -7,9 +7,9 @@
 // than the extra vector, keeps it) and x waits for the kernel that reads p anyway,
 // so an iteration streams 8 vectors beside the product instead of 10; one more kernel after the last
 // iteration adds the pending alpha p.  All scalars live in a device state block:
-// every reduction writes per-CTA partials and the last CTA to finish (atomic ticket) sums
-// them in CTA order, so results are bitwise reproducible, and computes alpha / beta /
-// convergence on the device.  Each kernel returns immediately once the state says the
+// every reduction writes per-CTA partials and the last CTA to finish (atomic ticket; with one FP32
+// right-hand side every CTA of the next kernel, see k_step_p) sums them in CTA order, so results are
+// bitwise reproducible, and computes alpha / beta / convergence on the device.  Each kernel returns immediately once the state says the
 // solve is done, so a CUDA graph holding `unroll` iterations can be replayed without a
 // host round trip per iteration; the host reads the state once per replay and stops at
 // convergence or at the iteration cap.  Up to 32 right-hand sides run in lockstep with
@@ -113,10 +113,16 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
     if (st->done) return;
     using P = Pack<T, V>;
     const bool first = st->it == 0;
+    const int k = int(threadIdx.x % (R / V)) * V;  // R / V divides the CTA's threads
+    T a[V], b[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        a[i] = T(st->alpha[k + i]);
+        b[i] = T(st->beta[k + i]);
+    }
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n * (R / V);
          t += int64_t(gridDim.x) * blockDim.x) {
         const int64_t node = t / (R / V);
-        const int k = int(t % (R / V)) * V;
         const int64_t o = 3 * node * R + k;
         P rv[3], xv[3], pv[3];
 #pragma unroll
@@ -135,11 +141,10 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
         for (int i = 0; i < V; ++i) {
             T z[3] = {rv[0].v[i], rv[1].v[i], rv[2].v[i]};
             if constexpr (sizeof(T) == 4) apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], z[0], z[1], z[2]);
-            const T a = T(st->alpha[k + i]), b = T(st->beta[k + i]);
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                if (!first) xv[j].v[i] += a * pv[j].v[i];
-                pv[j].v[i] = first ? z[j] : T(z[j] + b * pv[j].v[i]);
+                if (!first) xv[j].v[i] += a[i] * pv[j].v[i];
+                pv[j].v[i] = first ? z[j] : T(z[j] + b[i] * pv[j].v[i]);
             }
         }
 #pragma unroll
@@ -462,38 +467,48 @@ __global__ void __launch_bounds__(kThreads, spmm_ctas<T, R, true>())
     }
 }
 
-// r -= alpha q; z = M r; rz, rr -> beta, convergence, iteration count.
-template <typename T, int R>
+// r -= alpha q; z = M r; rz, rr -> beta, convergence, iteration count.  One thread per node and V right-hand
+// sides, few CTAs (kRUpdateCtas): 137,781 nodes and 32 right-hand sides took 69 us of 23 us of HBM time with
+// one right-hand side a thread, alpha converted from FP64 for every node, and a last CTA that added up 1,216
+// CTAs' sums; 43 us here.
+template <typename T, int R, int V>
 __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __restrict__ M, const T* __restrict__ q,
                                                         T* r, T* z, double* part, PcgState* st) {
     if (st->done) return;
-    Dot<T> v[2];
-    Dot<T>&d_rz = v[0], &d_rr = v[1];
-    const int64_t total_t = n * R;
-    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < ((total_t + 31) / 32) * 32;
-         t += int64_t(gridDim.x) * blockDim.x) {
-        if (t < total_t) {
-            const int64_t node = t / R;
-            const int k = int(t % R);
-            const int64_t o = 3 * node * R + k;
-            const T a = T(st->alpha[k]);
-            const T r0 = r[o] - a * q[o], r1 = r[o + R] - a * q[o + R], r2 = r[o + 2 * R] - a * q[o + 2 * R];
-            r[o] = r0;
-            r[o + R] = r1;
-            r[o + 2 * R] = r2;
-            T z0, z1, z2;
-            apply_block(M + 9 * node, r0, r1, r2, z0, z1, z2);
-            if constexpr (sizeof(T) == 8) {
-                z[o] = z0;
-                z[o + R] = z1;
-                z[o + 2 * R] = z2;
+    using P = Pack<T, V>;
+    Dot<T> v[2][V];
+    const int k0 = int(threadIdx.x % (R / V)) * V;
+    T a[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) a[i] = T(st->alpha[k0 + i]);
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n * (R / V); t += stride) {
+        const int64_t node = t / (R / V);
+        const int64_t o = 3 * node * R + k0;
+        P rv[3], qv[3], zv[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            rv[j] = *reinterpret_cast<const P*>(r + o + j * R);
+            qv[j] = *reinterpret_cast<const P*>(q + o + j * R);
+        }
+        T m[9];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) m[j] = __ldg(M + 9 * node + j);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) rv[j].v[i] -= a[i] * qv[j].v[i];
+            apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], zv[0].v[i], zv[1].v[i], zv[2].v[i]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                v[0][i].add(rv[j].v[i], zv[j].v[i]);
+                v[1][i].add(rv[j].v[i], rv[j].v[i]);
             }
-            d_rz.add(r0, z0);
-            d_rz.add(r1, z1);
-            d_rz.add(r2, z2);
-            d_rr.add(r0, r0);
-            d_rr.add(r1, r1);
-            d_rr.add(r2, r2);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            *reinterpret_cast<P*>(r + o + j * R) = rv[j];
+            if constexpr (sizeof(T) == 8) *reinterpret_cast<P*>(z + o + j * R) = zv[j];
         }
     }
     if (block_partials<R, 2>(v, part, &st->ticket)) {
@@ -670,8 +685,7 @@ __global__ void __launch_bounds__(kThreads) k_rz(int64_t nv, const T* __restrict
 }
 
 // ---- FP64 refinement helpers --------------------------------------------------------------
-// True residual r = F - A u per scalar row with its rounding scale |F| + |A||u|; per RHS
-// ||r||^2 -> st->norm2 and || |F| + |A||u| ||^2 -> st->anorm2.  kExtra: each row sum is the
+// True residual r = F - A u per scalar row; per RHS ||r||^2 -> st->norm2.  kExtra: each row sum is the
 // compensated dot product "Dot2" of Ogita, Rump and Oishi (SIAM J. Sci. Comput. 26 (2005)
 // 1955-1988): every product is split exactly into its rounded value and error by an FMA,
 // every addition by Knuth's two-sum, and the errors are summed alongside, so r is as
@@ -682,7 +696,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
                                                           const double* __restrict__ u, double* r, double* part,
                                                           PcgState* st) {
     const int64_t nv = 3 * A.n * R;
-    Dot<double> v[2];
+    Dot<double> v[1];
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < ((nv + 31) / 32) * 32;
          e += int64_t(gridDim.x) * blockDim.x) {
         if (e < nv) {
@@ -693,7 +707,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
             const int64_t rs = __ldg(A.indptr + node);
             const int L = __ldg(A.indptr + node + 1) - int(rs);
             const double f = F[e];
-            double s = f, comp = 0.0, sc = fabs(f);
+            double s = f, comp = 0.0;
             for (int l = 0; l < L; ++l) {
                 const int64_t col = __ldg(A.indices + rs + l);
                 const double* ub = u + 3 * col * R + k;
@@ -701,7 +715,6 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
                 for (int q = 0; q < 3; ++q) {
                     const double m = __ldg(block_value(A, rs, L, l, 3 * c + q));
                     const double x = ub[q * R];
-                    sc = fma(fabs(m), fabs(x), sc);
                     if (kExtra) {
                         const double pr = __dmul_rn(m, x);
                         const double pe = fma(m, x, -pr);  // m x = pr + pe exactly
@@ -718,16 +731,44 @@ __global__ void __launch_bounds__(kThreads) k_residual_ex(const BsrView<double> 
             const double rv = kExtra ? __dadd_rn(s, comp) : s;
             r[e] = rv;
             v[0].add(rv, rv);
-            v[1].add(sc, sc);
         }
     }
-    if (block_partials<R, 2>(v, part, &st->ticket)) {
-        __shared__ double tot[2][kMaxR];
-        last_block_totals<R, 2>(part, gridDim.x, tot);
-        if (threadIdx.x < R) {
-            st->norm2[threadIdx.x] = tot[0][threadIdx.x];
-            st->anorm2[threadIdx.x] = tot[1][threadIdx.x];
+    if (block_partials<R, 1>(v, part, &st->ticket)) {
+        __shared__ double tot[1][kMaxR];
+        last_block_totals<R, 1>(part, gridDim.x, tot);
+        if (threadIdx.x < R) st->norm2[threadIdx.x] = tot[0][threadIdx.x];
+        __syncthreads();
+        if (threadIdx.x == 0) st->ticket = 0;
+    }
+}
+
+// || |F| + |A||u| ||^2, the rounding scale of the residual of u.  Once for the u that is returned: formed
+// beside every residual it was half of their FP64 work (137,781 rows, 32 right-hand sides: 3.50 ms a
+// residual, 1.92 ms without and 1.97 ms once here).
+template <int R>
+__global__ void __launch_bounds__(kThreads) k_residual_scale(const BsrView<double> A, const double* __restrict__ F,
+                                                             const double* __restrict__ u, double* part, PcgState* st) {
+    const int64_t nv = 3 * A.n * R;
+    Dot<double> v[1];
+    for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < nv; e += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t rowc = e / R;  // scalar row 3 node + c
+        const int k = int(e % R);
+        const int64_t node = rowc / 3;
+        const int c = int(rowc - 3 * node);
+        const int64_t rs = __ldg(A.indptr + node);
+        const int L = __ldg(A.indptr + node + 1) - int(rs);
+        double sc = fabs(F[e]);
+        for (int l = 0; l < L; ++l) {
+            const double* ub = u + 3 * int64_t(__ldg(A.indices + rs + l)) * R + k;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) sc = fma(fabs(__ldg(block_value(A, rs, L, l, 3 * c + q))), fabs(ub[q * R]), sc);
         }
+        v[0].add(sc, sc);
+    }
+    if (block_partials<R, 1>(v, part, &st->ticket)) {
+        __shared__ double tot[1][kMaxR];
+        last_block_totals<R, 1>(part, gridDim.x, tot);
+        if (threadIdx.x < R) st->anorm2[threadIdx.x] = tot[0][threadIdx.x];
         __syncthreads();
         if (threadIdx.x == 0) st->ticket = 0;
     }
@@ -750,7 +791,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_zero(int64_t nv, const do
     if (block_partials<R, 1>(v, part, &st->ticket)) {
         __shared__ double tot[1][kMaxR];
         last_block_totals<R, 1>(part, gridDim.x, tot);
-        if (threadIdx.x < R) st->norm2[threadIdx.x] = st->anorm2[threadIdx.x] = tot[0][threadIdx.x];
+        if (threadIdx.x < R) st->norm2[threadIdx.x] = tot[0][threadIdx.x];
         __syncthreads();
         if (threadIdx.x == 0) st->ticket = 0;
     }
@@ -861,6 +902,9 @@ inline unsigned step_grid(int64_t n) {
 // One FP32 right-hand side on the padded row-SoA copy: the search direction has 4 floats a node.
 inline bool pad_direction(const BsrView<float>& A) { return A.rsoa == 2; }
 
+// CTAs of the residual update per SM: enough loads in flight, few sums for its last CTA to add
+constexpr int kRUpdateCtas = 4;
+
 template <typename T, int R>
 int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* z, T* p, T* q, double* part, PcgState* st, int variant,
                       int count, cudaStream_t s) {
@@ -886,7 +930,8 @@ int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* z, T* p, T
         else
             k_xp_update<T, R, 1><<<vec_grid(k_xp_update<T, R, 1>, A.n * R), kThreads, 0, s>>>(A.n, M, r, z, x, p, st);
         launch_spmv_pq<T, R>(A, p, q, part, st, variant, s);
-        k_r_update<T, R><<<vec_grid(k_r_update<T, R>, A.n * R), kThreads, 0, s>>>(A.n, M, q, r, z, part, st);
+        const unsigned g = std::min<unsigned>(vec_grid(k_r_update<T, R, V>, A.n * (R / V)), sm_count() * kRUpdateCtas);
+        k_r_update<T, R, V><<<g, kThreads, 0, s>>>(A.n, M, q, r, z, part, st);
     }
     FEM_LAUNCH_CHECK("pcg iteration");
     return FEM_OK;
@@ -1040,7 +1085,7 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
     const bool extra = o->residual == FEM_RESIDUAL_EXTRA;
     InnerResult ir{0, FEM_OK};
     PcgState h;
-    // r = F - K u (FP64 or compensated), its norms and rounding scales -> h
+    // r = F - K u (FP64 or compensated), its norms -> h
     auto true_residual = [&](const double* u, double* r) -> int {
         if (extra)
             k_residual_ex<R, true><<<vec_grid(k_residual_ex<R, true>, nv), kThreads, 0, s>>>(K64, F, u, r, part, st);
@@ -1192,6 +1237,10 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
     // that stopped above rtol (iteration cap, stall, recursive residual drifting from the true
     // one) does not report success.
     const double worst = worst_rel();
+    k_residual_scale<R><<<vec_grid(k_residual_scale<R>, nv), kThreads, 0, s>>>(K64, F, U, part, st);
+    FEM_LAUNCH_CHECK("k_residual_scale");
+    FEM_CUDA(cudaMemcpyAsync(&h, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
+    FEM_CUDA(cudaStreamSynchronize(s));
     double floor_rel = 0.0;
     for (int k = 0; k < R; ++k)
         if (bnorm[k] > 0) floor_rel = std::max(floor_rel, 0x1p-53 * sqrt(h.anorm2[k]) / bnorm[k]);

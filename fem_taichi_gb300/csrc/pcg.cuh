@@ -23,15 +23,23 @@ struct PcgState {
     unsigned ticket;
 };
 
-// This CTA's sums of v[s] (per RHS) into part[blockIdx.x] slots slot0 .. slot0 + NS - 1.
-template <int R, int NS, typename T>
-__device__ void write_partials(const Dot<T> (&v)[NS], double* part, int slot0) {
+// This CTA's sums of v[s] (per RHS) into part[blockIdx.x] slots slot0 .. slot0 + NS - 1.  v[s][i] is of
+// right-hand side (lane % (R / V)) V + i; each becomes a double in one lane (rhs_sum would convert the V
+// sums of a warp one after the other on the FP64 pipe).
+template <int R, int NS, int V, typename T>
+__device__ void write_partials(const Dot<T> (&v)[NS][V], double* part, int slot0) {
     __shared__ double sm[kThreads / 32][NS][kMaxR];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-        const double w = rhs_sum<R>(v[s]);
-        if (lane < R) sm[warp][s][lane] = w;
+        Dot<T> d = rhs_dot<R / V>(v[s][0]);
+#pragma unroll
+        for (int i = 1; i < V; ++i) {
+            const Dot<T> di = rhs_dot<R / V>(v[s][i]);
+            if (lane / (R / V) == i) d = di;
+        }
+        const double w = d.value();
+        if (lane < R) sm[warp][s][lane % (R / V) * V + lane / (R / V)] = w;
     }
     __syncthreads();
     if (threadIdx.x < R) {
@@ -46,16 +54,20 @@ __device__ void write_partials(const Dot<T> (&v)[NS], double* part, int slot0) {
 
 // Block-level reduction of up to kSlots values per RHS into part[blockIdx.x]; returns true
 // in every thread of the CTA that finished last (after which part[] is complete).
-template <int R, int NS, typename T>
-__device__ bool block_partials(const Dot<T> (&v)[NS], double* part, unsigned* ticket) {
+template <int R, int NS, int V, typename T>
+__device__ bool block_partials(const Dot<T> (&v)[NS][V], double* part, unsigned* ticket) {
     __shared__ bool last;
-    write_partials<R, NS, T>(v, part, 0);
+    write_partials<R, NS>(v, part, 0);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (last) __threadfence();
     return last;
+}
+template <int R, int NS, typename T>
+__device__ bool block_partials(const Dot<T> (&v)[NS], double* part, unsigned* ticket) {
+    return block_partials<R, NS>(reinterpret_cast<const Dot<T>(&)[NS][1]>(v), part, ticket);
 }
 
 // In the last CTA (all threads call it): tot[s][k] = sum over CTAs of slot s, RHS k.  The
@@ -66,13 +78,24 @@ __device__ void last_block_totals(const double* part, int nblocks, double (&tot)
     constexpr int G = kThreads / R;
     __shared__ double red[NS][kThreads];
     const int t = threadIdx.x, k = t % R, g = t / R;
+    // 8 of a slot's loads in flight: with 32 right-hand sides a thread reads an eighth of the CTAs' sums,
+    // and waiting for each four of them was most of the residual update's tail
+    double acc[NS] = {};
+    for (int b = g; b < nblocks; b += 8 * G) {
+        double w[NS][8];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        double acc = 0.0;
-#pragma unroll 4
-        for (int b = g; b < nblocks; b += G) acc += __ldcg(part + (int64_t(b) * kSlots + slot0 + s) * kMaxR + k);
-        red[s][t] = acc;
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                w[s][i] = b + i * G < nblocks ? __ldcg(part + (int64_t(b + i * G) * kSlots + slot0 + s) * kMaxR + k) : 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                if (b + i * G < nblocks) acc[s] += w[s][i];
     }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) red[s][t] = acc[s];
     __syncthreads();
 #pragma unroll
     for (int off = G / 2; off >= 1; off >>= 1) {

@@ -55,14 +55,16 @@ struct Dot<float> {
 // pairs are added as pairs (two-sums on the FP32 pipes; the FP64 form's five adds and the
 // conversions cost 16 FP64 cycles each per warp and SM).
 template <int R>
-__device__ __forceinline__ double rhs_sum(const Dot<double>& d) {
+__device__ __forceinline__ Dot<double> rhs_dot(const Dot<double>& d) {
     double v = d.value();
 #pragma unroll
     for (int off = 16; off >= R; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
+    Dot<double> out;
+    out.v = v;
+    return out;
 }
 template <int R>
-__device__ __forceinline__ double rhs_sum(const Dot<float>& d) {
+__device__ __forceinline__ Dot<float> rhs_dot(const Dot<float>& d) {
     float s = d.s, c = d.c;
 #pragma unroll
     for (int off = 16; off >= R; off >>= 1) {
@@ -73,7 +75,14 @@ __device__ __forceinline__ double rhs_sum(const Dot<float>& d) {
         s = t;
         c = __fadd_rn(__fadd_rn(c, c2), err);
     }
-    return double(s) + double(c);
+    Dot<float> out;
+    out.s = s;
+    out.c = c;
+    return out;
+}
+template <int R, typename T>
+__device__ __forceinline__ double rhs_sum(const Dot<T>& d) {
+    return rhs_dot<R>(d).value();
 }
 
 // BsrView::rsoa for a fem_bsr layout code
