@@ -20,6 +20,7 @@
 // loop forms the true residual r = F - K u with the FP64 matrix, scales it to unit norm,
 // solves K d = r approximately in FP32, and updates u += |r| d in FP64.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "amg.cuh"
@@ -99,17 +100,15 @@ __global__ void __launch_bounds__(kThreads) k_init(int64_t n, const T* __restric
     }
 }
 
-// x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration; FP64: the
-// z of k_r_update: formed here again an iteration of 8 right-hand sides and 65,331 nodes took 304 us,
-// 297 with z read).  One thread per node and V right-hand sides (rows of r, z, x and p on V * sizeof(T)-byte
-// boundaries).
+// x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration).  One
+// thread per node and V right-hand sides (rows of r, x and p on V * sizeof(T)-byte boundaries).
 template <typename T, int V>
 struct alignas(V * sizeof(T)) Pack {
     T v[V];
 };
 template <typename T, int R, int V>
 __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __restrict__ M, const T* __restrict__ r,
-                                                         const T* __restrict__ zv, T* x, T* p, const PcgState* __restrict__ st) {
+                                                         T* x, T* p, const PcgState* __restrict__ st) {
     if (st->done) return;
     using P = Pack<T, V>;
     const bool first = st->it == 0;
@@ -127,20 +126,19 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
         P rv[3], xv[3], pv[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            rv[j] = *reinterpret_cast<const P*>((sizeof(T) == 8 ? zv : r) + o + j * R);
+            rv[j] = *reinterpret_cast<const P*>(r + o + j * R);
             if (!first) {
                 xv[j] = *reinterpret_cast<const P*>(x + o + j * R);
                 pv[j] = *reinterpret_cast<const P*>(p + o + j * R);
             }
         }
         T m[9];
-        if constexpr (sizeof(T) == 4)
 #pragma unroll
-            for (int q = 0; q < 9; ++q) m[q] = __ldg(M + 9 * node + q);
+        for (int q = 0; q < 9; ++q) m[q] = __ldg(M + 9 * node + q);
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-            T z[3] = {rv[0].v[i], rv[1].v[i], rv[2].v[i]};
-            if constexpr (sizeof(T) == 4) apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], z[0], z[1], z[2]);
+            T z[3];
+            apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], z[0], z[1], z[2]);
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 if (!first) xv[j].v[i] += a[i] * pv[j].v[i];
@@ -152,6 +150,39 @@ __global__ void __launch_bounds__(kThreads) k_xp_update(int64_t n, const T* __re
             if (!first) *reinterpret_cast<P*>(x + o + j * R) = xv[j];
             *reinterpret_cast<P*>(p + o + j * R) = pv[j];
         }
+    }
+}
+
+// The FP64 form, with the z of k_r_update: formed here again an iteration of 8 right-hand sides and 65,331
+// nodes took 304 us, 297 with z read.  One thread per V entries, not per node: a small mesh has three
+// times the threads.
+template <int R, int V>
+__global__ void __launch_bounds__(kThreads) k_xp_update_z(int64_t nv, const double* __restrict__ z, double* x,
+                                                           double* p, const PcgState* __restrict__ st) {
+    if (st->done) return;
+    using P = Pack<double, V>;
+    const bool first = st->it == 0;
+    const int k = int(threadIdx.x * V % R);  // R divides V times the CTA's threads
+    double a[V], b[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        a[i] = st->alpha[k + i];
+        b[i] = st->beta[k + i];
+    }
+    for (int64_t o = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * V; o < nv;
+         o += int64_t(gridDim.x) * blockDim.x * V) {
+        P pv = *reinterpret_cast<const P*>(z + o);
+        if (!first) {
+            const P q = *reinterpret_cast<const P*>(p + o);
+            P xv = *reinterpret_cast<const P*>(x + o);
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                xv.v[i] += a[i] * q.v[i];
+                pv.v[i] += b[i] * q.v[i];
+            }
+            *reinterpret_cast<P*>(x + o) = xv;
+        }
+        *reinterpret_cast<P*>(p + o) = pv;
     }
 }
 
@@ -925,13 +956,22 @@ int launch_iterations(const BsrView<T>& A, const T* M, T* x, T* r, T* z, T* p, T
         }
     }
     for (int i = 0; i < count; ++i) {
-        if (aligned16(x))
-            k_xp_update<T, R, V><<<vec_grid(k_xp_update<T, R, V>, A.n * (R / V)), kThreads, 0, s>>>(A.n, M, r, z, x, p, st);
-        else
-            k_xp_update<T, R, 1><<<vec_grid(k_xp_update<T, R, 1>, A.n * R), kThreads, 0, s>>>(A.n, M, r, z, x, p, st);
+        auto xp = [&](auto pack) {
+            constexpr int W = decltype(pack)::value;
+            if constexpr (sizeof(T) == 8)
+                k_xp_update_z<R, W><<<vec_grid(k_xp_update_z<R, W>, 3 * A.n * R / W), kThreads, 0, s>>>(3 * A.n * R, z, x,
+                                                                                                        p, st);
+            else
+                k_xp_update<T, R, W><<<vec_grid(k_xp_update<T, R, W>, A.n * (R / W)), kThreads, 0, s>>>(A.n, M, r, x, p, st);
+        };
+        if (aligned16(x)) xp(std::integral_constant<int, V>());
+        else xp(std::integral_constant<int, 1>());
         launch_spmv_pq<T, R>(A, p, q, part, st, variant, s);
-        const unsigned g = std::min<unsigned>(vec_grid(k_r_update<T, R, V>, A.n * (R / V)), sm_count() * kRUpdateCtas);
-        k_r_update<T, R, V><<<g, kThreads, 0, s>>>(A.n, M, q, r, z, part, st);
+        // FP64: the sums of two right-hand sides a thread are a longer chain on its pipe than the loads
+        // are worth (2 right-hand sides of 8,125 nodes: 38.9 against 36.6 us an iteration)
+        constexpr int VR = sizeof(T) == 8 ? 1 : V;
+        const unsigned g = std::min<unsigned>(vec_grid(k_r_update<T, R, VR>, A.n * (R / VR)), sm_count() * kRUpdateCtas);
+        k_r_update<T, R, VR><<<g, kThreads, 0, s>>>(A.n, M, q, r, z, part, st);
     }
     FEM_LAUNCH_CHECK("pcg iteration");
     return FEM_OK;

@@ -78,21 +78,31 @@ __device__ void last_block_totals(const double* part, int nblocks, double (&tot)
     constexpr int G = kThreads / R;
     __shared__ double red[NS][kThreads];
     const int t = threadIdx.x, k = t % R, g = t / R;
-    // 8 of a slot's loads in flight: with 32 right-hand sides a thread reads an eighth of the CTAs' sums,
-    // and waiting for each four of them was most of the residual update's tail
+    // Loads of a slot in flight: with 32 right-hand sides a thread reads an eighth of the CTAs' sums, and
+    // waiting for each four of them was most of the residual update's tail; with few it reads one to five,
+    // and the tests of eight cost more (FP64, one right-hand side of 8,125 nodes: 25.4 -> 27.1 us an iteration).
+    constexpr int U = R >= 8 ? 8 : 1;
     double acc[NS] = {};
-    for (int b = g; b < nblocks; b += 8 * G) {
-        double w[NS][8];
+    if constexpr (U == 1) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int s = 0; s < NS; ++s) {
+#pragma unroll 4
+            for (int b = g; b < nblocks; b += G) acc[s] += __ldcg(part + (int64_t(b) * kSlots + slot0 + s) * kMaxR + k);
+        }
+    } else {
+        for (int b = g; b < nblocks; b += U * G) {
+            double w[NS][U];
 #pragma unroll
-            for (int s = 0; s < NS; ++s)
-                w[s][i] = b + i * G < nblocks ? __ldcg(part + (int64_t(b + i * G) * kSlots + slot0 + s) * kMaxR + k) : 0.0;
+            for (int i = 0; i < U; ++i)
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+                for (int s = 0; s < NS; ++s)
+                    w[s][i] = b + i * G < nblocks ? __ldcg(part + (int64_t(b + i * G) * kSlots + slot0 + s) * kMaxR + k) : 0.0;
 #pragma unroll
-            for (int s = 0; s < NS; ++s)
-                if (b + i * G < nblocks) acc[s] += w[s][i];
+            for (int i = 0; i < U; ++i)
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+                    if (b + i * G < nblocks) acc[s] += w[s][i];
+        }
     }
 #pragma unroll
     for (int s = 0; s < NS; ++s) red[s][t] = acc[s];
