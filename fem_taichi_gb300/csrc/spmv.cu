@@ -17,10 +17,12 @@ int sm_count() {
 }
 
 int value_stream(const fem_bsr* A, int nrhs, bool multigrid) {
+    const int64_t values = 9 * 4 * A->nnzb, vectors = 4 * 3 * 4 * A->n_brow * nrhs;
+    const int64_t set = values * (multigrid ? 2 : 1) + vectors;
+    if (A->dtype != FEM_F32 || set < (int64_t(16) << 20)) return 0;  // small calls skip the queries
     int dev = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) return 0;
-    const int64_t values = 9 * 4 * A->nnzb, vectors = 4 * 3 * 4 * A->n_brow * nrhs;
-    return A->dtype == FEM_F32 && values * (multigrid ? 2 : 1) + vectors > int64_t(l2) / 8 * 5;
+    return set > int64_t(l2) / 8 * 5;
 }
 
 int resident_ctas(const void* kernel, int threads, size_t smem) {
