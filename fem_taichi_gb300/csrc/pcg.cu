@@ -262,13 +262,19 @@ __device__ __forceinline__ int64_t step_node(int64_t& stride) {
     return (int64_t(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
 }
 
+// Whether the solve was over when the kernel started, agreed on by the CTA: CTA 0 of the same grid may set
+// `done`, so the warps of a CTA that starts late may read either value, and no warp may leave alone (the
+// others' sums and scalars come through shared memory it fills).  A CTA of which any warp sees it set would
+// have found the same end itself.
+__device__ __forceinline__ bool step_done(const PcgState* st) { return __syncthreads_or(st->done) != 0; }
+
 // x += alpha p of the iteration before; p = z + beta p, z = M r (p = z on the first iteration).  CTA 0
-// records the iteration's outcome; the others form it for themselves and never read what it writes
-// (a CTA that sees `done` already set would have found the same).
+// records the iteration's outcome; the others form it for themselves and read nothing it writes but `done`
+// (step_done).
 __global__ void __launch_bounds__(kStepThreads) k_step_p(int64_t n, const float* __restrict__ M,
                                                           const float* __restrict__ r, float* x, float4* p,
                                                           const double* part, int nb, PcgState* st) {
-    if (st->done) return;
+    if (step_done(st)) return;
     const bool first = st->it == 0;
     __shared__ double sm[8];
     __shared__ float sa, sb;
@@ -337,7 +343,7 @@ __global__ void __launch_bounds__(kStepThreads) k_step_p(int64_t n, const float*
 __global__ void __launch_bounds__(kStepThreads) k_step_r(int64_t n, const float* __restrict__ M,
                                                           const float* __restrict__ q, float* r, double* part, int nb,
                                                           PcgState* st) {
-    if (st->done) return;
+    if (step_done(st)) return;
     __shared__ double sm[4];
     __shared__ float sa;
     __shared__ bool go;
