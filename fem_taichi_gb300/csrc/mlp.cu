@@ -509,13 +509,15 @@ struct SquareSum {
 // Thread per node.  24 squares summed in FP64 were 2 FP64 instructions each on a pipe that takes one per
 // warp and 64 cycles, and single-float accesses 64 and 96 bytes apart 32 sectors each: 214,221 nodes
 // with 8 probes 36 us; with SquareSum and 16-byte accesses 17 us.  SquareSum holds where the
-// largest residual is within [1e-10, 1e18]: below, squares lose bits to the least FP32 exponent; above,
-// they overflow; NaN passes through either way.  Those nodes are summed in FP64.
+// largest of a node's 3 R residuals is at least 1e-10 (below, squares lose bits to the least FP32 exponent)
+// and 3 R times its square at most 1e38 (above, the sum of the squares may overflow); NaN passes through
+// either way.  Other nodes are summed in FP64.
 template <bool kWide>
 __global__ void __launch_bounds__(256) k_loss(int64_t n, int R, const float* __restrict__ out,
                                               const float* __restrict__ yh, const float* __restrict__ zh,
                                               float* dout, double* part, double scale) {
     constexpr int V = kWide ? 4 : 1;
+    const float big2_max = 1e38f / (3.f * float(R));
     double acc = 0.0;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         float o[6];
@@ -573,7 +575,7 @@ __global__ void __launch_bounds__(256) k_loss(int64_t n, int R, const float* __r
                     for (int c = 0; c < 3; ++c) G[3 * r + c] += 2.f * e[r][k] * y[c][k];
             }
         }
-        if (big >= 1e-10f && big <= 1e18f) {
+        if (big >= 1e-10f && big * big <= big2_max) {
             acc += sq.value();
         } else {
             for (int k0 = 0; k0 < R; k0 += V) {
