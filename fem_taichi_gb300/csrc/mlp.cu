@@ -184,7 +184,7 @@ __device__ __forceinline__ void store_row_bf16(unsigned char* tile, int row, int
     // 16 consecutive k values = two 16-byte core rows
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        __nv_bfloat162 p[4];
+        alignas(16) __nv_bfloat162 p[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(v[8 * h + 2 * j], v[8 * h + 2 * j + 1]);
         *reinterpret_cast<uint4*>(tile + core_off(row, k0 + 8 * h, K)) = *reinterpret_cast<uint4*>(p);
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(256) k_loss(int64_t n, int R, const float* __r
         const float* yi = yh + 3 * i * R;
         const float* zi = zh + 3 * i * R;
         auto residual = [&](int k0, float (&y)[3][V], float (&e)[3][V]) {  // of probes k0..
-            float z[3][V];
+            alignas(16) float z[3][V];
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
                 if (kWide) {
@@ -816,7 +816,7 @@ __device__ __forceinline__ void put_cols(unsigned char* tile, int g, int t, uint
     *reinterpret_cast<uint4*>(tile + g * (kTile * 16) + t * 16) = v;
 }
 __device__ __forceinline__ uint4 pack8(const float* v) {
-    __nv_bfloat162 b[4];
+    alignas(16) __nv_bfloat162 b[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) b[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
     return *reinterpret_cast<uint4*>(b);
