@@ -197,19 +197,22 @@ constexpr int kStepThreads = 1024;
 constexpr int kStepNodes = 2;    // nodes of a thread in flight
 constexpr int kPq = 0, kRz = 1;  // slots of kMaxCtas partial sums: p.q; r.z and r.r
 
-// The sums of v over this CTA's W warps to its entries of the slots slot0..
+// The sums of v over this CTA's W warps to its entries of the slots slot0..  The warps' sums become doubles
+// side by side in one warp per slot, not one after the other.
 template <int NS, int W>
 __device__ __forceinline__ void step_partials(const Dot<float> (&v)[NS], double* part, int slot0) {
-    __shared__ double sm[NS][W];
+    __shared__ float sm[NS][3][W];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-        const double w = rhs_sum<1>(v[s]);
-        if (lane == 0) sm[s][warp] = w;
+        const Dot<float> w = rhs_dot<1>(v[s]);
+        if (lane < 3) sm[s][lane][warp] = lane == 0 ? w.s : lane == 1 ? w.c : w.d;
     }
     __syncthreads();
     if (warp < NS) {
-        double a = lane < W ? sm[warp][lane] : 0.0;
+        Dot<float> w;
+        if (lane < W) w.s = sm[warp][0][lane], w.c = sm[warp][1][lane], w.d = sm[warp][2][lane];
+        double a = w.value();
 #pragma unroll
         for (int off = W / 2; off >= 1; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
         if (lane == 0) part[(slot0 + warp) * kMaxCtas + blockIdx.x] = a;
@@ -399,11 +402,8 @@ __global__ void __launch_bounds__(kStepThreads) k_step_r(int64_t n, const float*
                 r[3 * node + j] = rv[h][j];
             }
             apply_block(m[h], rv[h][0], rv[h][1], rv[h][2], z[0], z[1], z[2]);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                v[0].add(rv[h][j], z[j]);
-                v[1].add(rv[h][j], rv[h][j]);
-            }
+            v[0].add3(rv[h][0], z[0], rv[h][1], z[1], rv[h][2], z[2]);
+            v[1].add3(rv[h][0], rv[h][0], rv[h][1], rv[h][1], rv[h][2], rv[h][2]);
         }
         i += kStepNodes * stride;
         if (i >= n) break;
@@ -536,11 +536,8 @@ __global__ void __launch_bounds__(kThreads) k_r_update(int64_t n, const T* __res
 #pragma unroll
             for (int j = 0; j < 3; ++j) rv[j].v[i] -= a[i] * qv[j].v[i];
             apply_block(m, rv[0].v[i], rv[1].v[i], rv[2].v[i], zv[0].v[i], zv[1].v[i], zv[2].v[i]);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                v[0][i].add(rv[j].v[i], zv[j].v[i]);
-                v[1][i].add(rv[j].v[i], rv[j].v[i]);
-            }
+            v[0][i].add3(rv[0].v[i], zv[0].v[i], rv[1].v[i], zv[1].v[i], rv[2].v[i], zv[2].v[i]);
+            v[1][i].add3(rv[0].v[i], rv[0].v[i], rv[1].v[i], rv[1].v[i], rv[2].v[i], rv[2].v[i]);
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j) {

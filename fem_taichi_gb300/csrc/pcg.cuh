@@ -24,8 +24,8 @@ struct PcgState {
 };
 
 // This CTA's sums of v[s] (per RHS) into part[blockIdx.x] slots slot0 .. slot0 + NS - 1.  v[s][i] is of
-// right-hand side (lane % (R / V)) V + i; each becomes a double in one lane (rhs_sum would convert the V
-// sums of a warp one after the other on the FP64 pipe).
+// right-hand side (lane % (R / V)) V + i; each becomes a double in one lane (converting the V sums of a
+// warp one after the other would take the FP64 pipe V times).
 template <int R, int NS, int V, typename T>
 __device__ void write_partials(const Dot<T> (&v)[NS][V], double* part, int slot0) {
     __shared__ double sm[kThreads / 32][NS][kMaxR];

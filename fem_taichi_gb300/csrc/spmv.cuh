@@ -11,6 +11,7 @@
 // count; a fixed grid gives a fixed row -> CTA mapping, hence deterministic partial sums.
 #pragma once
 
+#include "dot.cuh"
 #include "fem_common.cuh"
 
 namespace fem {
@@ -25,64 +26,22 @@ struct BsrView {
     int stream = 0;         // the values leave L2 first (value_stream; padded row-SoA only)
 };
 
-// Dot-product accumulator of the solver.  FP64 vectors: plain FP64 fused multiply-adds.
-// FP32 vectors: every product is formed exactly (FMA error term) and summed with a
-// compensated two-sum in FP32 pairs (about 48 significant bits), and becomes a double once
-// per thread, so the per-element work stays on the FP32 pipes (GB300's FP64 pipe is ~64x
-// slower) while the dot products keep FP64-class accuracy.
-template <typename T>
-struct Dot {
-    double v = 0.0;
-    __device__ __forceinline__ void add(T a, T b) { v = fma(double(a), double(b), v); }
-    __device__ __forceinline__ double value() const { return v; }
-};
-template <>
-struct Dot<float> {
-    float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void add(float a, float b) {
-        const float pr = __fmul_rn(a, b);
-        const float e = __fmaf_rn(a, b, -pr);
-        const float t = __fadd_rn(s, pr);
-        const float bb = __fsub_rn(t, s);
-        const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(pr, bb));
-        s = t;
-        c = __fadd_rn(c, __fadd_rn(err, e));
-    }
-    __device__ __forceinline__ double value() const { return double(s) + double(c); }
-};
-
-// Sum of d over the lanes of a warp that hold the same right-hand side (lane % R), as a double.  FP32
-// pairs are added as pairs (two-sums on the FP32 pipes; the FP64 form's five adds and the
-// conversions cost 16 FP64 cycles each per warp and SM).
+// Sum of d over the lanes of a warp that hold the same right-hand side (lane % R).  FP32 sums are joined on
+// the FP32 pipes (the FP64 form's five adds and the conversions cost 16 FP64 cycles each per warp
+// and SM).
 template <int R>
-__device__ __forceinline__ Dot<double> rhs_dot(const Dot<double>& d) {
-    double v = d.value();
+__device__ __forceinline__ Dot<double> rhs_dot(Dot<double> d) {
 #pragma unroll
-    for (int off = 16; off >= R; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    Dot<double> out;
-    out.v = v;
-    return out;
+    for (int off = 16; off >= R; off >>= 1) d.v += __shfl_xor_sync(0xffffffffu, d.v, off);
+    return d;
 }
 template <int R>
-__device__ __forceinline__ Dot<float> rhs_dot(const Dot<float>& d) {
-    float s = d.s, c = d.c;
+__device__ __forceinline__ Dot<float> rhs_dot(Dot<float> d) {
 #pragma unroll
-    for (int off = 16; off >= R; off >>= 1) {
-        const float s2 = __shfl_xor_sync(0xffffffffu, s, off), c2 = __shfl_xor_sync(0xffffffffu, c, off);
-        const float t = __fadd_rn(s, s2);
-        const float b = __fsub_rn(t, s);
-        const float err = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(s2, b));
-        s = t;
-        c = __fadd_rn(__fadd_rn(c, c2), err);
-    }
-    Dot<float> out;
-    out.s = s;
-    out.c = c;
-    return out;
-}
-template <int R, typename T>
-__device__ __forceinline__ double rhs_sum(const Dot<T>& d) {
-    return rhs_dot<R>(d).value();
+    for (int off = 16; off >= R; off >>= 1)
+        d.join(__shfl_xor_sync(0xffffffffu, d.s, off), __shfl_xor_sync(0xffffffffu, d.c, off),
+               __shfl_xor_sync(0xffffffffu, d.d, off));
+    return d;
 }
 
 // BsrView::rsoa for a fem_bsr layout code
@@ -135,9 +94,7 @@ struct StoreY {
         y[o + stride] = a1;
         y[o + 2 * stride] = a2;
         if (want_dot) {
-            dot.add(x[o], a0);
-            dot.add(x[o + stride], a1);
-            dot.add(x[o + 2 * stride], a2);
+            dot.add3(x[o], a0, x[o + stride], a1, x[o + 2 * stride], a2);
         }
     }
 };
@@ -151,9 +108,7 @@ struct StoreYPad {
         y[o] = a0;
         y[o + 1] = a1;
         y[o + 2] = a2;
-        dot.add(xr.x, a0);
-        dot.add(xr.y, a1);
-        dot.add(xr.z, a2);
+        dot.add3(xr.x, a0, xr.y, a1, xr.z, a2);
     }
 };
 
