@@ -37,6 +37,8 @@
 //     (LoadF, :220-226) are applied in the same pass, and the row is written in either
 //     the BSR block order or the reference's scalar-CSR order (FEM_model_csr.py:150-173).
 #include <climits>
+#include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "fem_common.cuh"
@@ -69,9 +71,9 @@ struct ElemParams {
     int64_t e_begin, e_end;  // elements [e_begin, e_end) of this launch
     double* rec;
     double lm;         // lam / mu
-    double mu8;        // mu / 8
+    double mu8;        // mu / 8 times the square of what dnr is divided by
     double wc[3][3];   // centrifugal operator: f = wc . x (UnitVectorF)
-    DevTables tab;
+    double dnr[8][24]; // dN_a/dxi_i at Gauss point g at [g][3a+i], divided by the largest
     // tm[s][c]: product of the 1D shape factors of two corners along one axis at a Gauss point
     // on the negative (s = 0) or positive (s = 1) side: c = 0 both corners negative, 1 mixed,
     // 2 both positive; tmx the same times DE / 512 (x is contracted first)
@@ -79,12 +81,12 @@ struct ElemParams {
 };
 
 struct ElemSmem {
-    double dnr[8][kRPad];       // dN_a/dxi_i at Gauss point g at [g][3a+i]; padded row: the 8 rows
+    double dnr[8][kRPad];       // ElemParams::dnr; padded row: the 8 rows
                                 // start in 8 different bank pairs (a 24-double row put every
                                 // even g in one bank and every odd g in another)
     double cf[kEpc][8][3];      // Walsh sums of the element-local coordinates; later D1
     double wx[kEpc][8][3];      // W x_a: centrifugal density per unit mass at corner a
-    double R[kEpc][8][kRPad];   // R_a(g)[i] (x 64) at [el][g][3a+i]
+    double R[kEpc][8][kRPad];   // R_a(g)[i] (scaled as dnr, x 64) at [el][g][3a+i]
     double Rs[kEpc][8][kRPad];  // mu R_a(g)[i] / det_g, scaled so that the products have no factor
     double det[kEpc][8];        // x 512
     double d2[kEpc][18];        // second mass contraction
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(kElemThreads, 48 / kEpc) k_hex8_element(const 
     const bool valid = e_raw < p.e_end;
     const int64_t e = valid ? e_raw : p.e_end - 1;   // the lanes of absent elements repeat the last one
 
-    for (int k = tid; k < 8 * 8 * 3; k += kElemThreads) s.dnr[k / 24][k % 24] = (&p.tab.dnr[0][0][0])[k];
+    for (int k = tid; k < 8 * 8 * 3; k += kElemThreads) s.dnr[k / 24][k % 24] = (&p.dnr[0][0])[k];
     double c[3];
     {
         const int64_t node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(kWideEpc * 32) k_hex8_element_wide(const ElemP
     const int64_t e_raw = p.e_begin + int64_t(blockIdx.x) * kWideEpc + el;
     const bool valid = e_raw < p.e_end;
     const int64_t e = valid ? e_raw : p.e_end - 1;
-    for (int k = tid; k < 8 * 8 * 3; k += kWideEpc * 32) s.dnr[k / 24][k % 24] = (&p.tab.dnr[0][0][0])[k];
+    for (int k = tid; k < 8 * 8 * 3; k += kWideEpc * 32) s.dnr[k / 24][k % 24] = (&p.dnr[0][0])[k];
     double c[3];
     {
         const int64_t node = __ldg(reinterpret_cast<const int*>(p.conn4) + 8 * e + t);
@@ -997,6 +999,61 @@ int check_assembly_inputs(const fem_mesh* mesh, const fem_material* mat, void* w
 }  // namespace
 
 namespace fem {
+namespace {
+
+// Unevaluated sum of two doubles, for the constants of the FP64 element kernels.
+struct Pair {
+    double h, l;
+};
+Pair two_sum(double a, double b) {
+    const double s = a + b, z = s - a;
+    return {s, (a - (s - z)) + (b - z)};
+}
+Pair product(Pair a, Pair b) {
+    const double p = a.h * b.h, e = std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
+    const double s = p + e;
+    return {s, e - (s - p)};
+}
+Pair quotient(Pair a, Pair b) {
+    const double q = a.h / b.h, e = (std::fma(-q, b.h, a.h) + (a.l - q * b.l)) / b.h;
+    const double s = q + e;
+    return {s, e - (s - q)};
+}
+// a / b * c, correctly rounded but for ties
+double rounded_quotient(double a, Pair b, Pair c) { return product(quotient({a, 0.0}, b), c).h; }
+
+// The shape derivatives divided by the largest, (1 + g)^2 / 8, and the square of that.  A derivative is
+// +-(1 + g)^2 / 8, (1 - g^2) / 8 or (1 - g)^2 / 8 (g = kGS1); rounded as they are, the first is high by 0.7 of
+// its last place, everywhere it stands, and so were K's values: 1.3e-16 of themselves on average for
+// steel.  As 1, t and t^2, t = (1 - g) / (1 + g), the ones that matter most are exact, and with mu and
+// lam / mu rounded once K's error is rounding noise (100 jittered unit elements of steel: 1.7e-16 rms
+// against 80-bit arithmetic, 2.1e-16 with the table as it is).
+struct UnitShape {
+    double dnr[8][24];
+    Pair scale;
+};
+const UnitShape& unit_shape() {
+    static const UnitShape u = [] {
+        UnitShape v;
+        const Pair far = two_sum(1.0, kGS1), near = two_sum(1.0, -kGS1);
+        const Pair a = product(far, far), t = quotient(near, far), t2 = product(t, t);
+        const double values[3] = {1.0, t.h, t2.h};
+        const ShapeTables& s = shape_tables();
+        for (int g = 0; g < 8; ++g)
+            for (int k = 0; k < 24; ++k) {
+                const double d = s.dnr[g][k / 3][k % 3], r = std::fabs(d) * 8 / a.h;   // one of the three, to rounding
+                v.dnr[g][k] = std::copysign(values[r > 0.6 ? 0 : r > 0.15 ? 1 : 2], d);
+            }
+        v.scale = product(a, a);
+        v.scale.h /= 64;
+        v.scale.l /= 64;
+        return v;
+    }();
+    return u;
+}
+
+}  // namespace
+
 int sm_count();
 int launch_hex8_element_dd(const fem_mesh* mesh, const fem_material* mat, void* workspace, cudaStream_t st,
                            int64_t e_begin, int64_t e_end);
@@ -1017,8 +1074,11 @@ int launch_hex8_element(const fem_mesh* mesh, const fem_material* mat, void* wor
     ep.e_end = e_end;
     ep.rec = static_cast<double*>(workspace);
     const double EX = mat->EX, PO = mat->PO;
-    ep.lm = 2 * PO / (1 - 2 * PO);   // FEM_model_bsr.py:435-449: D0 = lam + 2 mu and lam, D1 = mu
-    ep.mu8 = EX / 2 / (1 + PO) / 8;
+    const UnitShape& us = unit_shape();
+    std::memcpy(ep.dnr, us.dnr, sizeof(ep.dnr));
+    // FEM_model_bsr.py:435-449: D0 = lam + 2 mu and lam, D1 = mu
+    ep.lm = rounded_quotient(2 * PO, two_sum(1.0, -2 * PO), {1.0, 0.0});
+    ep.mu8 = rounded_quotient(EX, two_sum(1.0, PO), us.scale) / 16;
     {
         const double w0 = mat->omega[0], w1 = mat->omega[1], w2 = mat->omega[2];
         const double wc[3][3] = {{w1 * w1 + w2 * w2, -w0 * w1, -w0 * w2},   // UnitVectorF, FEM_model_bsr.py:291-300
@@ -1027,7 +1087,6 @@ int launch_hex8_element(const fem_mesh* mesh, const fem_material* mat, void* wor
         for (int i = 0; i < 3; ++i)
             for (int j = 0; j < 3; ++j) ep.wc[i][j] = wc[i][j];
     }
-    ep.tab = make_tables();
     {
         // 1D shape factors (1 + s x) / 2 at x = +-kGS1: al for a corner on the Gauss point's
         // side, be for the other side

@@ -69,22 +69,6 @@ struct ShapeTables {
 };
 const ShapeTables& shape_tables();
 
-// Kernel-parameter copy of the tables (passed by value, staged into shared memory).
-struct DevTables {
-    double dnr[8][8][3];
-    double nr[8][8];
-};
-inline DevTables make_tables() {
-    const ShapeTables& t = shape_tables();
-    DevTables d;
-    for (int g = 0; g < 8; ++g)
-        for (int a = 0; a < 8; ++a) {
-            d.nr[g][a] = t.nr[g][a];
-            for (int k = 0; k < 3; ++k) d.dnr[g][a][k] = t.dnr[g][a][k];
-        }
-    return d;
-}
-
 // Upper-triangular node-pair numbering (a <= b), row-major: 36 pairs per element.
 __host__ __device__ constexpr int pair_index(int a, int b) {
     return a * 8 - (a * (a - 1)) / 2 + (b - a);
