@@ -225,15 +225,19 @@ __device__ __noinline__ void sym3_eig_jacobi(double a00, double a11, double a22,
 
 // Eigenvalues, descending, of a symmetric 3x3 (the same entries as sym3_eig_jacobi) with few FP64
 // instructions: the FP32 pipes find the eigenvectors, FP64 only applies and corrects them.
-//  1. Cyclic Jacobi in FP32 accumulates its rotations in a quaternion q (components of 24 bits).
+//  1. Cyclic Jacobi in FP32 accumulates its rotations in a quaternion q, rounded to multiples of 2^-22
+//     so that the entries of R(q) are exact in FP64.
 //  2. R(q) is |q|^2 times an orthogonal matrix whatever q is, so B = R^T A R / |q|^4 has A's
-//     eigenvalues to FP64 rounding; its off-diagonals are FP32 noise, ~1e-7 |A|.
+//     eigenvalues; its off-diagonals are FP32 noise, ~2e-7 |A|.  With theta_j the FP32 eigenvalues
+//     (R^T R is diagonal), B_ij = theta_j delta_ij + R_i . (A - theta_j) R_j / |q|^4: the vectors are as
+//     small as the off-diagonals, so of the two products only the first rounds at the size of A.
 //  3. Jacobi rotations in FP64 with tan(phi) = t from FP32.  The rotation is orthogonal for any t
 //     (c = 1 / sqrt(1 + t^2) refined to FP64), and what an inexact t leaves is carried, not dropped:
 //     each sweep takes the off-diagonals down by another ~1e-7, so one sweep serves separated
 //     eigenvalues (the neglected shift e^2 / gap is below 1e-18 |A|) and two serve equal ones.
-// About 150 FP64 instructions against 630 of the Jacobi form (no FP64 division or square root):
-// k_stress_node on 1,010,025 nodes 1.37 -> 0.45 ms.  A matrix outside the FP32 range, or with an
+// About 160 FP64 instructions against 630 of the Jacobi form (no FP64 division or square root):
+// k_stress_node on 1,010,025 nodes 1.37 -> 0.47 ms.  Rms error, of |A|, on random tensors 0.92e-16 (Jacobi
+// 1.25e-16; 1.6e-16 with R rounded and B formed without theta), on uniaxial ones 0.74e-16 (0.68e-16).  A matrix outside the FP32 range, or with an
 // infinity or NaN, takes sym3_eig_jacobi.
 __device__ __forceinline__ float tan_rotation(float h, float apq) {  // h = a_qq - a_pp
     const float theta = __fdividef(0.5f * h, apq);
@@ -286,24 +290,29 @@ __device__ __forceinline__ void sym3_eig_desc(double a00, double a11, double a22
     }
     double d0, d1, d2, e01, e02, e12;
     {
+        // multiples of 2^-22 (the sums lie in [2, 4]): products and sums of four are exact in 53 bits
+        auto grid = [](float v) { return __fsub_rn(__fadd_rn(v, 3.f), 3.f); };
+        qw = grid(qw), qx = grid(qx), qy = grid(qy), qz = grid(qz);
         const double w = qw, x = qx, y = qy, z = qz, x2 = 2.f * qx, y2 = 2.f * qy, z2 = 2.f * qz;
-        const double ww = w * w, xx = x * x, yy = y * y, zz = z * z;   // exact: 24-bit factors
+        const double ww = w * w, xx = x * x, yy = y * y, zz = z * z;
         const double a = ww + xx, b = yy + zz, cd = ww - xx, dd = yy - zz;
         const double wz = w * z2, wy = w * y2, wx = w * x2;
         const double R[3][3] = {{a - b, fma(x, y2, -wz), fma(x, z2, wy)},
                                 {fma(x, y2, wz), cd + dd, fma(y, z2, -wx)},
                                 {fma(x, z2, -wy), fma(y, z2, wx), cd - dd}};
-        const double eps = (a + b) - 1.0;                          // |q|^2 - 1, FP32 rounding only
+        const double eps = (a + b) - 1.0;                          // |q|^2 - 1
         const double f = fma(eps, fma(3.0, eps, -2.0), 1.0);       // |q|^-4
-        double C[3][3];   // A R
+        const double th[3] = {f00, f11, f22};
+        double C[3][3];   // (A - theta_j) R_j
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            C[0][j] = fma(a02, R[2][j], fma(a01, R[1][j], a00 * R[0][j]));
-            C[1][j] = fma(a12, R[2][j], fma(a11, R[1][j], a01 * R[0][j]));
-            C[2][j] = fma(a22, R[2][j], fma(a12, R[1][j], a02 * R[0][j]));
+            C[0][j] = fma(a02, R[2][j], fma(a01, R[1][j], (a00 - th[j]) * R[0][j]));
+            C[1][j] = fma(a12, R[2][j], fma(a01, R[0][j], (a11 - th[j]) * R[1][j]));
+            C[2][j] = fma(a12, R[1][j], fma(a02, R[0][j], (a22 - th[j]) * R[2][j]));
         }
-        auto dot = [&](int i, int j) { return f * fma(R[2][i], C[2][j], fma(R[1][i], C[1][j], R[0][i] * C[0][j])); };
-        d0 = dot(0, 0), d1 = dot(1, 1), d2 = dot(2, 2), e01 = dot(0, 1), e02 = dot(0, 2), e12 = dot(1, 2);
+        auto dot = [&](int i, int j) { return fma(R[2][i], C[2][j], fma(R[1][i], C[1][j], R[0][i] * C[0][j])); };
+        d0 = fma(f, dot(0, 0), th[0]), d1 = fma(f, dot(1, 1), th[1]), d2 = fma(f, dot(2, 2), th[2]);
+        e01 = f * dot(0, 1), e02 = f * dot(0, 2), e12 = f * dot(1, 2);
     }
     const float rm = __fdividef(1.f, m);
     for (int sweep = 0; sweep < 4; ++sweep) {
