@@ -10,22 +10,22 @@
 //    accumulates column j of Q (coalesced loads along a row of Q) against all b columns of X.  The
 //    per-CTA partials are summed in a fixed order (deterministic): kSeg warps of a block each sum
 //    a consecutive share of the CTAs for 32 outputs, loads running ahead, then the shares in order.
-//  k_ts_nn: W = beta W + alpha Q C (C m x b staged in shared memory): one thread per row of Q, which
-//    a warp reads 32 x 32 values at a time, coalesced, into its own shared-memory tile, the next
-//    tile's loads in flight; the row's sums over the columns are b independent chains.
+//  k_ts_nn: W = beta W + alpha Q C (C m x b staged in shared memory): one thread per row of Q and one
+//    or two columns of W; a warp reads Q 32 x 32 values at a time, coalesced, into its own shared-memory
+//    tile, the next tile's loads in flight.
 // FP64 throughout and bound by the FP64 pipe (n m b FMAs each: 199 us at 65,559 x 190 x 10), so the
-// column count of X / W is a template width close to b (4, 8, 10, 12, 16, 24, 32) rather than a
-// power of two: padded columns would be FMAs on zeros.  At that size the products took 251 + 84 us
-// (whole chunks per CTA: 4 on some SMs, 3 on others; one thread summing 513 partials) and 479 us
-// (a warp per row, lanes over the columns: the butterfly adds of 10 sums were as many FP64
-// instructions as the FMAs); now 215 + 15 and
-// 253 us.
+// column count of X is a template width close to b (4, 8, 10, 12, 16, 24, 32) rather than a power of
+// two: padded columns would be FMAs on zeros.  At that size the products took 251 + 84 us (whole
+// chunks per CTA: 4 on some SMs, 3 on others; one thread summing 513 partials) and 479 us (a warp per
+// row, lanes over the columns: the butterfly adds of 10 sums were as many FP64 instructions as the FMAs);
+// now 215 + 15 and 298 us.
 #include <algorithm>
 #include <type_traits>
 
 #include "fem_common.cuh"
 
 namespace fem {
+int sm_count();
 namespace {
 
 constexpr int kChunk = 64;     // rows per step of the transposed product
@@ -95,7 +95,9 @@ __global__ void __launch_bounds__(kSeg * 32) k_ts_tn_reduce(int m, int b, int nb
 // Columns [B blockIdx.y, B (blockIdx.y + 1)) of W.  A row's sum over the m columns of Q is a tree down to
 // chains of four, not one chain: with m = 190 random terms its rms error is 1.4e-16 of the sum, 4.6e-16 as
 // a chain (1.45e-16 as 32 lanes and a butterfly).  The tree adds a quarter to the FP64 instructions.
-template <int B>
+// kSplit: the CTA's two warps share 32 rows, one takes every other tile of 32 columns; the two totals
+// of a row are the same sums either way.
+template <int B, bool kSplit>
 __global__ void __launch_bounds__(kNnThreads) k_ts_nn(int64_t n, int m, int b, const double* __restrict__ Q,
                                                         int64_t ldq, const double* __restrict__ C, int64_t ldc,
                                                         double alpha, double beta, double* W, int64_t ldw) {
@@ -106,12 +108,12 @@ __global__ void __launch_bounds__(kNnThreads) k_ts_nn(int64_t n, int m, int b, c
         cs[i] = j < m && c < bs ? C[int64_t(j) * ldc + c0 + c] : 0.0;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    double* tile = cs + m8 * B + (threadIdx.x >> 5) * (32 * 33);
-    const int64_t groups = (n + 31) / 32, nwarps = (int64_t(gridDim.x) * kNnThreads) >> 5;
-    for (int64_t gr = (int64_t(blockIdx.x) * kNnThreads + threadIdx.x) >> 5; gr < groups; gr += nwarps) {
-        const int64_t r0 = gr * 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* tile = cs + m8 * B + warp * (32 * 33);
+    constexpr int kStep = kSplit ? 64 : 32, kRows = kSplit ? 32 : kNnThreads;   // a CTA's rows
+    for (int64_t r0 = int64_t(blockIdx.x) * kRows + (kSplit ? 0 : 32 * warp); r0 < n; r0 += int64_t(gridDim.x) * kRows) {
         const int rows = int(std::min<int64_t>(32, n - r0));
+        const int first = kSplit ? 32 * warp : 0;
         double even[B], odd[B], q[32];   // sums over every other tile of 32 columns
 #pragma unroll
         for (int c = 0; c < B; ++c) even[c] = odd[c] = 0.0;
@@ -120,13 +122,13 @@ __global__ void __launch_bounds__(kNnThreads) k_ts_nn(int64_t n, int m, int b, c
 #pragma unroll
             for (int r = 0; r < 32; ++r) q[r] = r < rows && j0 + lane < m ? __ldg(p + int64_t(r) * ldq) : 0.0;
         };
-        load(0);
-        for (int j0 = 0; j0 < m; j0 += 32) {
+        load(first);
+        for (int j0 = first; j0 < m; j0 += kStep) {
             __syncwarp();
 #pragma unroll
             for (int r = 0; r < 32; ++r) tile[r * 33 + lane] = q[r];
             __syncwarp();
-            if (j0 + 32 < m) load(j0 + 32);
+            if (j0 + kStep < m) load(j0 + kStep);
             const double* cj = cs + j0 * B;
             const double* tl = tile + lane * 33;
             const int nj = min(32, m8 - j0);
@@ -159,11 +161,22 @@ __global__ void __launch_bounds__(kNnThreads) k_ts_nn(int64_t n, int m, int b, c
 #pragma unroll
             for (int c = 0; c < B; ++c) {
                 const double v = even[c] + t[c];
-                even[c] = odd[c];
-                odd[c] = v;
+                even[c] = kSplit ? v : odd[c];
+                odd[c] = kSplit ? 0.0 : v;
             }
         }
-        if (lane < rows) {
+        if constexpr (kSplit) {   // warp 1's total to warp 0, through the front of its own tile
+            __syncwarp();
+            if (warp == 1)
+#pragma unroll
+                for (int c = 0; c < B; ++c) tile[c * 32 + lane] = even[c];
+            __syncthreads();
+            if (warp == 0)
+#pragma unroll
+                for (int c = 0; c < B; ++c) odd[c] = tile[32 * 33 + c * 32 + lane];
+            __syncthreads();
+        }
+        if (lane < rows && !(kSplit && warp)) {
             double* w = W + (r0 + lane) * ldw + c0;
 #pragma unroll
             for (int c = 0; c < B; ++c) {
@@ -192,28 +205,18 @@ int ts_tn(int64_t n, int m, int b, const double* Q, int64_t ldq, const double* X
     return FEM_OK;
 }
 
-template <int B>
+template <int B, bool kSplit>
 int ts_nn(int64_t n, int m, int b, const double* Q, int64_t ldq, const double* C, int64_t ldc, double alpha,
           double beta, double* W, int64_t ldw, cudaStream_t st) {
     const size_t smem = (size_t((m + 7) & ~7) * B + (kNnThreads / 32) * 32 * 33) * sizeof(double);
-    FEM_CUDA(cudaFuncSetAttribute(k_ts_nn<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    // a warp per 32 rows; every group of rows in one wave where they fit
-    const int64_t need = (n + kNnThreads - 1) / kNnThreads;
-    const dim3 grid(unsigned(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(1) << 20))), (b + B - 1) / B);
-    k_ts_nn<B><<<grid, kNnThreads, smem, st>>>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw);
+    const int64_t rows = kSplit ? 32 : kNnThreads;
+    const dim3 grid(unsigned(std::min<int64_t>((n + rows - 1) / rows, int64_t(1) << 20)), (b + B - 1) / B);
+    k_ts_nn<B, kSplit><<<grid, kNnThreads, smem, st>>>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw);
     FEM_LAUNCH_CHECK("k_ts_nn");
     return FEM_OK;
 }
 
 int width(int b) { return b <= 4 ? 4 : b <= 8 ? 8 : b <= 10 ? 10 : b <= 12 ? 12 : b <= 16 ? 16 : b <= 24 ? 24 : 32; }
-
-// Columns of W per CTA of k_ts_nn: the width that pads b least, at most 12 (the tree's registers)
-int nn_width(int b) {
-    int best = 4;
-    for (int w : {8, 10, 12})
-        if ((b + w - 1) / w * w <= (b + best - 1) / best * best) best = w;
-    return best;
-}
 
 }  // namespace
 }  // namespace fem
@@ -254,13 +257,16 @@ extern "C" int fem_ts_gemm_nn(int64_t n, int m, int b, const double* Q, int64_t 
     FEM_REQUIRE(n > 0 && m > 0 && m <= kMaxCols && b > 0 && b <= 32 && Q && C && W, "bad arguments");
     FEM_REQUIRE(ldq >= m && ldc >= b && ldw >= b, "leading dimensions too small");
     cudaStream_t st = as_stream(stream);
-    auto run = [&](auto width_c) {
-        return ts_nn<decltype(width_c)::value>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw, st);
-    };
-    switch (nn_width(b)) {
-        case 4: return run(std::integral_constant<int, 4>());
-        case 8: return run(std::integral_constant<int, 8>());
-        case 10: return run(std::integral_constant<int, 10>());
-        default: return run(std::integral_constant<int, 12>());
-    }
+    // An SM sub-partition takes one FP64 warp instruction every 64 cycles, so the time is that of the
+    // sub-partition with the most (32 rows, column) warps, and of one warp's chain when there are few.  parts:
+    // sub-partitions (608).  Two warps a row group (times in us, m = 190) at 2,100 x 16 (1.7 warps each) 22.8
+    // against 24.9, at 4,200 x 10 (2.2) 33.1 against 28.9; two columns a warp at 8,400 x 8 (3.5) 41.3 against
+    // 37.3, at 8,400 x 10 (4.3) 49.3 against 76.0 (a second wave of CTAs), at 65,559 x 10 298 against 312.  An odd
+    // b pads a column: 65,559 x 3 127 against 115, but 13,000 x 9 (6.0) 67.9 against 78.0.  Wider columns were
+    // slower throughout (65,559 x 10 in one: 340).
+    const int64_t warps = (n + 31) / 32 * b, parts = 4 * int64_t(sm_count());
+    if (4 * warps <= 7 * parts) return ts_nn<1, true>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw, st);
+    if (warps <= 4 * parts || (b % 2 && warps > 8 * parts))
+        return ts_nn<1, false>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw, st);
+    return ts_nn<2, false>(n, m, b, Q, ldq, C, ldc, alpha, beta, W, ldw, st);
 }
