@@ -268,7 +268,7 @@ __device__ __forceinline__ Dot<T> spmv1_rows_epi(const BsrView<T>& A, const T* _
 // Bound by L1 (84 lines of x per 27-block row at R = 32) and the latency of the gathers.  Product of
 // 137,781 rows at R = 32: 207 us with one right-hand side per lane and values loaded in line (1,188
 // instructions a row, most of them addresses); 190 us with vectors of right-hand sides (560, every step
-// waiting on values from HBM); 125 us staged.  L1 capacity decides the rest: 2 rows staged and 2 CTAs an SM
+// waiting on values from HBM); 125 us staged, 119 us with the slot groups beyond a row's end left out.  L1 capacity decides the rest: 2 rows staged and 2 CTAs an SM
 // leave it 192 KB (3 rows: 156 us; 3 CTAs with p.q: 339 instead of 268 us an iteration of the solve);
 // fewer right-hand sides gather less and take 3 CTAs (R = 8: 59 against 69 us).  V and G: 4-slot groups of a 28-slot row in 2 x 4 or 8
 // groups leave 1 in 8 idle, more groups would idle half.
@@ -359,13 +359,9 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
         for (int j = 0; j < 3; ++j)
 #pragma unroll
             for (int i = 0; i < V; ++i) acc[j][i] = 0.f;
-        // one step: 4 slots of every group, values and columns from `val` and `col`
-        auto step = [&](int c0, const float* val, const int32_t* col) {
-            const int s = c0 + 4 * g;
-            const bool in = s < Lp;
-            // slots beyond the row: the row's own x times 0
-            const int4 idx = in ? *reinterpret_cast<const int4*>(col + s)
-                                : make_int4(int(row), int(row), int(row), int(row));
+        // 4 slots, values and columns from `val` and `col`; the groups beyond the row's end sit out
+        auto step = [&](int s, const float* val, const int32_t* col) {
+            const int4 idx = *reinterpret_cast<const int4*>(col + s);
             X xv[4][3];
             const int cc[4] = {idx.x, idx.y, idx.z, idx.w};
 #pragma unroll
@@ -389,8 +385,7 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
             for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const float4 w = in ? *reinterpret_cast<const float4*>(vs + (3 * j + c) * Lp)
-                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 w = *reinterpret_cast<const float4*>(vs + (3 * j + c) * Lp);
 #pragma unroll
                     for (int i = 0; i < V; ++i) {
                         acc[j][i] = fmaf(w.x, xv[0][c].v[i], acc[j][i]);
@@ -402,10 +397,10 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
         };
         if (Lp <= kStageSlots) {
 #pragma unroll 1
-            for (int c0 = 0; c0 < Lp; c0 += CS) step(c0, st.val, st.col);
+            for (int s = 4 * g; s < Lp; s += CS) step(s, st.val, st.col);
         } else {
 #pragma unroll 1
-            for (int c0 = 0; c0 < Lp; c0 += CS) step(c0, A.vals + 9 * rs[0], A.indices + rs[0]);
+            for (int s = 4 * g; s < Lp; s += CS) step(s, A.vals + 9 * rs[0], A.indices + rs[0]);
         }
         __syncwarp();   // the ring slot may be refilled
         // reduce-scatter: after a level with offset off, lane keeps half of its right-hand sides
