@@ -290,10 +290,10 @@ constexpr int spmm_ctas() {
 
 __device__ __forceinline__ void copy_async16(void* dst, const void* src, uint64_t pol) {
     asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(
-                     unsigned(__cvta_generic_to_shared(dst))), "l"(src), "l"(pol));
+                     unsigned(__cvta_generic_to_shared(dst))), "l"(src), "l"(pol) : "memory");
 }
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(dst))), "l"(src));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
 }
 
 template <int R, typename Epi>
@@ -343,13 +343,13 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
                 if (lane < L / 4) copy_async16(st.col + 4 * lane, A.indices + r0 + 4 * lane);
             }
         }
-        asm volatile("cp.async.commit_group;");
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
     for (int d = 0; d < kStage - 1; ++d) fetch(d, rs[d], len[d]);
     for (int t = 0; t < steps; ++t) {
         fetch(t + kStage - 1, rs[kStage - 1], len[kStage - 1]);
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStage - 1));
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStage - 1) : "memory");
         __syncwarp();   // every lane's copies of this row have landed
         const int64_t row = first + stride * t;
         const int Lp = len[0];
@@ -434,7 +434,7 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
 #pragma unroll
         for (int d = 0; d < kStage - 1; ++d) rs[d] = rs[d + 1], len[d] = len[d + 1];
     }
-    asm volatile("cp.async.wait_all;");
+    asm volatile("cp.async.wait_all;" ::: "memory");
     return dot;
 }
 
