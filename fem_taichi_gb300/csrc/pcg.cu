@@ -1143,7 +1143,8 @@ int solve_r(const fem_bsr* A64, const fem_bsr* A32, const double* M64, fem_amg* 
     FEM_CUDA(cudaMemsetAsync(st, 0, sizeof(PcgState), s));
     double bnorm[kMaxR];
     {
-        // ||F_k||; a mixed solve starts from u = 0, whose residual F goes to its r64
+        // ||F_k||; a mixed solve starts from u = 0, whose residual F goes to its r64 (F - K 0 is NaN where K is
+        // not finite, and a NaN norm reads as converged)
         double* r0 = o->mixed ? reinterpret_cast<double*>(ws + L.v64[1]) : nullptr;
         k_residual_zero<R><<<vec_grid(k_residual_zero<R>, nv), kThreads, 0, s>>>(nv, F, r0, part, st);
         FEM_LAUNCH_CHECK("k_residual_zero");
