@@ -94,7 +94,8 @@ struct ElemSmem {
 };
 
 // Class of the corner pair (a, b) for the mass: per axis 0 both corners on the negative side,
-// 1 mixed, 2 both positive (corner sides as in monomial_sign); M_ab depends only on it.
+// 1 mixed, 2 both positive; M_ab depends only on it.  Corners on the negative side of xi: 1, 2, 5, 6 (mask
+// 0x66), of eta: 2, 3, 6, 7 (0xCC), of zeta: 0-3 (0x0F).
 __device__ __forceinline__ int mass_class(int a, int b) {
     const int nx = (0x66 >> a) & 1, ny = (0xCC >> a) & 1, nz = (0x0F >> a) & 1;
     const int mx = (0x66 >> b) & 1, my = (0xCC >> b) & 1, mz = (0x0F >> b) & 1;
@@ -666,9 +667,8 @@ struct Gather64Params {
     const double* loads;
 };
 
-template <int W>
 struct Gather64Smem {
-    double acc[W][kG64Rows][kG64RowStride];
+    double acc[kG64Warps][kG64Rows][kG64RowStride];
 };
 
 // Lane-per-slot path for one row of any length (K and M; F is summed by the caller).
@@ -719,14 +719,13 @@ __device__ void gather_row_long64(const Gather64Params& p, int64_t row, int lane
     }
 }
 
-template <int W>
-__global__ void __launch_bounds__(W * 32, 24 / W) k_gather64(const Gather64Params p) {
+__global__ void __launch_bounds__(kG64Warps * 32, 6) k_gather64(const Gather64Params p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Gather64Smem<W>& S = *reinterpret_cast<Gather64Smem<W>*>(smem_raw);
+    Gather64Smem& S = *reinterpret_cast<Gather64Smem*>(smem_raw);
     const unsigned full = 0xffffffffu;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane >> 3, b = lane & 7;
-    const int64_t row0 = p.row_begin + (int64_t(blockIdx.x) * W + w) * kG64Rows;
+    const int64_t row0 = p.row_begin + (int64_t(blockIdx.x) * kG64Warps + w) * kG64Rows;
     if (row0 >= p.row_end) return;  // uniform per warp
     const int64_t row = row0 + r;
     const bool vrow = row < p.row_end;
@@ -1160,12 +1159,11 @@ int launch_gather64(const fem_mesh* mesh, const fem_assembly_out* out, const voi
     gp.F = out->F;
     gp.fixed = out->fixed;
     gp.loads = out->loads;
-    constexpr int W = kG64Warps;
-    const size_t smem = sizeof(Gather64Smem<W>);
-    FEM_CUDA(cudaFuncSetAttribute(k_gather64<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int64_t rows_per_cta = int64_t(W) * kG64Rows;
+    const size_t smem = sizeof(Gather64Smem);
+    FEM_CUDA(cudaFuncSetAttribute(k_gather64, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    const int64_t rows_per_cta = int64_t(kG64Warps) * kG64Rows;
     const int64_t blocks = (row_end - row_begin + rows_per_cta - 1) / rows_per_cta;
-    k_gather64<W><<<unsigned(blocks), W * 32, smem, st>>>(gp);
+    k_gather64<<<unsigned(blocks), kG64Warps * 32, smem, st>>>(gp);
     FEM_LAUNCH_CHECK("k_gather64");
     return FEM_OK;
 }

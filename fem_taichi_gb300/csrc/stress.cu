@@ -232,13 +232,14 @@ __device__ __noinline__ void sym3_eig_jacobi(double a00, double a11, double a22,
 //     (R^T R is diagonal), B_ij = theta_j delta_ij + R_i . (A - theta_j) R_j / |q|^4: the vectors are as
 //     small as the off-diagonals, so of the two products only the first rounds at the size of A.
 //  3. Jacobi rotations in FP64 with tan(phi) = t from FP32.  The rotation is orthogonal for any t
-//     (c = 1 / sqrt(1 + t^2) refined to FP64), and what an inexact t leaves is carried, not dropped:
+//     (c = 1 / sqrt(1 + t^2): from y, the same in FP32, and r = 1 - (1 + t^2) y^2, by the binomial series of
+//     y (1 - r)^(-1/2) to second order; r is about 1e-7), and what an inexact t leaves is carried, not dropped:
 //     each sweep takes the off-diagonals down by another ~1e-7, so one sweep serves separated
 //     eigenvalues (the neglected shift e^2 / gap is below 1e-18 |A|) and two serve equal ones.
 // About 160 FP64 instructions against 630 of the Jacobi form (no FP64 division or square root):
 // k_stress_node on 1,010,025 nodes 1.37 -> 0.47 ms.  Rms error, of |A|, on random tensors 0.92e-16 (Jacobi
-// 1.25e-16; 1.6e-16 with R rounded and B formed without theta), on uniaxial ones 0.74e-16 (0.68e-16).  A matrix outside the FP32 range, or with an
-// infinity or NaN, takes sym3_eig_jacobi.
+// 1.25e-16; 1.6e-16 with R rounded and B formed without theta), on uniaxial ones 0.74e-16 (0.68e-16).
+// A matrix outside the FP32 range, or with an infinity or NaN, takes sym3_eig_jacobi.
 __device__ __forceinline__ float tan_rotation(float h, float apq) {  // h = a_qq - a_pp
     const float theta = __fdividef(0.5f * h, apq);
     const float t = __fdividef(1.f, fabsf(theta) + __fsqrt_rn(fmaf(theta, theta, 1.f)));
