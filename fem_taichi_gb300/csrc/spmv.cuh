@@ -185,14 +185,22 @@ __device__ __forceinline__ Dot<float> spmv4_rows_epi(const BsrView<float>& A, co
             }
 #pragma unroll
             for (int q = 0; q < 9; ++q) w[q] = load_l2(reinterpret_cast<const float4*>(v0 + int64_t(q) * L), pol);
+            // the products of two slots in one chain, then added: with one chain over the row the product of
+            // 8,125 rows is off by 8.5e-8 (rms), 6.7e-8 here (7.4e-8 with a sum per block added)
             return [=](float& b0, float& b1, float& b2) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < 4; j += 2) {
                     // component j of each value's float4 = slot s + j
-                    auto wq = [&](int q) { return j == 0 ? w[q].x : j == 1 ? w[q].y : j == 2 ? w[q].z : w[q].w; };
-                    b0 = fmaf(wq(0), xv[j].x, fmaf(wq(1), xv[j].y, fmaf(wq(2), xv[j].z, b0)));
-                    b1 = fmaf(wq(3), xv[j].x, fmaf(wq(4), xv[j].y, fmaf(wq(5), xv[j].z, b1)));
-                    b2 = fmaf(wq(6), xv[j].x, fmaf(wq(7), xv[j].y, fmaf(wq(8), xv[j].z, b2)));
+                    auto pair = [&](int q, float b) {
+                        const float v0 = j ? w[q].z : w[q].x, v1 = j ? w[q + 1].z : w[q + 1].x, v2 = j ? w[q + 2].z : w[q + 2].x;
+                        const float u0 = j ? w[q].w : w[q].y, u1 = j ? w[q + 1].w : w[q + 1].y, u2 = j ? w[q + 2].w : w[q + 2].y;
+                        float t = fmaf(v2, xv[j].z, fmaf(v1, xv[j].y, v0 * xv[j].x));
+                        t = fmaf(u2, xv[j + 1].z, fmaf(u1, xv[j + 1].y, fmaf(u0, xv[j + 1].x, t)));
+                        return b + t;
+                    };
+                    b0 = pair(0, b0);
+                    b1 = pair(3, b1);
+                    b2 = pair(6, b2);
                 }
             };
         };
@@ -268,10 +276,14 @@ __device__ __forceinline__ Dot<T> spmv1_rows_epi(const BsrView<T>& A, const T* _
 // Bound by L1 (84 lines of x per 27-block row at R = 32) and the latency of the gathers.  Product of
 // 137,781 rows at R = 32: 207 us with one right-hand side per lane and values loaded in line (1,188
 // instructions a row, most of them addresses); 190 us with vectors of right-hand sides (560, every step
-// waiting on values from HBM); 125 us staged, 119 us with the slot groups beyond a row's end left out.  L1 capacity decides the rest: 2 rows staged and 2 CTAs an SM
-// leave it 192 KB (3 rows: 156 us; 3 CTAs with p.q: 339 instead of 268 us an iteration of the solve);
-// fewer right-hand sides gather less and take 3 CTAs (R = 8: 59 against 69 us).  V and G: 4-slot groups of a 28-slot row in 2 x 4 or 8
-// groups leave 1 in 8 idle, more groups would idle half.
+// waiting on values from HBM); 125 us staged, 119 us with the slot groups beyond a row's end left out.  L1
+// capacity decides the rest: 2 rows staged and 2 CTAs an SM leave it 192 KB (3 rows: 156 us; 3 CTAs with
+// p.q: 339 instead of 268 us an iteration of the solve);
+// fewer right-hand sides gather less and take 3 CTAs (R = 8: 59 against 69 us).  V and G: 4-slot groups of a
+// 28-slot row in 2 x 4 or 8 groups leave 1 in 8 idle, more groups would idle half.  kTwo: two sums a row
+// and right-hand side, so that the chains are as short as block sums added were (8,125 rows against FP64:
+// 7.1e-8 to 7.4e-8, 8.4e-8 with one; block sums 7.5e-8 to 8.5e-8, at R = 32, one group, 10.4e-8: there
+// one is enough).  At R = 16 they leave V = 4 no third CTA: 84 us of 141,426 rows, 82 with V = 2.
 template <int V>
 struct alignas(4 * V) FloatVec {
     float v[V];
@@ -298,7 +310,8 @@ __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
 
 template <int R, typename Epi>
 __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, const float* __restrict__ x, const Epi& epi) {
-    constexpr int V = R >= 16 ? 4 : R == 8 ? 2 : 1, LP = R / V, G = 32 / LP, CS = 4 * G;
+    constexpr int V = R >= 32 ? 4 : R >= 8 ? 2 : 1, LP = R / V, G = 32 / LP, CS = 4 * G;
+    constexpr bool kTwo = R < 32;
     constexpr unsigned full = 0xffffffffu;
     constexpr int kWarps = 8;
     struct Stage {
@@ -354,11 +367,11 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
         const int64_t row = first + stride * t;
         const int Lp = len[0];
         const Stage& st = ring[wid][t % kStage];
-        float acc[3][V];
+        float acc[3][V], odd[3][V];   // kTwo: of slots 0, 1 and 2, 3 of every four
 #pragma unroll
         for (int j = 0; j < 3; ++j)
 #pragma unroll
-            for (int i = 0; i < V; ++i) acc[j][i] = 0.f;
+            for (int i = 0; i < V; ++i) acc[j][i] = odd[j][i] = 0.f;
         // 4 slots, values and columns from `val` and `col`; the groups beyond the row's end sit out
         auto step = [&](int s, const float* val, const int32_t* col) {
             const int4 idx = *reinterpret_cast<const int4*>(col + s);
@@ -390,8 +403,9 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
                     for (int i = 0; i < V; ++i) {
                         acc[j][i] = fmaf(w.x, xv[0][c].v[i], acc[j][i]);
                         acc[j][i] = fmaf(w.y, xv[1][c].v[i], acc[j][i]);
-                        acc[j][i] = fmaf(w.z, xv[2][c].v[i], acc[j][i]);
-                        acc[j][i] = fmaf(w.w, xv[3][c].v[i], acc[j][i]);
+                        float& a = kTwo ? odd[j][i] : acc[j][i];
+                        a = fmaf(w.z, xv[2][c].v[i], a);
+                        a = fmaf(w.w, xv[3][c].v[i], a);
                     }
                 }
         };
@@ -403,6 +417,12 @@ __device__ __forceinline__ Dot<float> spmm4_rows_epi(const BsrView<float>& A, co
             for (int s = 4 * g; s < Lp; s += CS) step(s, A.vals + 9 * rs[0], A.indices + rs[0]);
         }
         __syncwarp();   // the ring slot may be refilled
+        if constexpr (kTwo) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < V; ++i) acc[j][i] += odd[j][i];
+        }
         // reduce-scatter: after a level with offset off, lane keeps half of its right-hand sides
         int off = LP;
 #pragma unroll
